@@ -200,8 +200,7 @@ nbgb_status nbgb_compute_forces(nbgb_calculator* calc, const nbgb_particle_data*
  * device or fail with NBGB_ERR_OOM; a warm-up call with count 0 does exactly
  * that and nothing else.  cudaDeviceReset after the first call on a device
  * is not supported.  The call cannot run while `stream` is being captured
- * (it returns NBGB_ERR_INVALID_ARG): it reads a device error word back and
- * waits for the stream.  All calls share the scratch: calls that overlap on
+ * (it returns NBGB_ERR_INVALID_ARG): it waits for the stream.  All calls share the scratch: calls that overlap on
  * the GPU race and must be serialised by the caller.  Work is enqueued on
  * `stream` (NULL = legacy default stream) and the call waits for it. */
 nbgb_status nbgb_compute_forces_direct_noalloc(const nbgb_particle_data* d_particles, float G,

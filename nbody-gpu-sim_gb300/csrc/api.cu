@@ -82,17 +82,10 @@ static void validate_params(nbgb_method m, const nbgb_params& p) {
     fail(NBGB_ERR_INVALID_ARG, "Validation Error: CUDA block size must be between 1 and 1024");
 }
 
-int64_t direct_pad(int64_t n) { return ceil_div(std::max<int64_t>(n, 1), kDirTile) * kDirTile; }
-
 void check_device_errors(nbgb_calculator* c) {
-  uint32_t* h = c->h_err.ensure(1);
-  uint32_t* d = c->err.ensure(1);
-  NBGB_CUDA(cudaMemcpyAsync(h, d, sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream));
   NBGB_CUDA(cudaStreamSynchronize(c->stream));
-  uint32_t bits = *h;
+  const uint32_t bits = c->err.take();
   if (bits) {
-    NBGB_CUDA(cudaMemsetAsync(d, 0, sizeof(uint32_t), c->stream));
-    NBGB_CUDA(cudaStreamSynchronize(c->stream));
     std::string msg = "device error word 0x" + std::to_string(bits) + ":";
     nbgb_status s = NBGB_ERR_CUDA;
     if (bits & kErrWaitTimeout) {
@@ -123,15 +116,44 @@ void check_device_errors(nbgb_calculator* c) {
   }
 }
 
-static void direct_forces(nbgb_calculator* c, const float4* pm, int64_t n, float* ax, float* ay,
-                          float* az) {
-  DirectPlan p = plan_direct(n, n, c->variant);
+static void direct_forces(nbgb_calculator* c, const DirectSource& src, int64_t n, float* ax,
+                          float* ay, float* az) {
+  const DirectPlan p = plan_direct(n);
   float4* part = nullptr;
-  if (p.splits > 1) part = c->partial.ensure((size_t)p.splits * p.n_tgt_pad);
+  uint32_t* ticket = nullptr;
+  if (p.splits > 1) {
+    part = c->partial.ensure((size_t)p.splits * p.n_tgt_pad);
+    if (c->ticket.cap < (size_t)p.i_blocks) {  // counters start, and are left, at zero
+      ticket = c->ticket.ensure((size_t)p.i_blocks);
+      NBGB_CUDA(cudaMemsetAsync(ticket, 0, c->ticket.bytes(), c->stream));
+    }
+    ticket = c->ticket.ptr;
+  }
   const float eps = c->params.softening;
-  launch_direct(p, pm, pm, n, c->params.G, eps * eps,
-                (c->params.flags & NBGB_FLAG_COMPENSATED) != 0, part, ax, ay, az,
-                c->err.ensure(1), c->stream);
+  launch_direct(p, src, n, c->params.G, eps * eps,
+                (c->params.flags & NBGB_FLAG_COMPENSATED) != 0, part, ticket, ax, ay, az,
+                c->stream);
+}
+
+// Direct forces straight from the caller's SoA arrays.  Accelerations that
+// share memory with an input go through a packed copy instead: CTAs finish
+// while others still read.
+bool direct_from_soa(const nbgb_particle_data* d) {
+  const float* in[4] = {d->pos_x, d->pos_y, d->pos_z, d->mass};
+  const float* out[3] = {d->acc_x, d->acc_y, d->acc_z};
+  for (const float* o : out)
+    for (const float* i : in)
+      if (o < i + d->count && i < o + d->count) return false;
+  return true;
+}
+
+static void forces_soa(nbgb_calculator* c, const nbgb_particle_data* d) {
+  StageTimer* t = stage_timer(c);
+  if (t) t->st = c->stream;
+  stage_mark(t, "direct.forces");
+  direct_forces(c, DirectSource{nullptr, d->pos_x, d->pos_y, d->pos_z, d->mass},
+                (int64_t)d->count, d->acc_x, d->acc_y, d->acc_z);
+  if (t) t->end();
 }
 
 void forces_packed(nbgb_calculator* c, const float4* pm, int64_t n, float* ax, float* ay,
@@ -142,7 +164,7 @@ void forces_packed(nbgb_calculator* c, const float4* pm, int64_t n, float* ax, f
   switch (c->method) {
     case NBGB_DIRECT_N2:
       stage_mark(t, "direct.forces");
-      direct_forces(c, pm, n, ax, ay, az);
+      direct_forces(c, DirectSource{pm, nullptr, nullptr, nullptr, nullptr}, n, ax, ay, az);
       break;
     case NBGB_BARNES_HUT:
       bh_forces(c, pm, n, ax, ay, az);
@@ -216,14 +238,6 @@ void StageTimer::harvest() {
 void StageTimer::reset() {
   std::fill(total_ms.begin(), total_ms.end(), 0.0);
   std::fill(samples.begin(), samples.end(), 0);
-}
-
-static DirectVariant default_variant() {
-  const char* v = std::getenv("NBGB_DIRECT_VARIANT");
-  if (v && std::strcmp(v, "scalar4") == 0) return DirectVariant::kScalar4;
-  if (v && std::strcmp(v, "paired8") == 0) return DirectVariant::kPaired8;
-  // packed FP32x2 halves the FP32 issue slots: 54.5 vs 48.5 TFLOP/s at N = 1M
-  return DirectVariant::kPaired8;
 }
 
 static void check_particles(const nbgb_particle_data* d, bool need_vel, bool need_old) {
@@ -315,12 +329,10 @@ nbgb_status nbgb_calculator_create(nbgb_method method, const nbgb_params* params
     c->method = method;
     c->params = p;
     if (p.flags & NBGB_FLAG_STAGE_TIMINGS) c->timer = std::make_unique<StageTimer>();
-    c->variant = default_variant();
     NBGB_CUDA(cudaGetDevice(&c->device));
     NBGB_CUDA(cudaStreamCreate(&c->stream));
     c->own_stream = true;
-    uint32_t* e0 = c->err.ensure(1);
-    NBGB_CUDA(cudaMemsetAsync(e0, 0, sizeof(uint32_t), c->stream));
+    c->err.ensure(1);
     *out = c.release();
   });
 }
@@ -408,10 +420,13 @@ nbgb_status nbgb_compute_forces(nbgb_calculator* calc, const nbgb_particle_data*
     const int64_t n = (int64_t)d->count;
     calc->last_n = n;
     if (n == 0) return;
-    const int64_t n_pad = direct_pad(n);
-    float4* pm = calc->pm.ensure((size_t)n_pad);
-    launch_pack_soa(d->pos_x, d->pos_y, d->pos_z, d->mass, n, n_pad, pm, calc->stream);
-    forces_packed(calc, pm, n, d->acc_x, d->acc_y, d->acc_z);
+    if (calc->method == NBGB_DIRECT_N2 && direct_from_soa(d)) {
+      forces_soa(calc, d);
+    } else {
+      float4* pm = calc->pm.ensure((size_t)n);
+      launch_pack_soa(d->pos_x, d->pos_y, d->pos_z, d->mass, n, n, pm, calc->stream);
+      forces_packed(calc, pm, n, d->acc_x, d->acc_y, d->acc_z);
+    }
     finish_call(calc);
   });
 }
@@ -423,11 +438,14 @@ nbgb_status nbgb_integrate(nbgb_calculator* calc, const nbgb_particle_data* d, f
     const int64_t n = (int64_t)d->count;
     calc->last_n = n;
     if (n == 0) return;
-    const int64_t n_pad = direct_pad(n);
-    float4* pm = calc->pm.ensure((size_t)n_pad);
+    const bool soa = calc->method == NBGB_DIRECT_N2 && direct_from_soa(d);
+    float4* pm = soa ? nullptr : calc->pm.ensure((size_t)n);
     // storeOldAccelerations + updatePositions fused, emitting the packed input.
-    launch_vv_positions(*d, dt, true, pm, n_pad, calc->stream);
-    forces_packed(calc, pm, n, d->acc_x, d->acc_y, d->acc_z);
+    launch_vv_positions(*d, dt, true, pm, n, calc->stream);
+    if (soa)
+      forces_soa(calc, d);
+    else
+      forces_packed(calc, pm, n, d->acc_x, d->acc_y, d->acc_z);
     launch_vv_velocities(*d, dt, calc->stream);
     finish_call(calc);
   });
@@ -606,12 +624,11 @@ nbgb_status nbgb_system_create(nbgb_calculator* calc, const nbgb_particle_data* 
       s->ay64.ensure((size_t)n);
       s->az64.ensure((size_t)n);
     }
-    const int64_t n_pad = direct_pad(n);
-    float4* pm = s->pm.ensure((size_t)n_pad);
-    std::vector<float4> hp((size_t)n_pad, make_float4(0.f, 0.f, 0.f, 0.f));
+    float4* pm = s->pm.ensure((size_t)n);
+    std::vector<float4> hp((size_t)n);
     for (int64_t i = 0; i < n; ++i)
       hp[(size_t)i] = make_float4(h->pos_x[i], h->pos_y[i], h->pos_z[i], h->mass[i]);
-    NBGB_CUDA(cudaMemcpyAsync(pm, hp.data(), (size_t)n_pad * sizeof(float4),
+    NBGB_CUDA(cudaMemcpyAsync(pm, hp.data(), (size_t)n * sizeof(float4),
                               cudaMemcpyHostToDevice, st));
     system_forces(s.get());
     check_device_errors(calc);

@@ -1443,7 +1443,7 @@ void bh_forces(nbgb_calculator* c, const float4* pm, int64_t n, float* ax, float
         bh_build(h, pm, st, err, groups, c->params.group_size, true, timer);
       break;
     }
-    NBGB_CUDA(cudaMemsetAsync(err, 0, sizeof(uint32_t), st));
+    c->err.take();  // the skipped kernels' capacity bit (the stream is idle)
     h.cap = (int64_t)hs[0] + (int64_t)hs[0] / 8 + 64;
   }
   BHWalkParams wp{c->params.G, c->params.softening, c->params.theta, c->params.leaf_capacity,

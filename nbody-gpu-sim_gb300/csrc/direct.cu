@@ -4,19 +4,19 @@
 // (src/cuda/force_direct.cu:10-98).  Law: a_i = G * sum_{j != i} m_j d
 // (d^2 + eps^2)^-3/2 with d = x_j - x_i.
 //
-// Layout: sources are a packed float4 array (x, y, z, m), padded with zero
-// mass up to a multiple of the j-tile, so the inner loop has no bounds test
-// and no self test: with eps > 0 the j == i term is exactly 0 (d = 0).
-// j-tiles of kTile bodies are staged into shared memory by the bulk-copy
-// engine (cp.async.bulk + mbarrier, kStages deep) and read as broadcast
-// 16-byte shared loads.  Each thread owns I targets in registers.
+// Layout: sources are read either from the caller's SoA arrays or from a
+// packed float4 (x, y, z, m) array and staged in shared memory as x, y, z and
+// m rows, so that two consecutive sources arrive as the two halves of a
+// packed FP32x2 operand (direct_pair.cuh).  With eps > 0 the j == i term is
+// exactly 0 (d = 0), so the inner loop has no self test.
 //
-// Accumulation: per target, each j-tile is summed in plain FP32 and folded
-// into a running (sum, error) pair with an error-free two-sum (compensated
-// per j-tile).  COMP = false gives the plain single-accumulator FP32 sum.
+// Accumulation: per target and j-tile slice (at most 256 sources), two plain
+// FP32 partial sums (even and odd sources); their sum is folded into a
+// running (sum, error) pair with an error-free two-sum.  COMP = false adds
+// the slices' sums in plain FP32.
 #include "common.cuh"
 #include "kernels.cuh"
-#include "direct_core.cuh"
+#include "direct_pair.cuh"
 
 namespace nbgb {
 
@@ -42,171 +42,234 @@ void launch_pack_soa(const float* x, const float* y, const float* z, const float
 }
 
 // ---------------------------------------------------------------------------
-// The direct kernel: CTA (blockIdx.x) owns kDirThreads*I targets, split
-// (blockIdx.y) owns a contiguous run of j-tiles.
+// The direct kernel.  A CTA owns 128*I targets (blockIdx.x) and a run of
+// a.jper sources (blockIdx.y); its two halves of 128 threads sum the two
+// halves of every 512-source tile for the same targets and are added up in
+// shared memory.  With more than one run the last CTA of a target block to
+// finish adds the runs' partial sums in run order (deterministic), so no
+// second launch is needed.
+//
+// What bounds it: the FP32 pipe (12 lane operations per interaction) once
+// every SM has two CTAs, launch and memory latency below about 4,000 bodies.
+// Pairing sources instead of targets leaves no operand duplication in the
+// inner loop; splitting the sources over CTAs fills the GPU at every size
+// (one CTA per 1,024 targets without a split before: N = 1,024 took 66 us).
 // ---------------------------------------------------------------------------
-template <int I, bool PAIRED, bool COMP, bool ZERO_SOFT>
-__global__ void __launch_bounds__(kDirThreads) direct_kernel(DirectArgs a) {
-  static_assert(!PAIRED || (I % 2 == 0), "paired path needs an even target count");
-  __shared__ alignas(128) float4 s_j[kDirStages][kDirTile];
-  __shared__ alignas(8) uint64_t s_bar[kDirStages];
-  TileRing ring{s_j, s_bar, 0};
-  ring_init(ring);
+template <bool SOA>
+__device__ __forceinline__ float4 load_body(const DirectArgs& a, int64_t i) {
+  if (SOA) return make_float4(a.sx[i], a.sy[i], a.sz[i], a.sm[i]);
+  return a.src[i];
+}
 
-  const int tid = threadIdx.x;
-  const int64_t tgt_base = (int64_t)blockIdx.x * (kDirThreads * I);
-  const int split = blockIdx.y;
-  const int64_t tile0 = (int64_t)split * a.tiles_per_split;
-  const int64_t tile1 = imin64(tile0 + a.tiles_per_split, a.n_tiles);
-  const int nt = (int)imax64(tile1 - tile0, 0);
+template <int I, bool COMP, bool ZERO_SOFT, bool SOA>
+__global__ void __launch_bounds__(kDirThreads, 2) direct_kernel(DirectArgs a) {
+  constexpr int T = kDirHalf * I;
+  __shared__ __align__(16) float s_t[2][4][kDirTile];
+  __shared__ bool s_last;
+  const int tid = threadIdx.x, half = tid / kDirHalf, tl = tid % kDirHalf;
+  const int64_t tgt_base = (int64_t)blockIdx.x * T;
+  const int64_t j0 = (int64_t)blockIdx.y * a.jper, j1 = imin64(j0 + a.jper, a.n_src);
+  const int nt = (int)ceil_div(j1 - j0, kDirTile);
 
-  // Targets: thread tid owns tgt_base + tid + q*kDirThreads (coalesced I/O).
-  float xi[I], yi[I], zi[I];
+  f2 xi[I], yi[I], zi[I];
+  float sx[I], sy[I], sz[I], ex[I], ey[I], ez[I];
 #pragma unroll
   for (int q = 0; q < I; ++q) {
-    int64_t i = tgt_base + tid + (int64_t)q * kDirThreads;
-    float4 p = (i < a.n_tgt) ? a.tgt[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-    xi[q] = p.x;
-    yi[q] = p.y;
-    zi[q] = p.z;
+    const int64_t i = tgt_base + tl + q * kDirHalf;
+    const float4 p = (i < a.n_tgt) ? load_body<SOA>(a, i) : make_float4(0.f, 0.f, 0.f, 0.f);
+    xi[q] = f2_make(p.x, p.x);
+    yi[q] = f2_make(p.y, p.y);
+    zi[q] = f2_make(p.z, p.z);
+    sx[q] = sy[q] = sz[q] = ex[q] = ey[q] = ez[q] = 0.f;
   }
-  float sx[I], sy[I], sz[I];
-  if (!direct_tiles<kDirThreads, I, PAIRED, COMP, ZERO_SOFT>(ring, a.src + tile0 * kDirTile, nt,
-                                                             xi, yi, zi, a.eps2, sx, sy, sz,
-                                                             a.err))
-    return;
-  const float G = a.G;
+  // the next tile is on its way to registers while the current one is summed
+  float4 v[kDirTile / kDirThreads];
+  auto fetch = [&](int t) {
 #pragma unroll
-  for (int q = 0; q < I; ++q) {
-    int64_t i = tgt_base + tid + (int64_t)q * kDirThreads;
-    if (i >= a.n_tgt) continue;
-    if (a.partial) {
-      a.partial[(int64_t)split * a.n_tgt_pad + i] = make_float4(sx[q], sy[q], sz[q], 0.f);
-    } else {
-      a.out_x[i] = G * sx[q];
-      a.out_y[i] = G * sy[q];
-      a.out_z[i] = G * sz[q];
+    for (int r = 0; r < kDirTile / kDirThreads; ++r) {
+      const int64_t j = j0 + (int64_t)t * kDirTile + r * kDirThreads + tid;
+      v[r] = (j < j1) ? load_body<SOA>(a, j) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
+  };
+  auto stage = [&](int b) {
+#pragma unroll
+    for (int r = 0; r < kDirTile / kDirThreads; ++r) {
+      s_t[b][0][r * kDirThreads + tid] = v[r].x;
+      s_t[b][1][r * kDirThreads + tid] = v[r].y;
+      s_t[b][2][r * kDirThreads + tid] = v[r].z;
+      s_t[b][3][r * kDirThreads + tid] = v[r].w;
+    }
+  };
+  fetch(0);
+  stage(0);
+  __syncthreads();
+  const f2 e2 = f2_make(a.eps2, a.eps2);
+  for (int t = 0; t < nt; ++t) {
+    if (t + 1 < nt) fetch(t + 1);
+    // this half's share of the tile, in whole steps of 8 (zero mass past the end)
+    const int cnt = (int)imin64(kDirTile, j1 - j0 - (int64_t)t * kDirTile);
+    const int mid = ((cnt + 1) / 2 + 7) & ~7;
+    const int jb = half ? mid : 0, je = half ? ((cnt + 7) & ~7) : mid;
+    f2 ax[I], ay[I], az[I];
+#pragma unroll
+    for (int q = 0; q < I; ++q) ax[q] = ay[q] = az[q] = f2_make(0.f, 0.f);
+    pair_sum<I, ZERO_SOFT>(s_t[t & 1], jb, je, xi, yi, zi, e2, ax, ay, az);
+#pragma unroll
+    for (int q = 0; q < I; ++q) {
+      fold<COMP>(f2_sum(ax[q]), sx[q], ex[q]);
+      fold<COMP>(f2_sum(ay[q]), sy[q], ey[q]);
+      fold<COMP>(f2_sum(az[q]), sz[q], ez[q]);
+    }
+    if (t + 1 < nt) stage((t + 1) & 1);
+    __syncthreads();
+  }
+  // add the second half's sums to the first's
+  float* s_r = &s_t[0][0][0];  // 6 rows of T floats (I = 2: 6 of the 16 KB)
+  static_assert(6 * T <= 2 * 4 * kDirTile, "reduction rows fit the tile buffers");
+  if (half) {
+#pragma unroll
+    for (int q = 0; q < I; ++q) {
+      const int o = tl + q * kDirHalf;
+      s_r[o] = sx[q];
+      s_r[T + o] = sy[q];
+      s_r[2 * T + o] = sz[q];
+      s_r[3 * T + o] = ex[q];
+      s_r[4 * T + o] = ey[q];
+      s_r[5 * T + o] = ez[q];
+    }
+  }
+  __syncthreads();
+  if (!half) {
+#pragma unroll
+    for (int q = 0; q < I; ++q) {
+      const int o = tl + q * kDirHalf;
+      const int64_t i = tgt_base + o;
+      fold<COMP>(s_r[o], sx[q], ex[q]);
+      fold<COMP>(s_r[T + o], sy[q], ey[q]);
+      fold<COMP>(s_r[2 * T + o], sz[q], ez[q]);
+      const float rx = sx[q] + (ex[q] + s_r[3 * T + o]), ry = sy[q] + (ey[q] + s_r[4 * T + o]),
+                  rz = sz[q] + (ez[q] + s_r[5 * T + o]);
+      if (a.splits > 1) {
+        a.partial[(int64_t)blockIdx.y * a.n_tgt_pad + i] = make_float4(rx, ry, rz, 0.f);
+      } else if (i < a.n_tgt) {
+        a.out_x[i] = a.G * rx;
+        a.out_y[i] = a.G * ry;
+        a.out_z[i] = a.G * rz;
+      }
+    }
+  }
+  if (a.splits == 1) return;
+  // the last CTA of this target block adds the partial sums
+  __threadfence();
+  __syncthreads();
+  if (tid == 0) s_last = atomicAdd(&a.ticket[blockIdx.x], 1u) == (uint32_t)(a.splits - 1);
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  if (tid == 0) a.ticket[blockIdx.x] = 0;  // ready for the next launch
+  for (int o = tid; o < T; o += kDirThreads) {
+    const int64_t i = tgt_base + o;
+    if (i >= a.n_tgt) break;
+    float rx = 0.f, ry = 0.f, rz = 0.f, fx = 0.f, fy = 0.f, fz = 0.f;
+#pragma unroll 4
+    for (int s = 0; s < a.splits; ++s) {
+      const float4 p = __ldcg(&a.partial[(int64_t)s * a.n_tgt_pad + i]);
+      fold<true>(p.x, rx, fx);
+      fold<true>(p.y, ry, fy);
+      fold<true>(p.z, rz, fz);
+    }
+    a.out_x[i] = a.G * (rx + fx);
+    a.out_y[i] = a.G * (ry + fy);
+    a.out_z[i] = a.G * (rz + fz);
   }
 }
 
-// Sum the j-split partials in split order (deterministic), then scale by G.
-__global__ void direct_reduce_kernel(const float4* __restrict__ partial, int splits,
-                                     int64_t n_tgt, int64_t n_tgt_pad, float G,
-                                     float* __restrict__ ox, float* __restrict__ oy,
-                                     float* __restrict__ oz) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n_tgt;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    float sx = 0.f, sy = 0.f, sz = 0.f, ex = 0.f, ey = 0.f, ez = 0.f, e;
-    for (int s = 0; s < splits; ++s) {
-      float4 p = partial[(int64_t)s * n_tgt_pad + i];
-      sx = two_sum(sx, p.x, e);
-      ex += e;
-      sy = two_sum(sy, p.y, e);
-      ey += e;
-      sz = two_sum(sz, p.z, e);
-      ez += e;
+// Targets per thread and source runs for n bodies: the pair with the least
+// estimated time, in SM clocks.  The busiest SM sums k CTAs at 8.65 (one
+// target per thread) or 8.95 interactions per clock together, 7.9 when it has
+// only one (81, 84 and 74 % of its 128 lanes / 12 operations); each round of resident CTAs costs kCtaClocks
+// to start (targets, first tile, half sums), and each run a load per target
+// at the end.  Measured, us per launch: N = 1,024 6.3 (one target per thread,
+// 8 runs; 10.4 unsplit), N = 8,192 32.9 (two, 9 runs; 35 with one target and 4
+// runs), N = 131,072 6,262 (two, 19 runs; 6,417 with one); four targets per
+// thread were nowhere faster (6,333 at N = 131,072).
+DirectPlan plan_direct(int64_t n, int max_splits) {
+  constexpr double kCtaClocks = 3000.0, kRunClocks = 60.0;
+  n = std::max<int64_t>(n, 1);
+  const int64_t sms = num_sms();
+  DirectPlan best;
+  double best_t = 1e300;
+  for (int I = 1; I <= 2; ++I) {
+    const int64_t T = (int64_t)kDirHalf * I, blocks = ceil_div(n, T);
+    const int64_t s_max = std::max<int64_t>(
+        1, std::min<int64_t>({ceil_div(n, 32), (int64_t)max_splits, ceil_div(16384, blocks)}));
+    for (int64_t s = 1; s <= s_max; ++s) {
+      const int64_t jper = ceil_div(ceil_div(n, s), 16) * 16;
+      if (ceil_div(n, jper) != s) continue;
+      const int64_t k = ceil_div(blocks * s, sms);
+      const double t = kCtaClocks * (double)ceil_div(k, 3) +
+                       (double)k * (double)(jper * T) / (k == 1 ? 7.9 : I == 1 ? 8.65 : 8.95) +
+                       (s > 1 ? 2000.0 + kRunClocks * (double)s : 0.0);
+      if (t < 0.99 * best_t) {
+        best_t = t;
+        best.per_thread = I;
+        best.i_blocks = blocks;
+        best.n_tgt_pad = blocks * T;
+        best.splits = (int)s;
+        best.jper = jper;
+      }
     }
-    ox[i] = G * (sx + ex);
-    oy[i] = G * (sy + ey);
-    oz[i] = G * (sz + ez);
   }
+  return best;
 }
 
-template <int I, bool PAIRED, bool COMP, bool ZS>
-static void launch_one(const DirectArgs& a, dim3 grid, cudaStream_t st) {
-  direct_kernel<I, PAIRED, COMP, ZS><<<grid, kDirThreads, 0, st>>>(a);
+template <int I, bool SOA>
+static void launch_one(const DirectArgs& a, dim3 grid, bool comp, bool zs, cudaStream_t st) {
+  if (zs)
+    comp ? direct_kernel<I, true, true, SOA><<<grid, kDirThreads, 0, st>>>(a)
+         : direct_kernel<I, false, true, SOA><<<grid, kDirThreads, 0, st>>>(a);
+  else
+    comp ? direct_kernel<I, true, false, SOA><<<grid, kDirThreads, 0, st>>>(a)
+         : direct_kernel<I, false, false, SOA><<<grid, kDirThreads, 0, st>>>(a);
   NBGB_LAUNCH_CHECK();
 }
 
-template <int I, bool PAIRED>
-static int occupancy_of() {
-  int blocks = 0;
-  NBGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-      &blocks, direct_kernel<I, PAIRED, true, false>, kDirThreads, 0));
-  return blocks > 0 ? blocks : 1;
-}
-
-DirectPlan plan_direct(int64_t n_src, int64_t n_tgt, DirectVariant v) {
-  DirectPlan p;
-  p.variant = v;
-  p.targets_per_cta = kDirThreads * direct_targets_per_thread(v);
-  p.n_tiles = ceil_div(std::max<int64_t>(n_src, 1), kDirTile);
-  p.n_src_pad = p.n_tiles * kDirTile;
-  p.i_blocks = ceil_div(std::max<int64_t>(n_tgt, 1), p.targets_per_cta);
-  p.n_tgt_pad = p.i_blocks * p.targets_per_cta;
-  int occ = (v == DirectVariant::kPaired8) ? occupancy_of<8, true>() : occupancy_of<4, false>();
-  int64_t slots = (int64_t)num_sms() * occ;
-  // Choose the j-split so that i_blocks * splits fills whole waves of the
-  // resident CTA slots (every CTA does the same work), with >= 4 tiles each.
-  int64_t max_split = std::max<int64_t>(1, std::min<int64_t>(p.n_tiles / 4, 128));
-  int best = 1;
-  double best_eff = -1.0;
-  for (int64_t s = 1; s <= max_split; ++s) {
-    int64_t items = p.i_blocks * s;
-    double waves = (double)items / (double)slots;
-    double eff = waves / std::ceil(waves);
-    // Prefer fewer splits unless the efficiency gain is material.
-    if (eff > best_eff + 0.02) {
-      best_eff = eff;
-      best = (int)s;
-    }
-    if (eff >= 0.97) break;
-  }
-  p.splits = best;
-  p.tiles_per_split = ceil_div(p.n_tiles, p.splits);
-  p.splits = (int)ceil_div(p.n_tiles, p.tiles_per_split);
-  return p;
-}
-
-int direct_targets_per_thread(DirectVariant v) {
-  return v == DirectVariant::kPaired8 ? 8 : 4;
-}
-
-void launch_direct(const DirectPlan& p, const float4* src, const float4* tgt, int64_t n_tgt,
-                   float G, float eps2, bool compensated, float4* partial, float* ox, float* oy,
-                   float* oz, uint32_t* err, cudaStream_t st) {
-  if (n_tgt <= 0) return;
-  DirectArgs a;
-  a.src = src;
-  a.tgt = tgt;
-  a.n_tgt = n_tgt;
+template <bool SOA>
+static void launch_direct_any(const DirectPlan& p, DirectArgs& a, bool comp, cudaStream_t st) {
   a.n_tgt_pad = p.n_tgt_pad;
-  a.n_tiles = p.n_tiles;
-  a.tiles_per_split = p.tiles_per_split;
+  a.jper = p.jper;
+  a.splits = p.splits;
+  const dim3 grid((unsigned)p.i_blocks, (unsigned)p.splits);
+  const bool zs = !(a.eps2 > 0.f);
+  if (p.per_thread == 1)
+    launch_one<1, SOA>(a, grid, comp, zs, st);
+  else
+    launch_one<2, SOA>(a, grid, comp, zs, st);
+}
+
+void launch_direct(const DirectPlan& p, const DirectSource& src, int64_t n, float G, float eps2,
+                   bool compensated, float4* partial, uint32_t* ticket, float* ox, float* oy,
+                   float* oz, cudaStream_t st) {
+  if (n <= 0) return;
+  DirectArgs a{};
+  a.src = src.pm;
+  a.sx = src.x;
+  a.sy = src.y;
+  a.sz = src.z;
+  a.sm = src.m;
+  a.n_src = n;
+  a.n_tgt = n;
   a.eps2 = eps2;
   a.G = G;
-  a.partial = (p.splits > 1) ? partial : nullptr;
+  a.partial = partial;
+  a.ticket = ticket;
   a.out_x = ox;
   a.out_y = oy;
   a.out_z = oz;
-  a.err = err;
-  dim3 grid((unsigned)p.i_blocks, (unsigned)p.splits);
-  const bool zs = !(eps2 > 0.f);
-  if (p.variant == DirectVariant::kPaired8) {
-    if (zs) {
-      compensated ? launch_one<8, true, true, true>(a, grid, st)
-                  : launch_one<8, true, false, true>(a, grid, st);
-    } else {
-      compensated ? launch_one<8, true, true, false>(a, grid, st)
-                  : launch_one<8, true, false, false>(a, grid, st);
-    }
-  } else {
-    if (zs) {
-      compensated ? launch_one<4, false, true, true>(a, grid, st)
-                  : launch_one<4, false, false, true>(a, grid, st);
-    } else {
-      compensated ? launch_one<4, false, true, false>(a, grid, st)
-                  : launch_one<4, false, false, false>(a, grid, st);
-    }
-  }
-  if (p.splits > 1) {
-    int threads = 256;
-    int64_t blocks = std::min<int64_t>(ceil_div(n_tgt, threads), (int64_t)num_sms() * 8);
-    direct_reduce_kernel<<<(unsigned)blocks, threads, 0, st>>>(partial, p.splits, n_tgt,
-                                                               p.n_tgt_pad, G, ox, oy, oz);
-    NBGB_LAUNCH_CHECK();
-  }
+  if (src.pm)
+    launch_direct_any<false>(p, a, compensated, st);
+  else
+    launch_direct_any<true>(p, a, compensated, st);
 }
 
 // ---------------------------------------------------------------------------

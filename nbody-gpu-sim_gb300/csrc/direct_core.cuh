@@ -1,8 +1,8 @@
-// direct_core.cuh -- the direct-sum tile engine shared by the one-system
-// kernel (direct.cu) and the ensemble work-queue kernel (ensemble.cu).
+// direct_core.cuh -- the direct-sum tile engine of the ensemble work-queue
+// kernel (ensemble.cu).
 //
 // One CTA of THREADS threads computes THREADS*I targets against a run of
-// kDirTile-body j-tiles that the bulk-copy engine streams into a kDirStages
+// kRingTile-body j-tiles that the bulk-copy engine streams into a kRingStages
 // ring of shared-memory buffers (cp.async.bulk + mbarrier).  The ring state
 // (barrier phases) lives across calls, so a persistent CTA can process many
 // work items without re-initialising barriers.
@@ -13,15 +13,18 @@
 
 namespace nbgb {
 
+constexpr int kRingTile = 256;   // bodies per shared-memory j-tile (4 KB)
+constexpr int kRingStages = 3;   // bulk-copy pipeline depth
+
 struct TileRing {
-  float4 (*buf)[kDirTile];  // [kDirStages][kDirTile] in shared memory
-  uint64_t* bar;            // [kDirStages] mbarriers, count 1
+  float4 (*buf)[kRingTile];  // [kRingStages][kRingTile] in shared memory
+  uint64_t* bar;            // [kRingStages] mbarriers, count 1
   uint32_t consumed;        // tiles consumed so far by this CTA (phase tracking)
 };
 
 __device__ __forceinline__ void ring_init(TileRing& r) {
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kDirStages; ++s) mbar_init(&r.bar[s], 1);
+    for (int s = 0; s < kRingStages; ++s) mbar_init(&r.bar[s], 1);
     fence_barrier_init();
   }
   __syncthreads();
@@ -29,22 +32,22 @@ __device__ __forceinline__ void ring_init(TileRing& r) {
 }
 
 // Sums, for I targets per thread, the contributions of tiles [0, nt) of
-// `src` (each kDirTile float4 (x,y,z,m), zero-mass padded).  Returns false
+// `src` (each kRingTile float4 (x,y,z,m), zero-mass padded).  Returns false
 // if a bounded wait ran out (the error word is set; all threads agree).
 template <int THREADS, int I, bool PAIRED, bool COMP, bool ZERO_SOFT>
 __device__ __forceinline__ bool direct_tiles(TileRing& ring, const float4* __restrict__ src, int nt,
                                              const float (&xi)[I], const float (&yi)[I],
                                              const float (&zi)[I], float eps2, float (&sx)[I],
                                              float (&sy)[I], float (&sz)[I], uint32_t* err) {
-  constexpr uint32_t kBytes = kDirTile * sizeof(float4);
+  constexpr uint32_t kBytes = kRingTile * sizeof(float4);
   const int tid = threadIdx.x;
   const uint32_t c0 = ring.consumed;
   if (tid == 0) {
-    for (int j = 0; j < kDirStages && j < nt; ++j) {
-      const int s = (int)((c0 + j) % kDirStages);
+    for (int j = 0; j < kRingStages && j < nt; ++j) {
+      const int s = (int)((c0 + j) % kRingStages);
       fence_proxy_async_smem();
       mbar_arrive_expect_tx(&ring.bar[s], kBytes);
-      bulk_g2s(ring.buf[s], src + (int64_t)j * kDirTile, kBytes, &ring.bar[s]);
+      bulk_g2s(ring.buf[s], src + (int64_t)j * kRingTile, kBytes, &ring.bar[s]);
     }
   }
   float ex[I], ey[I], ez[I];
@@ -57,8 +60,8 @@ __device__ __forceinline__ bool direct_tiles(TileRing& ring, const float4* __res
   int t = 0;
   for (; t < nt; ++t) {
     const uint32_t c = c0 + (uint32_t)t;
-    const int s = (int)(c % kDirStages);
-    const uint32_t parity = (c / kDirStages) & 1u;
+    const int s = (int)(c % kRingStages);
+    const uint32_t parity = (c / kRingStages) & 1u;
     if (!bad && !mbar_wait(&ring.bar[s], parity, err)) bad = true;
     if (!bad) {
       const float4* __restrict__ tile = ring.buf[s];
@@ -77,7 +80,7 @@ __device__ __forceinline__ bool direct_tiles(TileRing& ring, const float4* __res
         }
         const f2 e2 = f2_make(eps2, eps2);
 #pragma unroll 32
-        for (int k = 0; k < kDirTile; ++k) {
+        for (int k = 0; k < kRingTile; ++k) {
           const float4 pj = tile[k];
           const f2 xj = f2_make(pj.x, pj.x), yj = f2_make(pj.y, pj.y), zj = f2_make(pj.z, pj.z);
           const f2 mj = f2_make(pj.w, pj.w);
@@ -109,7 +112,7 @@ __device__ __forceinline__ bool direct_tiles(TileRing& ring, const float4* __res
         }
       } else {
 #pragma unroll 4
-        for (int k = 0; k < kDirTile; ++k) {
+        for (int k = 0; k < kRingTile; ++k) {
           const float4 pj = tile[k];
 #pragma unroll
           for (int q = 0; q < I; ++q) {
@@ -147,18 +150,18 @@ __device__ __forceinline__ bool direct_tiles(TileRing& ring, const float4* __res
       bad = true;
       break;
     }
-    if (tid == 0 && t + kDirStages < nt) {
+    if (tid == 0 && t + kRingStages < nt) {
       fence_proxy_async_smem();
       mbar_arrive_expect_tx(&ring.bar[s], kBytes);
-      bulk_g2s(ring.buf[s], src + (int64_t)(t + kDirStages) * kDirTile, kBytes, &ring.bar[s]);
+      bulk_g2s(ring.buf[s], src + (int64_t)(t + kRingStages) * kRingTile, kBytes, &ring.bar[s]);
     }
   }
   if (bad) {
     // drain (bounded) the copies still in flight on every stage
     if (tid == 0) {
-      for (int j = t; j < nt && j < t + kDirStages; ++j) {
+      for (int j = t; j < nt && j < t + kRingStages; ++j) {
         const uint32_t c = c0 + (uint32_t)j;
-        mbar_wait(&ring.bar[c % kDirStages], (c / kDirStages) & 1u, nullptr, 1u << 16);
+        mbar_wait(&ring.bar[c % kRingStages], (c / kRingStages) & 1u, nullptr, 1u << 16);
       }
     }
     return false;

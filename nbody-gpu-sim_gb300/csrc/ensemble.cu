@@ -41,7 +41,7 @@
 
 namespace nbgb {
 
-constexpr int64_t kChunk = 256;  // arena granularity (== kDirTile)
+constexpr int64_t kChunk = 256;  // arena granularity (== kRingTile)
 constexpr int kTimingRing = 8;   // direct-kernel event pairs in flight
 // The group walk's largest group in the batched build: fixed, so that a
 // system's lists (and results) do not depend on what else is resident; 64
@@ -134,8 +134,8 @@ __global__ void __launch_bounds__(THREADS) ens_direct_kernel(const DirectItem* _
                                                              float* __restrict__ ay,
                                                              float* __restrict__ az, float eps2,
                                                              float G, uint32_t* err) {
-  __shared__ alignas(128) float4 s_j[kDirStages][kDirTile];
-  __shared__ alignas(8) uint64_t s_bar[kDirStages];
+  __shared__ alignas(128) float4 s_j[kRingStages][kRingTile];
+  __shared__ alignas(8) uint64_t s_bar[kRingStages];
   __shared__ int s_item;
   TileRing ring{s_j, s_bar, 0};
   ring_init(ring);
@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(THREADS) ens_direct_kernel(const DirectItem* _
       zi[q] = p.z;
     }
     float sx[I], sy[I], sz[I];
-    const int nt = (int)ceil_div(w.n, kDirTile);
+    const int nt = (int)ceil_div(w.n, kRingTile);
     if (!direct_tiles<THREADS, I, PAIRED, true, false>(ring, pm + w.off, nt, xi, yi, zi, eps2, sx,
                                                        sy, sz, err))
       return;

@@ -9,48 +9,52 @@
 namespace nbgb {
 
 // ----------------------------------------------------------------- direct --
-constexpr int kDirThreads = 128;  // threads per CTA of the direct kernel
-constexpr int kDirTile = 256;     // bodies per shared-memory j-tile (4 KB)
-constexpr int kDirStages = 3;     // bulk-copy pipeline depth
-
-enum class DirectVariant : int {
-  kScalar4 = 0,  // 4 targets/thread, scalar FP32 (12 FP32 ops + 1 MUFU per pair)
-  kPaired8 = 1,  // 8 targets/thread, packed f32x2 arithmetic
-};
+constexpr int kDirThreads = 256;  // threads per CTA of the direct kernel
+constexpr int kDirHalf = 128;     // threads per half: a half sums its own sources
+constexpr int kDirTile = 512;     // sources per shared-memory tile (8 KB)
 
 struct DirectArgs {
-  const float4* src;  // padded sources (x, y, z, m)
-  const float4* tgt;  // targets (x, y, z, .)
-  int64_t n_tgt;
+  const float4* src;                              // packed sources (x, y, z, m), or
+  const float *sx, *sy, *sz, *sm;                 // the caller's SoA arrays
+  int64_t n_src;
+  int64_t n_tgt;                                  // the first n_tgt sources are the targets
   int64_t n_tgt_pad;
-  int64_t n_tiles;
-  int64_t tiles_per_split;
+  int64_t jper;                                   // sources per run (CTA)
+  int splits;                                     // runs
   float eps2;
   float G;
-  float4* partial;  // [splits][n_tgt_pad] when splits > 1, else null
+  float4* partial;                                // [splits][n_tgt_pad] when splits > 1
+  uint32_t* ticket;                               // per target block, zero between launches
   float* out_x;
   float* out_y;
   float* out_z;
-  uint32_t* err;
+};
+
+// Bodies of a direct sum: pm (packed), or the SoA arrays when pm is null.
+struct DirectSource {
+  const float4* pm;
+  const float *x, *y, *z, *m;
 };
 
 struct DirectPlan {
-  DirectVariant variant = DirectVariant::kScalar4;
-  int targets_per_cta = 0;
-  int64_t n_tiles = 0;
-  int64_t n_src_pad = 0;  // sources must be padded (zero mass) to this length
-  int64_t i_blocks = 0;
+  int per_thread = 1;     // targets per thread (1 or 2)
+  int64_t i_blocks = 0;   // target blocks of kDirHalf * per_thread
   int64_t n_tgt_pad = 0;
-  int splits = 1;
-  int64_t tiles_per_split = 0;
-  size_t partial_bytes() const { return splits > 1 ? (size_t)splits * n_tgt_pad * 16 : 0; }
+  int splits = 1;         // source runs
+  int64_t jper = 0;       // sources per run, a multiple of 16
 };
 
-int direct_targets_per_thread(DirectVariant v);
-DirectPlan plan_direct(int64_t n_src, int64_t n_tgt, DirectVariant v);
-void launch_direct(const DirectPlan& p, const float4* src, const float4* tgt, int64_t n_tgt,
-                   float G, float eps2, bool compensated, float4* partial, float* ox, float* oy,
-                   float* oz, uint32_t* err, cudaStream_t st);
+// Whether a direct sum may read the caller's arrays while it writes the
+// accelerations (no overlap).
+bool direct_from_soa(const nbgb_particle_data* d);
+constexpr int kDirMaxSplits = 128;
+DirectPlan plan_direct(int64_t n, int max_splits = kDirMaxSplits);
+// Forces on all n bodies of src.  With p.splits > 1: partial holds
+// splits * n_tgt_pad entries, ticket i_blocks counters that are zero before
+// the launch and zero again after it.
+void launch_direct(const DirectPlan& p, const DirectSource& src, int64_t n, float G, float eps2,
+                   bool compensated, float4* partial, uint32_t* ticket, float* ox, float* oy,
+                   float* oz, cudaStream_t st);
 void launch_pack_soa(const float* x, const float* y, const float* z, const float* m, int64_t n,
                      int64_t n_pad, float4* out, cudaStream_t st);
 

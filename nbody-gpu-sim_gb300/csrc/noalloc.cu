@@ -19,8 +19,8 @@
 // device; a warm-up call with count 0 does the reservation and nothing else.
 //
 // Limits: at most kNoAllocMaxBodies bodies per call, direct sum only; not
-// callable while its stream is being captured into a CUDA graph (it reads the
-// device error word back and waits for the stream); cudaDeviceReset after
+// callable while its stream is being captured into a CUDA graph (it waits for
+// the stream); cudaDeviceReset after
 // the first call on a device is not supported (the resolved addresses are
 // kept per device).  All calls share the same scratch arrays: calls whose
 // work overlaps on the GPU (different streams, or different host threads,
@@ -39,17 +39,18 @@ constexpr int64_t kNoAllocMaxBodies = 65536;  // multiple of the j-tile (256)
 constexpr int kNoAllocMaxSplits = 8;           // j-splits of the partial sums
 
 // Scratch (global memory beyond the caller's inputs and outputs):
-//   packed (x, y, z, m) bodies, zero-mass padded      1 MiB
-//   per-split partial accelerations                   8 MiB
-//   device error word (bounded-wait timeouts)         4 B
+//   packed (x, y, z, m) bodies (only for calls whose
+//   accelerations share memory with an input)         1 MiB
+//   per-run partial accelerations                     8 MiB
+//   finished-run counters per target block            2 KiB
 static __device__ __align__(256) float4 g_noalloc_bodies[kNoAllocMaxBodies];
 static __device__ __align__(256) float4 g_noalloc_partial[kNoAllocMaxSplits * kNoAllocMaxBodies];
-static __device__ __align__(256) uint32_t g_noalloc_err[64];
+static __device__ __align__(256) uint32_t g_noalloc_ticket[kNoAllocMaxBodies / kDirHalf];
 
 struct NoAllocScratch {
   float4* bodies = nullptr;
   float4* partial = nullptr;
-  uint32_t* err = nullptr;
+  uint32_t* ticket = nullptr;
   bool ready = false;
 };
 
@@ -69,7 +70,7 @@ static NoAllocScratch noalloc_scratch(int dev) {
     if (e == cudaSuccess)
       e = cudaGetSymbolAddress(reinterpret_cast<void**>(&s.partial), g_noalloc_partial);
     if (e == cudaSuccess)
-      e = cudaGetSymbolAddress(reinterpret_cast<void**>(&s.err), g_noalloc_err);
+      e = cudaGetSymbolAddress(reinterpret_cast<void**>(&s.ticket), g_noalloc_ticket);
     if (e != cudaSuccess) {
       cudaGetLastError();
       s = NoAllocScratch{};
@@ -82,16 +83,11 @@ static NoAllocScratch noalloc_scratch(int dev) {
   return s;
 }
 
-// The direct plan with its j-splits capped to the static partial-sum array.
-// `planned` receives the split count the regular planner chose.
+// The direct plan with its source runs capped to the static partial-sum array.
+// `planned` receives the run count the regular planner chooses.
 static DirectPlan noalloc_plan(int64_t n, int* planned) {
-  DirectPlan p = plan_direct(n, n, DirectVariant::kPaired8);
-  if (planned) *planned = p.splits;
-  if (p.splits > kNoAllocMaxSplits) {
-    p.tiles_per_split = ceil_div(p.n_tiles, kNoAllocMaxSplits);
-    p.splits = (int)ceil_div(p.n_tiles, p.tiles_per_split);
-  }
-  return p;
+  if (planned) *planned = plan_direct(n).splits;
+  return plan_direct(n, kNoAllocMaxSplits);
 }
 
 template <typename F>
@@ -145,20 +141,19 @@ extern "C" nbgb_status nbgb_compute_forces_direct_noalloc(const nbgb_particle_da
     // reserves) the scratch; a count of 0 stops right after that
     const NoAllocScratch s = noalloc_scratch(dev);
     if (n == 0) return;
-    // The error word keeps the previous call's value: clear it first.
-    NBGB_CUDA(cudaMemsetAsync(s.err, 0, sizeof(uint32_t), cs));
     const DirectPlan p = noalloc_plan(n, nullptr);
-    // Every padded body slot and every partial read below is rewritten by
-    // this call, so nothing else of the previous call's contents is used.
-    launch_pack_soa(d->pos_x, d->pos_y, d->pos_z, d->mass, n, p.n_src_pad, s.bodies, cs);
-    launch_direct(p, s.bodies, s.bodies, n, G, softening * softening, true, s.partial, d->acc_x,
-                  d->acc_y, d->acc_z, s.err, cs);
-    uint32_t bits = 0;
-    NBGB_CUDA(cudaMemcpyAsync(&bits, s.err, sizeof bits, cudaMemcpyDeviceToHost, cs));
+    // every partial sum read is rewritten by this call, and the counters start
+    // at zero, so nothing of a previous call's contents is used
+    if (p.splits > 1)
+      NBGB_CUDA(cudaMemsetAsync(s.ticket, 0, (size_t)p.i_blocks * sizeof(uint32_t), cs));
+    DirectSource src{nullptr, d->pos_x, d->pos_y, d->pos_z, d->mass};
+    if (!direct_from_soa(d)) {
+      launch_pack_soa(d->pos_x, d->pos_y, d->pos_z, d->mass, n, n, s.bodies, cs);
+      src = DirectSource{s.bodies, nullptr, nullptr, nullptr, nullptr};
+    }
+    launch_direct(p, src, n, G, softening * softening, true, s.partial, s.ticket, d->acc_x,
+                  d->acc_y, d->acc_z, cs);
     NBGB_CUDA(cudaStreamSynchronize(cs));
-    if (bits)
-      fail(NBGB_ERR_DEVICE_TIMEOUT,
-           "CUDA Error: a bounded device wait of the direct kernel ran out of iterations");
   });
 }
 
@@ -170,7 +165,7 @@ extern "C" nbgb_status nbgb_selftest_noalloc_plan(int64_t count, int32_t* planne
     int planned = 0;
     const DirectPlan p = noalloc_plan(count, &planned);
     if ((int64_t)p.splits * p.n_tgt_pad > kNoAllocMaxSplits * kNoAllocMaxBodies ||
-        p.n_src_pad > kNoAllocMaxBodies)
+        p.i_blocks > kNoAllocMaxBodies / kDirHalf)
       fail(NBGB_ERR_OVERFLOW, "the capped plan does not fit the static scratch");
     if (planned_splits) *planned_splits = planned;
     if (used_splits) *used_splits = p.splits;

@@ -77,6 +77,38 @@ struct HostPinned {
   }
 };
 
+// A calculator's device error word, in mapped pinned host memory: kernels OR
+// bits into it (only when something went wrong), and the host reads it after
+// a stream synchronisation without a copy of its own.
+struct ErrorWord {
+  uint32_t* host = nullptr;
+  uint32_t* dev = nullptr;
+  ErrorWord() = default;
+  ErrorWord(const ErrorWord&) = delete;
+  ErrorWord& operator=(const ErrorWord&) = delete;
+  ~ErrorWord() {
+    if (host) cudaFreeHost(host);
+  }
+  uint32_t* ensure(size_t) {
+    if (!dev) {
+      if (!host) {
+        NBGB_CUDA(cudaHostAlloc(&host, sizeof(uint32_t), cudaHostAllocMapped));
+        *host = 0;
+      }
+      NBGB_CUDA(cudaHostGetDevicePointer(&dev, host, 0));
+    }
+    return dev;
+  }
+  // The bits set so far, cleared; the stream must be idle.
+  uint32_t take() {
+    if (!host) return 0;
+    volatile uint32_t* w = host;
+    const uint32_t bits = *w;
+    if (bits) *w = 0;
+    return bits;
+  }
+};
+
 // Per-stage device times of a calculator (NBGB_FLAG_STAGE_TIMINGS): an event
 // is recorded on the calculator's stream where each stage of a force
 // evaluation begins and where the evaluation ends; harvest() waits for the
@@ -132,14 +164,13 @@ struct nbgb_calculator {
   cudaStream_t stream = nullptr;
   bool own_stream = false;
   int device = 0;
-  nbgb::DirectVariant variant = nbgb::DirectVariant::kScalar4;
 
   nbgb::DevBuf<float4> pm;        // packed (x, y, z, m) input of the last drop-in call
-  nbgb::DevBuf<float4> partial;   // direct j-split partials
-  nbgb::DevBuf<uint32_t> err;     // device error word
+  nbgb::DevBuf<float4> partial;   // direct: partial sums of the source runs
+  nbgb::DevBuf<uint32_t> ticket;  // direct: finished runs per target block (zero between calls)
+  nbgb::ErrorWord err;            // device error word
   nbgb::DevBuf<int32_t> counts;   // per-target interaction / neighbour counts
   nbgb::DevBuf<double> red;       // reduction partials
-  nbgb::HostPinned<uint32_t> h_err;
   nbgb::HostPinned<double> h_red;
   int64_t last_n = 0;
 
@@ -183,8 +214,6 @@ void forces_packed(nbgb_calculator* c, const float4* pm, int64_t n, float* ax, f
 void bh_forces(nbgb_calculator* c, const float4* pm, int64_t n, float* ax, float* ay, float* az);
 void hash_forces(nbgb_calculator* c, const float4* pm, int64_t n, float* ax, float* ay,
                  float* az);
-// Sources padded for the direct kernel: returns the padded length.
-int64_t direct_pad(int64_t n);
 // Wait for the calculator's stream and turn device error bits into an Error.
 void check_device_errors(nbgb_calculator* c);
 // Record msg as this thread's nbgb_last_error() text; returns s.
