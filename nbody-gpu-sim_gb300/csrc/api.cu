@@ -277,10 +277,34 @@ void nbgb::system_sync_velocity(nbgb_system* s) {
   s->pending_half = false;
 }
 
+// A small direct-sum system: its steps, and its a(0), run in steps.cu.
+static bool system_in_one_launch(const nbgb_system* s) {
+  return !s->fp64 && s->calc->method == NBGB_DIRECT_N2 && direct_small_fit(s->n);
+}
+
+static void system_small_steps(nbgb_system* s, int32_t steps, double kick0, double h) {
+  nbgb_calculator* c = s->calc;
+  const float eps = c->params.softening;
+  const StateArrays a{s->x.ptr,  s->y.ptr,  s->z.ptr,  s->vx.ptr, s->vy.ptr,
+                      s->vz.ptr, s->ax.ptr, s->ay.ptr, s->az.ptr, s->pm.ptr};
+  float4* ex = s->exch.ensure((size_t)2 * s->n);
+  if (!s->exch_ctr.ptr)
+    NBGB_CUDA(cudaMemsetAsync(s->exch_ctr.ensure(2), 0, 2 * sizeof(uint32_t), c->stream));
+  StageTimer* t = stage_timer(c);
+  if (t) t->st = c->stream;
+  stage_mark(t, "direct.forces");
+  launch_direct_steps(a, s->n, steps, kick0, h, h, eps * eps, c->params.G,
+                      (c->params.flags & NBGB_FLAG_COMPENSATED) != 0, ex, s->exch_ctr.ptr,
+                      c->err.ensure(1), c->stream);
+  if (t) t->end();
+}
+
 // Forces at the current state into the system's acceleration arrays.
 static void system_forces(nbgb_system* s) {
   nbgb_calculator* c = s->calc;
-  if (s->fp64) {
+  if (system_in_one_launch(s)) {
+    system_small_steps(s, 0, 0.0, 0.0);
+  } else if (s->fp64) {
     const double eps = (double)c->params.softening;
     launch_direct_f64_state(s->x.ptr, s->y.ptr, s->z.ptr, s->pm.ptr, s->n, (double)c->params.G,
                             eps * eps, s->ax64.ptr, s->ay64.ptr, s->az64.ptr, c->stream);
@@ -653,7 +677,19 @@ nbgb_status nbgb_system_step(nbgb_system* s, float dt, int32_t steps) {
     if (steps < 0) fail(NBGB_ERR_INVALID_ARG, "Validation Error: negative step count");
     nbgb_calculator* c = s->calc;
     const double h = (double)dt;
-    for (int32_t k = 0; k < steps; ++k) {
+    int32_t k = 0;
+    if (system_in_one_launch(s)) {
+      // with stage timings one step per launch, so that the stage counts steps
+      const int32_t most = stage_timer(c) ? 1 : kDirectStepsPerLaunch;
+      while (k < steps) {
+        const int32_t m = std::min(steps - k, most);
+        system_small_steps(s, m, s->pending_half ? 0.5 * s->last_dt + 0.5 * h : 0.5 * h, h);
+        s->pending_half = true;
+        s->last_dt = h;
+        k += m;
+      }
+    }
+    for (; k < steps; ++k) {
       double kick = s->pending_half ? 0.5 * s->last_dt + 0.5 * h : 0.5 * h;
       if (s->fp64)
         launch_kick_drift(s->n, s->x.ptr, s->y.ptr, s->z.ptr, s->vx.ptr, s->vy.ptr, s->vz.ptr,

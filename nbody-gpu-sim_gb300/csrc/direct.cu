@@ -189,15 +189,17 @@ __global__ void __launch_bounds__(kDirThreads, 2) direct_kernel(DirectArgs a) {
 // target per thread) or 8.95 interactions per clock together, 7.9 when it has
 // only one (81, 84 and 74 % of its 128 lanes / 12 operations); each round of resident CTAs costs kCtaClocks
 // to start (targets, first tile, half sums), and each run a load per target
-// at the end.  Measured, us per launch: N = 1,024 6.3 (one target per thread,
-// 8 runs; 10.4 unsplit), N = 8,192 32.9 (two, 9 runs; 35 with one target and 4
-// runs), N = 131,072 6,262 (two, 19 runs; 6,417 with one); four targets per
-// thread were nowhere faster (6,333 at N = 131,072).
+// at the end.  Measured, us per launch: N = 5,000 16.5 (two targets per thread,
+// 15 runs; 42 with one target, unsplit), N = 16,384 107 (two, 19 runs; 130
+// with one target, unsplit), N = 131,072 6,262 (two, 19 runs; 6,417 with
+// one); four targets per thread were nowhere faster (6,333 at N = 131,072).
+// Small systems go to steps.cu.
 DirectPlan plan_direct(int64_t n, int max_splits) {
   constexpr double kCtaClocks = 3000.0, kRunClocks = 60.0;
   n = std::max<int64_t>(n, 1);
   const int64_t sms = num_sms();
   DirectPlan best;
+  if ((best.small = direct_small_fit(n))) return best;
   double best_t = 1e300;
   for (int I = 1; I <= 2; ++I) {
     const int64_t T = (int64_t)kDirHalf * I, blocks = ceil_div(n, T);
@@ -251,6 +253,10 @@ void launch_direct(const DirectPlan& p, const DirectSource& src, int64_t n, floa
                    bool compensated, float4* partial, uint32_t* ticket, float* ox, float* oy,
                    float* oz, cudaStream_t st) {
   if (n <= 0) return;
+  if (p.small) {
+    launch_direct_small(src, n, G, eps2, compensated, ox, oy, oz, st);
+    return;
+  }
   DirectArgs a{};
   a.src = src.pm;
   a.sx = src.x;

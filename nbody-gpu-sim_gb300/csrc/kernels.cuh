@@ -37,6 +37,7 @@ struct DirectSource {
 };
 
 struct DirectPlan {
+  bool small = false;     // the small-system kernel (one CTA set, no runs)
   int per_thread = 1;     // targets per thread (1 or 2)
   int64_t i_blocks = 0;   // target blocks of kDirHalf * per_thread
   int64_t n_tgt_pad = 0;
@@ -57,6 +58,23 @@ void launch_direct(const DirectPlan& p, const DirectSource& src, int64_t n, floa
                    float* oz, cudaStream_t st);
 void launch_pack_soa(const float* x, const float* y, const float* z, const float* m, int64_t n,
                      int64_t n_pad, float4* out, cudaStream_t st);
+
+// Small systems (steps.cu): the forces of n bodies, or `steps` kick-drift +
+// force steps in one cooperative launch.  exch: 2 n entries; ctr: two
+// counters, zero before and after.
+constexpr int64_t kDirectSmallMaxBodies = 9728;  // 16 bytes per body in shared memory
+constexpr int32_t kDirectStepsPerLaunch = 256;   // bounds one launch's time
+struct StateArrays {
+  double *x, *y, *z, *vx, *vy, *vz;
+  float *ax, *ay, *az;
+  float4* pm;
+};
+bool direct_small_fit(int64_t n);
+void launch_direct_small(const DirectSource& src, int64_t n, float G, float eps2, bool comp,
+                         float* ox, float* oy, float* oz, cudaStream_t st);
+void launch_direct_steps(const StateArrays& s, int64_t n, int32_t steps, double kick0, double kick,
+                         double dt, float eps2, float G, bool comp, float4* exch, uint32_t* ctr,
+                         uint32_t* err, cudaStream_t st);
 
 // Energies: `partials` needs nblocks * 4 doubles; out[0..3] = KE, Px, Py, Pz
 // (kinetic) or out[0] = sum_i m_i phi_i / 2 without G (potential).

@@ -188,6 +188,8 @@ struct nbgb_system {
   nbgb::DevBuf<float> ax, ay, az;
   nbgb::DevBuf<double> ax64, ay64, az64;  // NBGB_FLAG_FP64: accelerations in FP64
   nbgb::DevBuf<float4> pm;
+  nbgb::DevBuf<float4> exch;     // several steps per launch: positions in exchange
+  nbgb::DevBuf<uint32_t> exch_ctr;
   nbgb::DevBuf<double> red;
   nbgb::HostPinned<double> h_red;
   bool fp64 = false;

@@ -23,7 +23,7 @@ def _state(nb, n, seed):
 
 
 @pytest.mark.parametrize("n", [1, 15, 16, 17, 127, 128, 129, 511, 512, 513, 1025, 2431, 2433, 4097,
-                               8191, 9729, 19457, 33000])
+                               4864, 4865, 7296, 7297, 8191, 9728, 9729, 19457, 33000])
 def test_block_run_and_tile_edges(nb, orc, n):
     s = _state(nb, n, 40 + n)
     calc = nb.DirectForceCalculator()
