@@ -769,31 +769,41 @@ nbgb_status nbgb_system_energy(nbgb_system* s, double* ke, double* pe, double mo
     system_sync_velocity(s);
     nbgb_calculator* c = s->calc;
     cudaStream_t st = c->stream;
-    int nb = reduce_blocks(s->n);
-    double* p = s->red.ensure((size_t)nb * 4 + 8);
     double* h = s->h_red.ensure(8);
-    launch_kinetic_f64(s->vx.ptr, s->vy.ptr, s->vz.ptr, s->pm.ptr, s->n, p, nb,
-                       p + (size_t)nb * 4, st);
-    NBGB_CUDA(cudaMemcpyAsync(h, p + (size_t)nb * 4, 4 * sizeof(double), cudaMemcpyDeviceToHost, st));
-    NBGB_CUDA(cudaStreamSynchronize(st));
-    double kin[4] = {h[0], h[1], h[2], h[3]};
-    double pot = 0.0;
-    if (pe) {
-      // FP64 positions and arithmetic (the state the system integrates) up
-      // to 2^18 bodies; above, the O(N^2) FP64 sum would take seconds on
-      // GB300's FP64 pipe, so the FP32 pair terms (Newton-refined rsqrt,
-      // compensated per tile, FP64 totals) are summed instead
-      if (s->n <= kPotentialF64MaxN) {
-        const double eps = (double)c->params.softening;
-        launch_potential_f64(s->x.ptr, s->y.ptr, s->z.ptr, s->pm.ptr, s->n, eps * eps, p, nb,
-                             p + (size_t)nb * 4, st);
-      } else {
+    double kin[4], pot = 0.0;
+    // FP64 positions and arithmetic (the state the system integrates) up to
+    // 2^18 bodies; above, the O(N^2) FP64 sum would take seconds on GB300's
+    // FP64 pipe, so the FP32 pair terms (Newton-refined rsqrt, compensated per
+    // tile, FP64 totals) are summed instead
+    if (pe && s->n <= kPotentialF64MaxN) {
+      const double eps = (double)c->params.softening;
+      if (!s->red_ticket.ptr)
+        NBGB_CUDA(cudaMemsetAsync(s->red_ticket.ensure(1), 0, sizeof(uint32_t), st));
+      double* d_out = nullptr;
+      NBGB_CUDA(cudaHostGetDevicePointer(&d_out, h, 0));
+      launch_energy_f64(EnergyArgs{s->x.ptr, s->y.ptr, s->z.ptr, s->vx.ptr, s->vy.ptr, s->vz.ptr,
+                                   s->pm.ptr, s->n, eps * eps,
+                                   s->red.ensure((size_t)energy_f64_blocks(s->n) * 5),
+                                   s->red_ticket.ptr, d_out},
+                        st);
+      NBGB_CUDA(cudaStreamSynchronize(st));
+      std::copy(h, h + 4, kin);
+      pot = (double)c->params.G * h[4];
+    } else {
+      int nb = reduce_blocks(s->n);
+      double* p = s->red.ensure((size_t)nb * 4 + 8);
+      launch_kinetic_f64(s->vx.ptr, s->vy.ptr, s->vz.ptr, s->pm.ptr, s->n, p, nb,
+                         p + (size_t)nb * 4, st);
+      NBGB_CUDA(cudaMemcpyAsync(h, p + (size_t)nb * 4, 4 * sizeof(double), cudaMemcpyDeviceToHost, st));
+      NBGB_CUDA(cudaStreamSynchronize(st));
+      std::copy(h, h + 4, kin);
+      if (pe) {
         const float eps = c->params.softening;
         launch_potential(s->pm.ptr, s->n, eps * eps, p, nb, p + (size_t)nb * 4, st);
+        NBGB_CUDA(cudaMemcpyAsync(h, p + (size_t)nb * 4, sizeof(double), cudaMemcpyDeviceToHost, st));
+        NBGB_CUDA(cudaStreamSynchronize(st));
+        pot = (double)c->params.G * h[0];
       }
-      NBGB_CUDA(cudaMemcpyAsync(h, p + (size_t)nb * 4, sizeof(double), cudaMemcpyDeviceToHost, st));
-      NBGB_CUDA(cudaStreamSynchronize(st));
-      pot = (double)c->params.G * h[0];
     }
     if (ke) *ke = kin[0];
     if (pe) *pe = pot;

@@ -283,7 +283,7 @@ void launch_direct(const DirectPlan& p, const DirectSource& src, int64_t n, floa
 // ---------------------------------------------------------------------------
 
 // Deterministic two-level reduction of per-thread doubles: block sums go to
-// `partials`, a single block then adds them in order.
+// `partials`, a single block then adds them in a fixed order.
 template <int NV>
 __device__ __forceinline__ void block_reduce_store(double (&v)[NV], double* partials) {
   __shared__ double s_red[32][NV];
@@ -315,17 +315,8 @@ __global__ void finish_reduce_kernel(const double* __restrict__ partials, int nb
   for (int b = threadIdx.x; b < nblocks; b += blockDim.x)
 #pragma unroll
     for (int k = 0; k < NV; ++k) v[k] += partials[(int64_t)b * NV + k];
-  __shared__ double s[NV][256];
-#pragma unroll
-  for (int k = 0; k < NV; ++k) s[k][threadIdx.x] = v[k];
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int k = 0; k < NV; ++k) {
-      double t = 0.0;
-      for (int j = 0; j < (int)blockDim.x; ++j) t += s[k][j];
-      out[k] = t;
-    }
-  }
+  // a tree over the 256 threads (one thread adding 256 values took 9 us each)
+  block_reduce_store<NV>(v, out);
 }
 
 // KE (and optionally momentum) from FP32 SoA velocities.
@@ -422,9 +413,9 @@ void launch_potential(const float4* src, int64_t n, float eps2, double* partials
 }
 
 // ----------------------------------------------- FP64-state kernels --
-// Forces and potential from FP64 positions in FP64 arithmetic: the
-// full-FP64 system variant and the energy of every FP64-state system.
-// 256-body tiles of (x, y, z, m) in shared memory, one target per thread,
+// Forces and energies from FP64 positions in FP64 arithmetic: the full-FP64
+// system variant and the energy of every FP64-state system.  Forces: 256-body
+// tiles of (x, y, z, m) in shared memory, one target per thread,
 // self excluded by index, rsqrt from the CUDA math library.
 __global__ void __launch_bounds__(256) direct_f64_state_kernel(
     const double* __restrict__ x, const double* __restrict__ y, const double* __restrict__ z,
@@ -463,35 +454,98 @@ __global__ void __launch_bounds__(256) direct_f64_state_kernel(
   }
 }
 
-__global__ void __launch_bounds__(256) pe_f64_kernel(const double* __restrict__ x,
-                                                     const double* __restrict__ y,
-                                                     const double* __restrict__ z,
-                                                     const float4* __restrict__ pm, int64_t n,
-                                                     double eps2, double* partials) {
-  __shared__ double4 s_j[256];
-  double acc[1] = {0.0};
-  for (int64_t base = (int64_t)blockIdx.x * 256; base < n; base += (int64_t)gridDim.x * 256) {
-    const int64_t i = base + threadIdx.x;
-    const bool valid = i < n;
-    const double xi = valid ? x[i] : 0.0, yi = valid ? y[i] : 0.0, zi = valid ? z[i] : 0.0;
-    double s = 0.0;
-    for (int64_t c = 0; c < n; c += 256) {
-      __syncthreads();
-      const int64_t j = c + threadIdx.x;
-      s_j[threadIdx.x] = (j < n) ? make_double4(x[j], y[j], z[j], (double)pm[j].w)
-                                 : make_double4(0.0, 0.0, 0.0, 0.0);
-      __syncthreads();
-      const int lim = (int)imin64(256, n - c);
-      for (int k = 0; k < lim; ++k) {
-        if (c + k == i) continue;
-        const double4 q = s_j[k];
-        const double dx = q.x - xi, dy = q.y - yi, dz = q.z - zi;
-        s -= q.w * rsqrt(fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2))));
-      }
-    }
-    if (valid) acc[0] += 0.5 * (double)pm[i].w * s;
+// Reciprocal square root in FP64: an FP32 seed y (relative error below 2^-22)
+// and one third-order step, y + y e (1/2 + 3/8 e) with e = 1 - d y^2 (the
+// binomial series of (1 - e)^(-1/2), remainder 5/16 e^3 < 2^-63); y^2 is exact
+// in FP64.  5 FP64 operations and two conversions.  Outside the seed's safe
+// range (and for zero, infinity and NaN) the math library's rsqrt.
+__device__ __forceinline__ double rsqrt_f64(double d) {
+  const uint32_t hi = (uint32_t)__double2hiint(d);
+  if (hi - 0x38f00000u > 0x0e000000u) return rsqrt(d);  // outside 2^-112 .. 2^112
+  const double y = (double)rsqrt_approx((float)d);
+  const double e = fma(-d, y * y, 1.0);
+  return fma(y * e, fma(0.375, e, 0.5), y);
+}
+
+// Kinetic energy, momentum and potential energy of an FP64-state system in
+// one launch.  PE: every unordered pair once, as 64 x 64 tiles of the upper
+// triangle dealt out to the CTAs (a thread keeps one target of the tile, the
+// sources are read from shared memory).  Bound by the FP64 pipe (2 lanes per
+// clock and SM, 12 operations per pair): small tiles, so that few bodies
+// still reach every SM.  N = 8,191: 6.9 ms as one 256-target CTA per row of
+// ordered pairs (32 CTAs), 0.93 ms now (0.64 at the FP64 rate).
+constexpr int kPeTile = 64;
+
+__global__ void __launch_bounds__(kPeTile) energy_f64_kernel(EnergyArgs a) {
+  __shared__ double4_16a s_j[kPeTile];
+  __shared__ bool s_last;
+  const int tid = threadIdx.x;
+  double v[5] = {0.0, 0.0, 0.0, 0.0, 0.0};  // KE, momentum, PE
+  for (int64_t i = blockIdx.x * (int64_t)kPeTile + tid; i < a.n; i += (int64_t)gridDim.x * kPeTile) {
+    const double p = a.vx[i], q = a.vy[i], r = a.vz[i], m = a.pm[i].w;
+    v[0] += 0.5 * m * (p * p + q * q + r * r);
+    v[1] += m * p;
+    v[2] += m * q;
+    v[3] += m * r;
   }
-  block_reduce_store<1>(acc, partials);
+  const int64_t tiles = ceil_div(a.n, kPeTile), pairs = tiles * (tiles + 1) / 2;
+  for (int64_t t = blockIdx.x; t < pairs; t += gridDim.x) {
+    // row r of the triangle holds the tiles (r, r) .. (r, tiles - 1) and starts
+    // at r tiles - r (r - 1) / 2; the root estimate is corrected exactly
+    const double b = (double)tiles + 0.5;
+    int64_t r = (int64_t)(b - sqrt(fmax(b * b - 2.0 * (double)t, 0.0)));
+    r = imax64(0, imin64(r, tiles - 1));
+    while (r > 0 && r * tiles - r * (r - 1) / 2 > t) --r;
+    while ((r + 1) * tiles - (r + 1) * r / 2 <= t) ++r;
+    const int64_t c = r + (t - (r * tiles - r * (r - 1) / 2));
+    const int64_t i = r * kPeTile + tid, j = c * kPeTile + tid;
+    __syncthreads();
+    if (j < a.n) {
+      s_j[tid].x = a.x[j];
+      s_j[tid].y = a.y[j];
+      s_j[tid].z = a.z[j];
+      s_j[tid].w = (double)a.pm[j].w;
+    }
+    __syncthreads();
+    if (i < a.n) {
+      const double xi = a.x[i], yi = a.y[i], zi = a.z[i];
+      const int lim = (int)imin64(kPeTile, a.n - c * kPeTile);
+      double s = 0.0;
+      // in a diagonal tile only the sources after the target
+#pragma unroll 4
+      for (int k = (r == c) ? tid + 1 : 0; k < lim; ++k) {
+        const double dx = s_j[k].x - xi, dy = s_j[k].y - yi, dz = s_j[k].z - zi;
+        s = fma(s_j[k].w, rsqrt_f64(fma(dx, dx, fma(dy, dy, fma(dz, dz, a.eps2)))), s);
+      }
+      v[4] -= (double)a.pm[i].w * s;
+    }
+  }
+  block_reduce_store<5>(v, a.partials);
+  if (tid == 0) {
+    __threadfence();
+    s_last = atomicAdd(a.ticket, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  if (tid == 0) *a.ticket = 0;  // ready for the next launch
+#pragma unroll
+  for (int k = 0; k < 5; ++k) v[k] = 0.0;
+  for (int b = tid; b < (int)gridDim.x; b += kPeTile)
+#pragma unroll
+    for (int k = 0; k < 5; ++k) v[k] += __ldcg(&a.partials[(int64_t)b * 5 + k]);
+  __syncthreads();
+  block_reduce_store<5>(v, a.out - (int64_t)blockIdx.x * 5);
+}
+
+int energy_f64_blocks(int64_t n) {
+  const int64_t tiles = ceil_div(std::max<int64_t>(n, 1), kPeTile);
+  return (int)std::min<int64_t>(tiles * (tiles + 1) / 2, (int64_t)num_sms() * 8);
+}
+
+void launch_energy_f64(const EnergyArgs& a, cudaStream_t st) {
+  energy_f64_kernel<<<(unsigned)energy_f64_blocks(a.n), kPeTile, 0, st>>>(a);
+  NBGB_LAUNCH_CHECK();
 }
 
 void launch_direct_f64_state(const double* x, const double* y, const double* z, const float4* pm,
@@ -501,15 +555,6 @@ void launch_direct_f64_state(const double* x, const double* y, const double* z, 
   const unsigned blocks =
       (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(n, 256), (int64_t)num_sms() * 8));
   direct_f64_state_kernel<<<blocks, 256, 0, st>>>(x, y, z, pm, n, G, eps2, ax, ay, az);
-  NBGB_LAUNCH_CHECK();
-}
-
-void launch_potential_f64(const double* x, const double* y, const double* z, const float4* pm,
-                          int64_t n, double eps2, double* partials, int nblocks, double* out,
-                          cudaStream_t st) {
-  pe_f64_kernel<<<nblocks, 256, 0, st>>>(x, y, z, pm, n, eps2, partials);
-  NBGB_LAUNCH_CHECK();
-  finish_reduce_kernel<1><<<1, 256, 0, st>>>(partials, nblocks, out);
   NBGB_LAUNCH_CHECK();
 }
 

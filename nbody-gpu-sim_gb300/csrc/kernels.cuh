@@ -105,13 +105,35 @@ void launch_kick_drift(int64_t n, double* x, double* y, double* z, double* vx, d
                        double kick, double dt, float4* pm, cudaStream_t st);
 void launch_kick(int64_t n, double* vx, double* vy, double* vz, const double* ax,
                  const double* ay, const double* az, double kick, cudaStream_t st);
-// Direct forces and potential energy in FP64 from FP64 positions (masses
-// from pm.w).
+// Direct forces in FP64 from FP64 positions (masses from pm.w).
 void launch_direct_f64_state(const double* x, const double* y, const double* z, const float4* pm,
                              int64_t n, double G, double eps2, double* ax, double* ay, double* az,
                              cudaStream_t st);
-void launch_potential_f64(const double* x, const double* y, const double* z, const float4* pm,
-                          int64_t n, double eps2, double* partials, int nblocks, double* out,
-                          cudaStream_t st);
+// Energies and momentum of an FP64 state.  partials: energy_f64_blocks(n) * 5
+// doubles; ticket: a counter, zero before and after; out: KE, Px, Py, Pz and
+// PE without G (device or mapped host memory).
+struct EnergyArgs {
+  const double *x, *y, *z, *vx, *vy, *vz;
+  const float4* pm;
+  int64_t n;
+  double eps2;
+  double* partials;
+  uint32_t* ticket;
+  double* out;
+};
+int energy_f64_blocks(int64_t n);
+void launch_energy_f64(const EnergyArgs& a, cudaStream_t st);
+
+// The state of a system into mapped host memory: x, y, z, vx, vy, vz (6 n
+// doubles), or rounded with the accelerations and masses (10 n floats).
+struct SystemView {
+  int64_t n;
+  const double *x, *y, *z, *vx, *vy, *vz;
+  const float *ax, *ay, *az;
+  const double *ax64, *ay64, *az64;  // null unless the system is FP64 throughout
+  const float4* pm;
+};
+void launch_export_f64(const SystemView& s, double* out, cudaStream_t st);
+void launch_export_f32(const SystemView& s, float* out, cudaStream_t st);
 
 }  // namespace nbgb

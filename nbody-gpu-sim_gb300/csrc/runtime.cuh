@@ -191,7 +191,9 @@ struct nbgb_system {
   nbgb::DevBuf<float4> exch;     // several steps per launch: positions in exchange
   nbgb::DevBuf<uint32_t> exch_ctr;
   nbgb::DevBuf<double> red;
+  nbgb::DevBuf<uint32_t> red_ticket;
   nbgb::HostPinned<double> h_red;
+  nbgb::HostPinned<double> h_state;  // small systems: state read back by one kernel
   bool fp64 = false;
   bool pending_half = false;  // v lags x by half a kick of size last_dt/2
   double last_dt = 0.0;
