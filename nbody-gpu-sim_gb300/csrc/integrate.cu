@@ -178,4 +178,43 @@ void launch_kick(int64_t n, double* vx, double* vy, double* vz, const double* ax
   kick_any(n, vx, vy, vz, ax, ay, az, kick, st);
 }
 
+// A system's state straight into mapped host memory (small systems: one
+// launch instead of a copy per array).
+__global__ void export_f64_kernel(SystemView s, double* __restrict__ out) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < s.n;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    out[i] = s.x[i];
+    out[s.n + i] = s.y[i];
+    out[2 * s.n + i] = s.z[i];
+    out[3 * s.n + i] = s.vx[i];
+    out[4 * s.n + i] = s.vy[i];
+    out[5 * s.n + i] = s.vz[i];
+  }
+}
+
+__global__ void export_f32_kernel(SystemView s, float* __restrict__ out) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < s.n;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    out[i] = (float)s.x[i];
+    out[s.n + i] = (float)s.y[i];
+    out[2 * s.n + i] = (float)s.z[i];
+    out[3 * s.n + i] = (float)s.vx[i];
+    out[4 * s.n + i] = (float)s.vy[i];
+    out[5 * s.n + i] = (float)s.vz[i];
+    out[6 * s.n + i] = s.ax64 ? (float)s.ax64[i] : s.ax[i];
+    out[7 * s.n + i] = s.ax64 ? (float)s.ay64[i] : s.ay[i];
+    out[8 * s.n + i] = s.ax64 ? (float)s.az64[i] : s.az[i];
+    out[9 * s.n + i] = s.pm[i].w;
+  }
+}
+
+void launch_export_f64(const SystemView& s, double* out, cudaStream_t st) {
+  export_f64_kernel<<<grid_for(s.n, 256), 256, 0, st>>>(s, out);
+  NBGB_LAUNCH_CHECK();
+}
+void launch_export_f32(const SystemView& s, float* out, cudaStream_t st) {
+  export_f32_kernel<<<grid_for(s.n, 256), 256, 0, st>>>(s, out);
+  NBGB_LAUNCH_CHECK();
+}
+
 }  // namespace nbgb
