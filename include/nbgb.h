@@ -517,8 +517,10 @@ nbgb_status nbgb_selftest_wait_timeout(uint32_t max_iters, uint32_t* error_bits)
  * a later call would trip over.  Process-wide; nothing reaches the GPU. */
 nbgb_status nbgb_selftest_fail_allocation(int32_t nth);
 
-/* Test hook for the Barnes-Hut group walk: the number of shared-memory stack
- * entries (64 .. 512, default 512) a warp uses before it spills the older
+/* Test hook for the Barnes-Hut walks: the number of shared-memory stack
+ * entries (64 .. 512, default 512) a warp uses.  Beyond it the reference walk
+ * (at most 384 entries) visits a subtree node by node without a stack, with
+ * the same interaction sets; the group walk spills the older
  * half of its traversal stack to a global overflow chunk.  Lowering it
  * exercises the spill path on small inputs; when more warps spill in one
  * walk than there are overflow chunks (256), or one warp outgrows its chunk,

@@ -34,17 +34,9 @@
 //      children in octant order with the reference's float operations
 //      (:514-538), so masses and centres of mass are bit-identical.
 //
-// Walk.  One warp walks its segment's pre-order range for 32 consecutive
-// targets (path-sorted, so spatially close).  Every lane applies the
-// reference's per-target rules (contains_i, leaf self-subtraction, opening
-// test 4h^2/(d^2+eps^2) < theta^2, :175-243); the warp descends into a node
-// if any active lane opens it, and a lane that accepted a node sleeps until
-// the cursor leaves that node's subtree.  Each lane therefore sums exactly
-// the reference's interaction set for its target (no stack, no local
-// memory, broadcast node loads).  With leaf_capacity > 1 a subtree holding
-// at most that many bodies is summed body by body when opened.  The group walk
-// (one list per group of nearby bodies) is in bh_group.cu; the node record,
-// state and shared parameters in bh_tree.cuh.
+// The reference walk is in bh_walk.cu, the group walk (one list per group of
+// nearby bodies) in bh_group.cu; the node record, state and shared parameters
+// in bh_tree.cuh.
 #include <algorithm>
 #include <atomic>
 #include <vector>
@@ -872,183 +864,6 @@ __global__ void com_kernel(Node* __restrict__ nodes, const float4* __restrict__ 
   }
 }
 
-// ----------------------------------------------------------------- walk --
-struct WalkArgs {
-  const Node* nodes;
-  const float4* spm;
-  const uint32_t* body;
-  const uint32_t* nstart;
-  SegView sv;
-  const WarpTask* tasks;
-  int64_t ntasks;
-  const int32_t* seg_root;
-  const int32_t* seg_end;
-  int64_t n;
-  int64_t cap;
-  float theta2;
-  float th_lo;  // theta2 * (1 - 2^-16)
-  float th_hi;  // theta2 * (1 + 2^-16)
-  float eps2;
-  float G;
-  int leaf_cap;
-  float* ax;
-  float* ay;
-  float* az;
-  int32_t* counts;                  // per-body interaction counts (or null)
-  unsigned long long* inter_total;  // sum of interactions (or null)
-  uint32_t* task_ctr;               // zeroed before the launch
-};
-
-// The reference's opening test `size2 / dist2 < theta2` with the correctly
-// rounded quotient (force_barnes_hut.cu:222-224), decided by two FP32
-// products against thresholds theta2 (1 -+ 2^-16) whenever size2 is not
-// within 2^-16 (relative) of theta2 * dist2 -- almost always -- and by the
-// IEEE division otherwise.  With |rounding| <= 2^-24 per product, a product
-// test that fires implies the exact quotient is below theta2 (1 - 2^-17),
-// resp. above theta2 (1 + 2^-17), so the outcome equals the IEEE comparison.
-__device__ __forceinline__ bool opening_accept(float size2, float d2, float th_lo, float th_hi,
-                                               float theta2) {
-  if (size2 < d2 * th_lo) return true;
-  if (size2 > d2 * th_hi) return false;
-  return __fdiv_rn(size2, d2) < theta2;
-}
-
-__device__ __forceinline__ void bh_add(float px, float py, float pz, float m, float xi, float yi,
-                                       float zi, float eps2, float& sx, float& sy, float& sz) {
-  const float dx = __fsub_rn(px, xi), dy = __fsub_rn(py, yi), dz = __fsub_rn(pz, zi);
-  const float d2 = __fadd_rn(__fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx))), eps2);
-  const float r = rsqrt_approx(d2);
-  const float f = (m * r) * (r * r);
-  sx = fmaf(f, dx, sx);
-  sy = fmaf(f, dy, sy);
-  sz = fmaf(f, dz, sz);
-}
-
-template <bool COUNT, bool BUCKET>
-__global__ void __launch_bounds__(256, BUCKET ? 6 : (COUNT ? 7 : 8)) bh_walk_kernel(WalkArgs a) {
-  const uint32_t total = a.nstart[a.n];
-  const bool tree_ok = (int64_t)total <= a.cap;
-  const int lane = threadIdx.x & 31;
-  // persistent warps take the next task (32 path-consecutive targets) from a
-  // counter: the walk cost per task varies a lot, so this balances the SMs
-  while (true) {
-    uint32_t t32 = 0;
-    if (lane == 0) t32 = atomicAdd(a.task_ctr, 1u);
-    const int64_t t = __shfl_sync(0xffffffffu, t32, 0);
-    if (t >= a.ntasks) break;
-    const WarpTask task = a.tasks[t];
-    const int64_t k = task.first + lane;
-    const bool valid = k < task.end;
-    const float4 pi = valid ? a.spm[k] : make_float4(0.f, 0.f, 0.f, 0.f);
-    const f2 pi_xy = f2_make(pi.x, pi.y);
-    float sx = 0.f, sy = 0.f, sz = 0.f;
-    int cnt = 0;
-    int resume = valid ? 0 : 0x7fffffff;
-    int node = tree_ok ? a.seg_root[task.seg] : 0;
-    const int node_end = tree_ok ? a.seg_end[task.seg] : 0;
-    while (node < node_end) {
-      // one 32-byte load (centre of mass + cube) as four x/y, z/w pairs, one
-      // 8-byte load (skip and flags, size2); x and y differences are taken
-      // as packed FP32x2 (same IEEE rounding per component)
-      f2 cm_xy, cm_zw, g_xy, g_zw;
-      ld_node2(&a.nodes[node], cm_xy, cm_zw, g_xy, g_zw);
-      float4 cm, g;
-      f2_split(cm_xy, cm.x, cm.y);
-      f2_split(cm_zw, cm.z, cm.w);
-      f2_split(g_xy, g.x, g.y);
-      f2_split(g_zw, g.z, g.w);
-      float tx, ty;  // target minus cube centre
-      f2_split(f2_sub(pi_xy, g_xy), tx, ty);
-      // the bucket walk also needs the node's body range (same 16-byte load)
-      int4 wr;
-      if (BUCKET) {
-        wr = __ldg(&a.nodes[node].walk);
-      } else {
-        const int2 w2 = __ldg(reinterpret_cast<const int2*>(&a.nodes[node].walk));
-        wr = make_int4(w2.x, w2.y, 0, 0);
-      }
-      const int skip = wr.x & (int)(kWalkZero - 1u);
-      if ((uint32_t)wr.x >= kWalkZero) {  // a leaf, or zero mass
-        if ((uint32_t)wr.x & kWalkZero) {  // force_barnes_hut.cu:172-173
-          node = skip;
-          continue;
-        }
-        // leaf (force_barnes_hut.cu:185-203)
-        if (node >= resume) {
-          float me = cm.w, cx = cm.x, cy = cm.y, cz = cm.z;
-          bool use = true;
-          if (fabsf(tx) <= g.w && fabsf(ty) <= g.w && fabsf(__fsub_rn(pi.z, g.z)) <= g.w) {
-            me = __fsub_rn(cm.w, pi.w);
-            use = me > 0.0f;
-            if (use) {
-              cx = __fdiv_rn(__fsub_rn(__fmul_rn(cm.x, cm.w), __fmul_rn(pi.x, pi.w)), me);
-              cy = __fdiv_rn(__fsub_rn(__fmul_rn(cm.y, cm.w), __fmul_rn(pi.y, pi.w)), me);
-              cz = __fdiv_rn(__fsub_rn(__fmul_rn(cm.z, cm.w), __fmul_rn(pi.z, pi.w)), me);
-            }
-          }
-          if (use) {
-            bh_add(cx, cy, cz, me, pi.x, pi.y, pi.z, a.eps2, sx, sy, sz);
-            if (COUNT) ++cnt;
-          }
-        }
-        node = skip;
-        continue;
-      }
-      // internal node (force_barnes_hut.cu:205-243)
-      const bool active = node >= resume;
-      const bool contains =
-          fabsf(tx) <= g.w && fabsf(ty) <= g.w && fabsf(__fsub_rn(pi.z, g.z)) <= g.w;
-      float dx, dy;
-      f2_split(f2_sub(cm_xy, pi_xy), dx, dy);
-      const float dz = __fsub_rn(cm.z, pi.z);
-      const float d2 = __fadd_rn(__fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx))), a.eps2);
-      const float size2 = __int_as_float(wr.y);
-      const bool accept = !contains && opening_accept(size2, d2, a.th_lo, a.th_hi, a.theta2);
-      const bool open = active && !accept;
-      if (active && accept) {
-        const float r = rsqrt_approx(d2);
-        const float f = (cm.w * r) * (r * r);
-        sx = fmaf(f, dx, sx);
-        sy = fmaf(f, dy, sy);
-        sz = fmaf(f, dz, sz);
-        if (COUNT) ++cnt;
-        resume = skip;
-      }
-      if (BUCKET && (int)((uint32_t)wr.w & ~kWalkNext) <= a.leaf_cap) {
-        // a subtree of at most leaf_cap bodies: the lanes that open it sum
-        // its bodies directly (all read the same body: one broadcast load)
-        if (open) {
-          const int64_t self = k - wr.z;
-          const int nb = (int)((uint32_t)wr.w & ~kWalkNext);
-          for (int j = 0; j < nb; ++j) {
-            const float4 q = __ldg(&a.spm[wr.z + j]);
-            if (j != self) {
-              bh_add(q.x, q.y, q.z, q.w, pi.x, pi.y, pi.z, a.eps2, sx, sy, sz);
-              if (COUNT) ++cnt;
-            }
-          }
-        }
-        node = skip;
-        continue;
-      }
-      node = __any_sync(0xffffffffu, open) ? node + 1 : skip;
-    }
-    if (valid) {
-      const int64_t i = a.sv.arena(a.body[k]);
-      a.ax[i] = a.G * sx;
-      a.ay[i] = a.G * sy;
-      a.az[i] = a.G * sz;
-      if (COUNT && a.counts) a.counts[i] = cnt;
-    }
-    if (COUNT && a.inter_total) {
-      unsigned long long c = valid ? (unsigned long long)cnt : 0ull;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) c += __shfl_down_sync(0xffffffffu, c, o);
-      if (lane == 0) atomicAdd(a.inter_total, c);
-    }
-  }
-}
-
 static unsigned grid1d(int64_t n, int threads = 256) {
   return (unsigned)std::max<int64_t>(
       1, std::min<int64_t>(ceil_div(std::max<int64_t>(n, 1), threads), (int64_t)num_sms() * 32));
@@ -1076,7 +891,7 @@ BHState* bh_state_new() { return new BHState(); }
 
 size_t bh_segment_table_bytes(const int64_t* n_per, int nseg) {
   int64_t ntask = 0;
-  for (int s = 0; s < nseg; ++s) ntask += ceil_div(n_per[s], 32);
+  for (int s = 0; s < nseg; ++s) ntask += ceil_div(n_per[s], bh_walk_targets(n_per[s]));
   return ((size_t)nseg * 2 + 1) * sizeof(int64_t) + (size_t)ntask * sizeof(WarpTask);
 }
 
@@ -1099,8 +914,16 @@ void bh_set_segments(BHState& h, const int64_t* off, const int64_t* n_per, int n
     if (n_per[s] < 1) fail(NBGB_ERR_INVALID_ARG, "Validation Error: empty Barnes-Hut segment");
     hoff[s] = off[s];
     hbase[s] = n;
-    for (int64_t f = n; f < n + n_per[s]; f += 32) ht[t++] = WarpTask{f, n + n_per[s], s, 0};
     n += n_per[s];
+  }
+  // the walk's tasks, those of 32 targets first
+  for (const int tw : {32, 16}) {
+    for (int s = 0; s < nseg; ++s) {
+      if (bh_walk_targets(n_per[s]) != tw) continue;
+      const int64_t end = hbase[s] + n_per[s];
+      for (int64_t f = hbase[s]; f < end; f += tw) ht[t++] = WarpTask{f, end, s, 0};
+    }
+    if (tw == 32) h.ntasks32 = t;
   }
   hbase[nseg] = n;
   char* d = grow(h.tables, bytes);
@@ -1277,68 +1100,13 @@ void bh_build(BHState& h, const float4* pm, cudaStream_t st, uint32_t* err, bool
   h.built = true;
 }
 
-// Resident 256-thread blocks per SM of one walk instantiation.
-template <bool COUNT, bool BUCKET>
-static int walk_occupancy() {
-  static const int occ = [] {
-    int b = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, bh_walk_kernel<COUNT, BUCKET>, 256, 0);
-    return std::max(b, 1);
-  }();
-  return occ;
-}
-
 // Forces for every segment: acc written at each segment's arena offset.
 void bh_walk(BHState& h, const BHWalkParams& p, float* ax, float* ay, float* az, int32_t* counts,
              unsigned long long* inter_total, uint32_t* err, cudaStream_t st) {
-  if (p.group_walk) {
+  if (p.group_walk)
     bh_group_walk(h, p, ax, ay, az, counts, inter_total, err, st);
-    return;
-  }
-  WalkArgs w;
-  w.nodes = h.nodes.ptr;
-  w.spm = h.spm.ptr;
-  w.body = h.body;
-  w.nstart = h.nstart.ptr;
-  w.sv = SegView{h.seg_off_p, h.seg_base_p, h.seg_of.ptr, h.box.ptr};
-  w.tasks = h.tasks_p;
-  w.ntasks = h.ntasks;
-  w.seg_root = h.seg_root.ptr;
-  w.seg_end = h.seg_end.ptr;
-  w.n = h.n;
-  w.cap = h.cap;
-  w.theta2 = p.theta * p.theta;
-  w.th_lo = w.theta2 * (1.0f - 1.52587890625e-05f);
-  w.th_hi = w.theta2 * (1.0f + 1.52587890625e-05f);
-  w.eps2 = p.softening * p.softening;
-  w.G = p.G;
-  w.leaf_cap = p.leaf_capacity;
-  w.ax = ax;
-  w.ay = ay;
-  w.az = az;
-  w.counts = counts;
-  w.inter_total = inter_total;
-  w.task_ctr = grow(h.walk_ctr, 1);
-  NBGB_CUDA(cudaMemsetAsync(w.task_ctr, 0, sizeof(uint32_t), st));
-  const bool count = counts != nullptr || inter_total != nullptr;
-  const bool bucket = p.leaf_capacity > 1;
-  // one resident wave of persistent warps
-  const int64_t need = ceil_div(h.ntasks * 32, 256);
-  auto grid = [&](int occ) {
-    return (unsigned)std::max<int64_t>(1, std::min<int64_t>(need, (int64_t)num_sms() * occ));
-  };
-  if (count) {
-    if (bucket)
-      bh_walk_kernel<true, true><<<grid(walk_occupancy<true, true>()), 256, 0, st>>>(w);
-    else
-      bh_walk_kernel<true, false><<<grid(walk_occupancy<true, false>()), 256, 0, st>>>(w);
-  } else {
-    if (bucket)
-      bh_walk_kernel<false, true><<<grid(walk_occupancy<false, true>()), 256, 0, st>>>(w);
-    else
-      bh_walk_kernel<false, false><<<grid(walk_occupancy<false, false>()), 256, 0, st>>>(w);
-  }
-  NBGB_LAUNCH_CHECK();
+  else
+    bh_reference_walk(h, p, ax, ay, az, counts, inter_total, st);
 }
 
 // Node capacity that any realistic input fits (the canonical tree has ~1.5N
@@ -1384,7 +1152,7 @@ void bh_reserve_buffers(BHState& h, bool groups) {
   grow(h.leaf_of, R);
   grow(h.seg_root, (size_t)nseg);
   grow(h.seg_end, (size_t)nseg);
-  grow(h.walk_ctr, 1);
+  grow(h.walk_ctr, 2);
   if (groups) {
     grow(h.groups, R);
     h.groups2.ensure(h.groups.cap);

@@ -9,7 +9,8 @@ namespace nbgb {
 struct BHState;
 struct StageTimer;
 
-// 32 consecutive path-sorted targets of one segment, walked by one warp.
+// Consecutive path-sorted targets of one segment (bh_walk_targets of its
+// size), walked by one warp.
 struct WarpTask {
   int64_t first;  // first sorted position
   int64_t end;    // one past the segment's last sorted position
@@ -26,6 +27,9 @@ struct BHWalkParams {
                       // accepted by the group's bounding box (opened buckets of at most
                       // leaf_capacity bodies list their bodies)
 };
+
+constexpr int64_t kWalk32MinBodies = 32768;
+int bh_walk_targets(int64_t n);
 
 BHState* bh_state_new();
 void bh_state_delete(BHState* p);

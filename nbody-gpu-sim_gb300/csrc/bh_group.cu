@@ -505,6 +505,7 @@ static void launch_group_walk(const GroupWalkArgs& g, int64_t n, bool two, cudaS
 static std::atomic<int> g_group_stack_limit{kGStack};
 
 void bh_set_group_stack_limit(int entries) { g_group_stack_limit.store(entries); }
+int bh_group_stack_limit() { return g_group_stack_limit.load(); }
 
 void bh_group_walk(BHState& h, const BHWalkParams& p, float* ax, float* ay, float* az,
                           int32_t* counts, unsigned long long* inter_total, uint32_t* err,

@@ -61,6 +61,7 @@ struct BHState {
   HostPinned<char> h_tables;
   int32_t nseg = 0;
   int64_t ntasks = 0;
+  int64_t ntasks32 = 0;  // the first tasks, of 32 targets; the others have 16
   // keys and order
   DevBuf<uint32_t> mkeys, mkeys_alt, midx, midx_alt;  // on-demand Morton sort
   DevBuf<u64> klo, khi, khi_alt;
@@ -78,7 +79,7 @@ struct BHState {
   DevBuf<char> ref_nodes;   // reference-identical build: the reference's node array
   DevBuf<int32_t> ref_pos;  // reference-identical build: original index -> sorted position
   DevBuf<float4> spm;      // bodies in path order
-  DevBuf<uint32_t> walk_ctr;  // next warp task of the walk
+  DevBuf<uint32_t> walk_ctr;  // next warp task of the walk (32 and 16 targets)
   DevBuf<int4> groups;        // group walk: first body, count, segment; cost classes 0 / 1
                               // from the front / back of groups, 2 / 3 of groups2
   DevBuf<int4> groups2;
@@ -161,5 +162,11 @@ inline T* grow(DevBuf<T>& b, size_t n) {
 void bh_group_walk(BHState& h, const BHWalkParams& p, float* ax, float* ay, float* az,
                    int32_t* counts, unsigned long long* inter_total, uint32_t* err,
                    cudaStream_t st);
+
+// The reference walk for every segment (bh_walk.cu).
+void bh_reference_walk(BHState& h, const BHWalkParams& p, float* ax, float* ay, float* az,
+                       int32_t* counts, unsigned long long* inter_total, cudaStream_t st);
+// Stack entries the walks use (bh_set_group_stack_limit).
+int bh_group_stack_limit();
 
 }  // namespace nbgb
