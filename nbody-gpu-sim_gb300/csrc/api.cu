@@ -122,12 +122,13 @@ static void direct_forces(nbgb_calculator* c, const DirectSource& src, int64_t n
   float4* part = nullptr;
   uint32_t* ticket = nullptr;
   if (p.splits > 1) {
-    part = c->partial.ensure((size_t)p.splits * p.n_tgt_pad);
-    if (c->ticket.cap < (size_t)p.i_blocks) {  // counters start, and are left, at zero
-      ticket = c->ticket.ensure((size_t)p.i_blocks);
-      NBGB_CUDA(cudaMemsetAsync(ticket, 0, c->ticket.bytes(), c->stream));
-    }
-    ticket = c->ticket.ptr;
+    // finished-run counters (start, and are left, at zero), then the sums
+    const size_t head = kDirMaxBlocks * sizeof(uint32_t) / sizeof(float4);
+    const size_t need = head + (size_t)p.splits * p.n_tgt_pad;
+    if (c->partial.cap < need)
+      NBGB_CUDA(cudaMemsetAsync(c->partial.ensure(need), 0, head * sizeof(float4), c->stream));
+    ticket = reinterpret_cast<uint32_t*>(c->partial.ptr);
+    part = c->partial.ptr + head;
   }
   const float eps = c->params.softening;
   launch_direct(p, src, n, c->params.G, eps * eps,

@@ -204,7 +204,7 @@ DirectPlan plan_direct(int64_t n, int max_splits) {
   for (int I = 1; I <= 2; ++I) {
     const int64_t T = (int64_t)kDirHalf * I, blocks = ceil_div(n, T);
     const int64_t s_max = std::max<int64_t>(
-        1, std::min<int64_t>({ceil_div(n, 32), (int64_t)max_splits, ceil_div(16384, blocks)}));
+        1, std::min<int64_t>({ceil_div(n, 32), (int64_t)max_splits, kDirMaxBlocks / blocks}));
     for (int64_t s = 1; s <= s_max; ++s) {
       const int64_t jper = ceil_div(ceil_div(n, s), 16) * 16;
       if (ceil_div(n, jper) != s) continue;

@@ -49,6 +49,7 @@ struct DirectPlan {
 // accelerations (no overlap).
 bool direct_from_soa(const nbgb_particle_data* d);
 constexpr int kDirMaxSplits = 128;
+constexpr int64_t kDirMaxBlocks = 16384;  // target blocks of a plan with several runs
 DirectPlan plan_direct(int64_t n, int max_splits = kDirMaxSplits);
 // Forces on all n bodies of src.  With p.splits > 1: partial holds
 // splits * n_tgt_pad entries, ticket i_blocks counters that are zero before

@@ -166,8 +166,8 @@ struct nbgb_calculator {
   int device = 0;
 
   nbgb::DevBuf<float4> pm;        // packed (x, y, z, m) input of the last drop-in call
-  nbgb::DevBuf<float4> partial;   // direct: partial sums of the source runs
-  nbgb::DevBuf<uint32_t> ticket;  // direct: finished runs per target block (zero between calls)
+  nbgb::DevBuf<float4> partial;   // direct: finished runs per target block (zero between
+                                  // calls), then the partial sums of the source runs
   nbgb::ErrorWord err;            // device error word
   nbgb::DevBuf<int32_t> counts;   // per-target interaction / neighbour counts
   nbgb::DevBuf<double> red;       // reduction partials
