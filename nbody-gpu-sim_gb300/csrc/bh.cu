@@ -46,56 +46,14 @@
 #include "common.cuh"
 #include "geom.cuh"
 #include "kernels.cuh"
+#include "pathkey.cuh"
+#include "pathsort.cuh"
 #include "runtime.cuh"
 #include "sort.cuh"
 
 namespace nbgb {
 
 void bh_state_delete(BHState* p) { delete p; }
-
-// ----------------------------------------------------------------- keys --
-__device__ __forceinline__ uint32_t spread3(uint32_t v) {
-  v &= 0x3FFu;
-  v = (v | (v << 16)) & 0x030000FFu;
-  v = (v | (v << 8)) & 0x0300F00Fu;
-  v = (v | (v << 4)) & 0x030C30C3u;
-  v = (v | (v << 2)) & 0x09249249u;
-  return v;
-}
-
-// computeMortonCode (force_barnes_hut.cu:42-50) on (p - min) * inv.
-__device__ __forceinline__ uint32_t morton_of(float4 p, const BBox& b) {
-  float nx = __fmul_rn(__fsub_rn(p.x, b.min[0]), b.inv[0]);
-  float ny = __fmul_rn(__fsub_rn(p.y, b.min[1]), b.inv[1]);
-  float nz = __fmul_rn(__fsub_rn(p.z, b.min[2]), b.inv[2]);
-  uint32_t ix = (uint32_t)__fmul_rn(fminf(fmaxf(nx, 0.0f), 1.0f), 1023.0f);
-  uint32_t iy = (uint32_t)__fmul_rn(fminf(fmaxf(ny, 0.0f), 1.0f), 1023.0f);
-  uint32_t iz = (uint32_t)__fmul_rn(fminf(fmaxf(nz, 0.0f), 1.0f), 1023.0f);
-  return (spread3(ix) << 2) | (spread3(iy) << 1) | spread3(iz);
-}
-
-// Octant path of a position through the reference's subdivision: the high
-// key (levels 1..21, 3 bits each, level 1 most significant) and the low key
-// (levels 22..32).
-__device__ __forceinline__ void path_key(float4 p, const BBox& b, u64& hi, u64& lo) {
-  float cx = b.center[0], cy = b.center[1], cz = b.center[2], h = b.half;
-  u64 a = 0, c = 0;
-#pragma unroll
-  for (int lev = 1; lev <= kMaxDepth; ++lev) {
-    const uint32_t o = (p.x >= cx ? 1u : 0u) | (p.y >= cy ? 2u : 0u) | (p.z >= cz ? 4u : 0u);
-    const float hs = __fmul_rn(h, 0.5f);
-    cx = __fadd_rn(cx, (o & 1u) ? hs : -hs);
-    cy = __fadd_rn(cy, (o & 2u) ? hs : -hs);
-    cz = __fadd_rn(cz, (o & 4u) ? hs : -hs);
-    h = hs;
-    if (lev <= kHiLevels)
-      a = (a << 3) | o;
-    else
-      c = (c << 3) | o;
-  }
-  hi = a;
-  lo = c;
-}
 
 // ----------------------------------------------------- segment setup --
 __global__ void seg_of_kernel(const int64_t* __restrict__ base, int nseg, int64_t n,
@@ -123,27 +81,61 @@ __device__ __forceinline__ float ord2f(uint32_t u) {
   return __uint_as_float((u & 0x80000000u) ? (u & 0x7fffffffu) : ~u);
 }
 
-// Per-segment min/max of the bodies.  A block reduces a contiguous chunk;
-// when the chunk lies in one segment (the common case) it issues one atomic
-// per bound, otherwise each warp (or lane) does.  Min/max are exact, so the
-// result equals the reference's computeBoundingBoxKernel (:78-122).
+// Per-segment min/max of the bodies, and from them the reference's derived
+// constants with its float operations
+//   Morton scale  inv = 1.0f / (max - min + 0.001f)            (:313-320)
+//   root centre   (min + max) * 0.5f                           (:418-419)
+//   root half     max(ex, ey, ez) * 0.5f + 0.001f, first max   (:420-422)
+// A block reduces a contiguous chunk; when the chunk lies in one segment (the
+// common case) it issues one atomic per bound, otherwise each lane does; the
+// last block derives the boxes.  Min/max are exact, so the result equals the
+// reference's computeBoundingBoxKernel (:78-122).  mm holds [6][nseg] maxima of
+// order-preserving integers (minima as the maxima of their complements) and a
+// block counter, all zero before the launch.
+__device__ __forceinline__ void seg_box(const uint32_t* mm, int nseg, int s, BBox* box,
+                                        uint32_t* err) {
+  BBox o;
+  bool ok = true;
+  for (int a = 0; a < 3; ++a) {
+    const float mn = ord2f(~__ldcg(&mm[a * nseg + s])), mx = ord2f(__ldcg(&mm[(3 + a) * nseg + s]));
+    o.min[a] = mn;
+    o.max[a] = mx;
+    ok = ok && isfinite(mn) && isfinite(mx);
+    o.inv[a] = __fdiv_rn(1.0f, __fadd_rn(__fsub_rn(mx, mn), 0.001f));
+    o.center[a] = __fmul_rn(__fadd_rn(mn, mx), 0.5f);
+  }
+  const float ex = __fsub_rn(o.max[0], o.min[0]), ey = __fsub_rn(o.max[1], o.min[1]),
+              ez = __fsub_rn(o.max[2], o.min[2]);
+  float ms = ex;
+  if (ms < ey) ms = ey;
+  if (ms < ez) ms = ez;
+  o.half = __fadd_rn(__fmul_rn(ms, 0.5f), 0.001f);
+  o.valid = ok ? 1 : 0;
+  if (!ok) raise_error(err, kErrBadInput);
+  box[s] = o;
+}
+
 __global__ void seg_bounds_kernel(const float4* __restrict__ pm, SegView sv, int64_t n, int nseg,
-                                  uint32_t* __restrict__ mm) {
+                                  uint32_t* __restrict__ mm, BBox* __restrict__ box,
+                                  uint32_t* err) {
   __shared__ float s_red[32][6];
   __shared__ int s_same;
+  __shared__ bool s_last;
   const int64_t c0 = (int64_t)blockIdx.x * blockDim.x * 4;
   const int64_t c1 = imin64(c0 + (int64_t)blockDim.x * 4, n);
-  if (c0 >= n) return;
-  if (threadIdx.x == 0) s_same = (sv.seg_of[c0] == sv.seg_of[c1 - 1]);
+  if (threadIdx.x == 0) s_same = nseg == 1 || sv.seg_of[c0] == sv.seg_of[c1 - 1];
   __syncthreads();
   const bool same = s_same;
   float v[6] = {1e30f, 1e30f, 1e30f, -1e30f, -1e30f, -1e30f};
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int s0 = same && nseg > 1 ? sv.seg_of[c0] : 0;
+  const int64_t d0 = sv.off[s0] - sv.base[s0];
+#pragma unroll
   for (int r = 0; r < 4; ++r) {
     const int64_t q = c0 + (int64_t)r * blockDim.x + threadIdx.x;
     if (q < c1) {
-      const float4 p = pm[sv.arena((uint32_t)q)];
       if (same) {
+        const float4 p = pm[q + d0];
         v[0] = fminf(v[0], p.x);
         v[1] = fminf(v[1], p.y);
         v[2] = fminf(v[2], p.z);
@@ -151,68 +143,43 @@ __global__ void seg_bounds_kernel(const float4* __restrict__ pm, SegView sv, int
         v[4] = fmaxf(v[4], p.y);
         v[5] = fmaxf(v[5], p.z);
       } else {
+        const float4 p = pm[sv.arena((uint32_t)q)];
         const int s = sv.seg_of[q];
-        atomicMin(&mm[0 * nseg + s], f2ord(p.x));
-        atomicMin(&mm[1 * nseg + s], f2ord(p.y));
-        atomicMin(&mm[2 * nseg + s], f2ord(p.z));
-        atomicMax(&mm[3 * nseg + s], f2ord(p.x));
-        atomicMax(&mm[4 * nseg + s], f2ord(p.y));
-        atomicMax(&mm[5 * nseg + s], f2ord(p.z));
+        const float w[6] = {fminf(1e30f, p.x),  fminf(1e30f, p.y),  fminf(1e30f, p.z),
+                            fmaxf(-1e30f, p.x), fmaxf(-1e30f, p.y), fmaxf(-1e30f, p.z)};
+        for (int a = 0; a < 3; ++a) {
+          atomicMax(&mm[a * nseg + s], ~f2ord(w[a]));
+          atomicMax(&mm[(3 + a) * nseg + s], f2ord(w[3 + a]));
+        }
       }
     }
   }
-  if (!same) return;
+  if (same) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1)
+    for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      v[a] = fminf(v[a], __shfl_down_sync(0xffffffffu, v[a], o));
-      v[3 + a] = fmaxf(v[3 + a], __shfl_down_sync(0xffffffffu, v[3 + a], o));
-    }
-  if (lane == 0)
-    for (int a = 0; a < 6; ++a) s_red[warp][a] = v[a];
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int w = 1; w < (int)(blockDim.x >> 5); ++w)
       for (int a = 0; a < 3; ++a) {
-        v[a] = fminf(v[a], s_red[w][a]);
-        v[3 + a] = fmaxf(v[3 + a], s_red[w][3 + a]);
+        v[a] = fminf(v[a], __shfl_down_sync(0xffffffffu, v[a], o));
+        v[3 + a] = fmaxf(v[3 + a], __shfl_down_sync(0xffffffffu, v[3 + a], o));
       }
-    const int s = sv.seg_of[c0];
-    for (int a = 0; a < 3; ++a) {
-      atomicMin(&mm[a * nseg + s], f2ord(v[a]));
-      atomicMax(&mm[(3 + a) * nseg + s], f2ord(v[3 + a]));
+    if (lane == 0)
+      for (int a = 0; a < 6; ++a) s_red[warp][a] = v[a];
+    __syncthreads();
+    if (threadIdx.x < 6) {
+      const int a = threadIdx.x;
+      float x = s_red[0][a];
+      for (int w = 1; w < (int)(blockDim.x >> 5); ++w)
+        x = a < 3 ? fminf(x, s_red[w][a]) : fmaxf(x, s_red[w][a]);
+      atomicMax(&mm[a * nseg + s0], a < 3 ? ~f2ord(x) : f2ord(x));
     }
   }
-}
-
-// Per segment: the reference's derived constants with its float operations
-//   Morton scale  inv = 1.0f / (max - min + 0.001f)            (:313-320)
-//   root centre   (min + max) * 0.5f                           (:418-419)
-//   root half     max(ex, ey, ez) * 0.5f + 0.001f, first max   (:420-422)
-__global__ void seg_box_kernel(const uint32_t* __restrict__ mm, int nseg, BBox* __restrict__ box,
-                               uint32_t* err) {
-  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < nseg; s += gridDim.x * blockDim.x) {
-    BBox o;
-    bool ok = true;
-    for (int a = 0; a < 3; ++a) {
-      const float mn = ord2f(mm[a * nseg + s]), mx = ord2f(mm[(3 + a) * nseg + s]);
-      o.min[a] = mn;
-      o.max[a] = mx;
-      ok = ok && isfinite(mn) && isfinite(mx);
-      o.inv[a] = __fdiv_rn(1.0f, __fadd_rn(__fsub_rn(mx, mn), 0.001f));
-      o.center[a] = __fmul_rn(__fadd_rn(mn, mx), 0.5f);
-    }
-    const float ex = __fsub_rn(o.max[0], o.min[0]), ey = __fsub_rn(o.max[1], o.min[1]),
-                ez = __fsub_rn(o.max[2], o.min[2]);
-    float ms = ex;
-    if (ms < ey) ms = ey;
-    if (ms < ez) ms = ez;
-    o.half = __fadd_rn(__fmul_rn(ms, 0.5f), 0.001f);
-    o.valid = ok ? 1 : 0;
-    if (!ok) raise_error(err, kErrBadInput);
-    box[s] = o;
-  }
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(&mm[6 * nseg], 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  for (int s = threadIdx.x; s < nseg; s += blockDim.x) seg_box(mm, nseg, s, box, err);
 }
 
 // High path key of every body in concatenated order (values = indices).
@@ -234,11 +201,11 @@ __global__ void seg_key_kernel(const uint32_t* __restrict__ idx, const int32_t* 
     sk[k] = (uint32_t)seg_of[idx[k]];
 }
 
-// Final order: segment, both path keys and the body itself per position.
+// Final order: segment, high path key and the body itself per position.
 __global__ void path_final_kernel(const float4* __restrict__ pm, SegView sv,
                                   const uint32_t* __restrict__ body, int64_t n,
                                   int32_t* __restrict__ kseg, u64* __restrict__ hi,
-                                  u64* __restrict__ lo, float4* __restrict__ spm) {
+                                  float4* __restrict__ spm) {
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n;
        k += (int64_t)gridDim.x * blockDim.x) {
     const uint32_t q = body[k];
@@ -248,7 +215,6 @@ __global__ void path_final_kernel(const float4* __restrict__ pm, SegView sv,
     path_key(p, sv.box[s], h, l);
     kseg[k] = s;
     hi[k] = h;
-    lo[k] = l;
     spm[k] = p;
   }
 }
@@ -267,10 +233,10 @@ __device__ __forceinline__ bool tie_less(const float4& pa, uint32_t a, const flo
 }
 
 // Runs of equal (segment, high key) -- bodies sharing their first 21
-// octants, tiny in practice -- are insertion-sorted by one thread per run;
-// positions of a run that moved get their body, low key and payload fixed.
-// A run already in order (e.g. coincident bodies) costs one comparison per
-// body.
+// octants, tiny in practice -- are insertion-sorted by one thread per run,
+// which also writes their low keys (nobody reads the low key of a body whose
+// high key differs from its neighbours').  A run already in order (e.g.
+// coincident bodies) costs one comparison per body.
 __global__ void tie_order_kernel(SegView sv, int64_t n, const int32_t* __restrict__ kseg,
                                  const u64* __restrict__ hi, uint32_t* __restrict__ body,
                                  u64* __restrict__ lo, float4* __restrict__ spm) {
@@ -281,7 +247,6 @@ __global__ void tie_order_kernel(SegView sv, int64_t n, const int32_t* __restric
     int64_t e = k + 1;
     while (e + 1 < n && hi[e + 1] == hi[k] && kseg[e + 1] == kseg[k]) ++e;
     const BBox b = sv.box[kseg[k]];
-    bool moved = false;
     for (int64_t i = k + 1; i <= e; ++i) {
       const uint32_t cur = body[i];
       const float4 pc = spm[i];
@@ -290,17 +255,15 @@ __global__ void tie_order_kernel(SegView sv, int64_t n, const int32_t* __restric
         body[j + 1] = body[j];
         spm[j + 1] = spm[j];
         --j;
-        moved = true;
       }
       body[j + 1] = cur;
       spm[j + 1] = pc;
     }
-    if (moved)
-      for (int64_t i = k; i <= e; ++i) {
-        u64 h, l;
-        path_key(spm[i], b, h, l);
-        lo[i] = l;
-      }
+    for (int64_t i = k; i <= e; ++i) {
+      u64 h, l;
+      path_key(spm[i], b, h, l);
+      lo[i] = l;
+    }
   }
 }
 
@@ -319,8 +282,12 @@ __global__ void morton_scatter_kernel(const float4* __restrict__ spm,
   }
 }
 
-__device__ __forceinline__ int common_levels(u64 h0, u64 l0, u64 h1, u64 l1) {
+// Common levels of sorted bodies i and j (low keys are written, and read, only
+// where the high keys agree).
+__device__ __forceinline__ int common_levels(const u64* hi, const u64* lo, int64_t i, int64_t j) {
+  const u64 h0 = hi[i], h1 = hi[j];
   if (h0 != h1) return (__clzll(h0 ^ h1) - 1) / 3;  // bit 63 unused
+  const u64 l0 = lo[i], l1 = lo[j];
   if (l0 != l1) return kHiLevels + (__clzll(l0 ^ l1) - 31) / 3;  // bits 63..33 unused
   return kMaxDepth;
 }
@@ -334,8 +301,8 @@ __global__ void lcp_count_kernel(const int32_t* __restrict__ kseg, const u64* __
        k += (int64_t)gridDim.x * blockDim.x) {
     const bool first = (k == 0) || kseg[k - 1] != kseg[k];
     const bool last = (k + 1 == n) || kseg[k + 1] != kseg[k];
-    const int lk = last ? 0 : common_levels(hi[k], lo[k], hi[k + 1], lo[k + 1]);
-    const int lp = first ? 0 : common_levels(hi[k - 1], lo[k - 1], hi[k], lo[k]);
+    const int lk = last ? 0 : common_levels(hi, lo, k, k + 1);
+    const int lp = first ? 0 : common_levels(hi, lo, k - 1, k);
     if (k + 1 < n) lcp[k] = (uint8_t)lk;
     const int fd = first ? 1 : lp + 1;
     const int top = last ? 0 : min(lk, kMaxDepth - 1);
@@ -353,24 +320,23 @@ __global__ void lcp_count_kernel(const int32_t* __restrict__ kseg, const u64* __
 // and segments contiguous, so the predicate is monotone in j: gallop, then
 // bisect (Karras-style, O(log range)).
 __device__ __forceinline__ bool same_prefix(const int32_t* kseg, const u64* hi, const u64* lo,
-                                            int32_t s0, u64 h0, u64 l0, int64_t j, int d) {
-  return kseg[j] == s0 && common_levels(h0, l0, hi[j], lo[j]) >= d;
+                                            int32_t s0, int64_t k, int64_t j, int d) {
+  return kseg[j] == s0 && common_levels(hi, lo, k, j) >= d;
 }
 
 __device__ __forceinline__ int64_t range_end(const int32_t* __restrict__ kseg,
                                              const u64* __restrict__ hi, const u64* __restrict__ lo,
                                              int64_t n, int64_t k, int d) {
-  const u64 h0 = hi[k], l0 = lo[k];
   const int32_t s0 = kseg[k];
   int64_t good = k, step = 1;
-  while (k + step < n && same_prefix(kseg, hi, lo, s0, h0, l0, k + step, d)) {
+  while (k + step < n && same_prefix(kseg, hi, lo, s0, k, k + step, d)) {
     good = k + step;
     step <<= 1;
   }
   int64_t bad = (k + step < n) ? k + step : n;
   while (bad - good > 1) {
     const int64_t mid = good + ((bad - good) >> 1);
-    if (same_prefix(kseg, hi, lo, s0, h0, l0, mid, d))
+    if (same_prefix(kseg, hi, lo, s0, k, mid, d))
       good = mid;
     else
       bad = mid;
@@ -877,7 +843,7 @@ size_t bh_state_bytes(const BHState* p) {
          h.seg_root.bytes() + h.seg_end.bytes() + h.seg_depth.bytes() + h.mkeys.bytes() + h.mkeys_alt.bytes() + h.midx.bytes() +
          h.midx_alt.bytes() + h.klo.bytes() + h.khi.bytes() + h.khi_alt.bytes() +
          h.pidx.bytes() + h.pidx_alt.bytes() + h.sk.bytes() + h.sk_alt.bytes() + h.kseg.bytes() +
-         h.hist.bytes() + h.scan_ws.bytes() + h.lcp.bytes() + h.ncnt.bytes() + h.nstart.bytes() +
+         h.psort_ws.bytes() + h.hist.bytes() + h.scan_ws.bytes() + h.lcp.bytes() + h.ncnt.bytes() + h.nstart.bytes() +
          h.scalars.bytes() + h.nodes.bytes() +
          h.node_parent.bytes() + h.node_nchild.bytes() + h.node_visit.bytes() +
          h.leaf_of.bytes() + h.ref_nodes.bytes() + h.ref_pos.bytes() + h.spm.bytes() +
@@ -892,7 +858,8 @@ BHState* bh_state_new() { return new BHState(); }
 size_t bh_segment_table_bytes(const int64_t* n_per, int nseg) {
   int64_t ntask = 0;
   for (int s = 0; s < nseg; ++s) ntask += ceil_div(n_per[s], bh_walk_targets(n_per[s]));
-  return ((size_t)nseg * 2 + 1) * sizeof(int64_t) + (size_t)ntask * sizeof(WarpTask);
+  return ((size_t)nseg * 2 + 1) * sizeof(int64_t) + (size_t)ntask * sizeof(WarpTask) +
+         ((size_t)nseg + 1) * sizeof(int32_t);
 }
 
 // Segment tables -- arena offsets, first concatenated index (prefix sums of
@@ -925,6 +892,7 @@ void bh_set_segments(BHState& h, const int64_t* off, const int64_t* n_per, int n
     }
     if (tw == 32) h.ntasks32 = t;
   }
+  h.sort_buckets = path_sort_buckets(n_per, nseg, reinterpret_cast<int32_t*>(ht + t));
   hbase[nseg] = n;
   char* d = grow(h.tables, bytes);
   NBGB_CUDA(cudaMemcpyAsync(d, staging, bytes, cudaMemcpyHostToDevice, st));
@@ -935,6 +903,7 @@ void bh_set_segments(BHState& h, const int64_t* off, const int64_t* n_per, int n
   h.seg_off_p = reinterpret_cast<int64_t*>(d);
   h.seg_base_p = h.seg_off_p + nseg;
   h.tasks_p = reinterpret_cast<WarpTask*>(h.seg_base_p + nseg + 1);
+  h.seg_bucket_p = reinterpret_cast<int32_t*>(h.tasks_p + t);
   int32_t* so = grow(h.seg_of, (size_t)h.reserve);
   seg_of_kernel<<<grid1d(n), 256, 0, st>>>(h.seg_base_p, nseg, n, so);
   NBGB_LAUNCH_CHECK();
@@ -953,12 +922,10 @@ void bh_build(BHState& h, const float4* pm, cudaStream_t st, uint32_t* err, bool
   const size_t R = (size_t)h.reserve;  // per-body buffers are sized for the reserve
   SegView sv{h.seg_off_p, h.seg_base_p, h.seg_of.ptr, grow(h.box, (size_t)nseg)};
   // 1. per-segment bounds and root cubes
-  uint32_t* mm = grow(h.seg_minmax, (size_t)nseg * 6);
-  NBGB_CUDA(cudaMemsetAsync(mm, 0xFF, (size_t)nseg * 3 * sizeof(uint32_t), st));
-  NBGB_CUDA(cudaMemsetAsync(mm + (size_t)nseg * 3, 0x00, (size_t)nseg * 3 * sizeof(uint32_t), st));
-  seg_bounds_kernel<<<(unsigned)ceil_div(n, 1024), 256, 0, st>>>(pm, sv, n, nseg, mm);
-  NBGB_LAUNCH_CHECK();
-  seg_box_kernel<<<(unsigned)ceil_div(nseg, 128), 128, 0, st>>>(mm, nseg, h.box.ptr, err);
+  uint32_t* mm = grow(h.seg_minmax, (size_t)nseg * 6 + 1);
+  NBGB_CUDA(cudaMemsetAsync(mm, 0, ((size_t)nseg * 6 + 1) * sizeof(uint32_t), st));
+  seg_bounds_kernel<<<(unsigned)ceil_div(n, 1024), 256, 0, st>>>(pm, sv, n, nseg, mm, h.box.ptr,
+                                                                 err);
   NBGB_LAUNCH_CHECK();
   // 2. keys and order
   uint32_t* hist = grow(h.hist, radix_hist_elems((int64_t)R));
@@ -969,33 +936,43 @@ void bh_build(BHState& h, const float4* pm, cudaStream_t st, uint32_t* err, bool
   u64* lo = grow(h.klo, R);
   uint32_t* pb = grow(h.pidx, R);
   uint32_t* pb2 = grow(h.pidx_alt, R);
-  stage_mark(timer, "barnes_hut.keys");
-  path_hi_index_kernel<<<grid1d(n), 256, 0, st>>>(pm, sv, n, hi, pb);
-  NBGB_LAUNCH_CHECK();
-  stage_mark(timer, "barnes_hut.sort");
-  bool alt = false;
-  radix_sort_pairs<u64>(hi, hi2, pb, pb2, n, 0, 64, hist, sws, st, &alt, err);
-  uint32_t* body = alt ? pb2 : pb;
-  uint32_t* body_other = alt ? pb : pb2;
-  stage_mark(timer, "barnes_hut.order");
-  if (nseg > 1) {
-    // stable sort by segment: (segment, path) order
-    uint32_t* sk = grow(h.sk, R);
-    uint32_t* sk2 = grow(h.sk_alt, R);
-    seg_key_kernel<<<grid1d(n), 256, 0, st>>>(body, h.seg_of.ptr, n, sk);
-    NBGB_LAUNCH_CHECK();
-    int bits = 1;
-    while (bits < 31 && (1 << bits) < nseg) ++bits;
-    bool alt2 = false;
-    radix_sort_pairs<uint32_t>(sk, sk2, body, body_other, n, 0, ((bits + 7) / 8) * 8, hist, sws,
-                               st, &alt2, err);
-    if (alt2) std::swap(body, body_other);
-  }
-  h.body = body;
   int32_t* kseg = grow(h.kseg, R);
   float4* spm = grow(h.spm, R);
-  path_final_kernel<<<grid1d(n), 256, 0, st>>>(pm, sv, body, n, kseg, hi, lo, spm);
-  NBGB_LAUNCH_CHECK();
+  uint32_t* cnt = grow(h.ncnt, R + 1);
+  uint32_t* body = pb;
+  if (h.sort_buckets > 0) {
+    path_sort(pm, sv, h.seg_bucket_p, h.sort_buckets, n, nseg,
+              PathSortBuffers{grow(h.psort_ws, path_sort_ws_bytes()), lo, cnt, hi2, pb2, pb, kseg,
+                              hi, spm},
+              timer, st);
+    stage_mark(timer, "barnes_hut.order");
+  } else {
+    stage_mark(timer, "barnes_hut.keys");
+    path_hi_index_kernel<<<grid1d(n), 256, 0, st>>>(pm, sv, n, hi, pb);
+    NBGB_LAUNCH_CHECK();
+    stage_mark(timer, "barnes_hut.sort");
+    bool alt = false;
+    radix_sort_pairs<u64>(hi, hi2, pb, pb2, n, 0, 64, hist, sws, st, &alt, err);
+    body = alt ? pb2 : pb;
+    uint32_t* body_other = alt ? pb : pb2;
+    stage_mark(timer, "barnes_hut.order");
+    if (nseg > 1) {
+      // stable sort by segment: (segment, path) order
+      uint32_t* sk = grow(h.sk, R);
+      uint32_t* sk2 = grow(h.sk_alt, R);
+      seg_key_kernel<<<grid1d(n), 256, 0, st>>>(body, h.seg_of.ptr, n, sk);
+      NBGB_LAUNCH_CHECK();
+      int bits = 1;
+      while (bits < 31 && (1 << bits) < nseg) ++bits;
+      bool alt2 = false;
+      radix_sort_pairs<uint32_t>(sk, sk2, body, body_other, n, 0, ((bits + 7) / 8) * 8, hist, sws,
+                                 st, &alt2, err);
+      if (alt2) std::swap(body, body_other);
+    }
+    path_final_kernel<<<grid1d(n), 256, 0, st>>>(pm, sv, body, n, kseg, hi, spm);
+    NBGB_LAUNCH_CHECK();
+  }
+  h.body = body;
   tie_order_kernel<<<grid1d(n), 256, 0, st>>>(sv, n, kseg, hi, body, lo, spm);
   NBGB_LAUNCH_CHECK();
   h.keys_valid = false;  // Morton (key, index) pairs are produced on demand
@@ -1041,7 +1018,6 @@ void bh_build(BHState& h, const float4* pm, cudaStream_t st, uint32_t* err, bool
   // 3.-4. node counts, numbering, emission
   stage_mark(timer, "barnes_hut.nodes");
   uint8_t* lcp = grow(h.lcp, R);
-  uint32_t* cnt = grow(h.ncnt, R + 1);
   uint32_t* nst = grow(h.nstart, R + 1);
   uint32_t* sc = grow(h.scalars, 2);
   lcp_count_kernel<<<grid1d(n), 256, 0, st>>>(kseg, hi, lo, n, lcp, cnt);
@@ -1125,7 +1101,7 @@ void bh_reserve_buffers(BHState& h, bool groups) {
   if (h.cap >= kMaxWalkNodes)
     fail(NBGB_ERR_OVERFLOW, "Barnes-Hut node capacity above 2^30 nodes: too many bodies in one tree build");
   grow(h.box, (size_t)nseg);
-  grow(h.seg_minmax, (size_t)nseg * 6);
+  grow(h.seg_minmax, (size_t)nseg * 6 + 1);
   grow(h.hist, radix_hist_elems((int64_t)R));
   grow(h.scan_ws, scan_workspace_elems((int64_t)radix_hist_elems((int64_t)R)) +
                       scan_workspace_elems((int64_t)R + 1));
@@ -1134,7 +1110,8 @@ void bh_reserve_buffers(BHState& h, bool groups) {
   grow(h.klo, R);
   grow(h.pidx, R);
   grow(h.pidx_alt, R);
-  if (nseg > 1) {
+  grow(h.psort_ws, path_sort_ws_bytes());
+  if (nseg > 1 && h.sort_buckets == 0) {
     grow(h.sk, R);
     grow(h.sk_alt, R);
   }

@@ -50,10 +50,13 @@ __device__ __forceinline__ bool has_next_sibling(const Node* nodes, int skip, in
 
 struct BHState {
   // segment tables (device; single-system calls fill one segment)
-  DevBuf<char> tables;           // seg_off [nseg], seg_base [nseg + 1], tasks [ntasks]
+  DevBuf<char> tables;           // seg_off [nseg], seg_base [nseg + 1], tasks [ntasks],
+                                 // first sort buckets [nseg + 1]
   int64_t* seg_off_p = nullptr;
   int64_t* seg_base_p = nullptr;
   WarpTask* tasks_p = nullptr;
+  int32_t* seg_bucket_p = nullptr;  // path sort: first bucket of each segment
+  int sort_buckets = 0;             // path sort buckets; 0: radix sort
   DevBuf<int32_t> seg_of;
   DevBuf<uint32_t> seg_minmax;   // [6][nseg] ordered-uint encoded bounds
   DevBuf<BBox> box;              // [nseg]
@@ -68,6 +71,7 @@ struct BHState {
   DevBuf<uint32_t> pidx, pidx_alt, sk, sk_alt;
   DevBuf<int32_t> kseg;          // segment of sorted position k
   DevBuf<uint32_t> hist, scan_ws;
+  DevBuf<char> psort_ws;         // path sort: ranks, counts, splitters
   DevBuf<uint8_t> lcp;
   DevBuf<uint32_t> ncnt;    // n + 1
   DevBuf<uint32_t> nstart;  // n + 1
