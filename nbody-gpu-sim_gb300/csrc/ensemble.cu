@@ -189,6 +189,12 @@ constexpr int kNumConfigs = sizeof(kConfigs) / sizeof(kConfigs[0]);
 template <int T, int I, bool P>
 static int occ_of() {
   int b = 0;
+  // the tree build's kernels need up to 195 KB of shared memory on an SM beside
+  // this kernel, which its own 12 KB would not leave (a 24-system burst 19.4 ms
+  // against 19.7)
+  NBGB_CUDA(cudaFuncSetAttribute(ens_direct_kernel<T, I, P>,
+                                 cudaFuncAttributePreferredSharedMemoryCarveout,
+                                 cudaSharedmemCarveoutMaxShared));
   NBGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, ens_direct_kernel<T, I, P>, T, 0));
   return std::max(b, 1);
 }
@@ -204,12 +210,23 @@ static int config_occupancy(int c) {
   }
 }
 
+// `placed`, if given, is recorded when every block of the launch is on an SM.
 static void launch_config(int c, int grid, const DirectItem* items, int n_items, uint32_t* counter,
                           const float4* pm, float* ax, float* ay, float* az, float eps2, float G,
-                          uint32_t* err, cudaStream_t st) {
-#define NBGB_ENS_LAUNCH(T, I, P)                                                             \
-  ens_direct_kernel<T, I, P><<<grid, T, 0, st>>>(items, n_items, counter, pm, ax, ay, az, eps2, \
-                                                 G, err)
+                          uint32_t* err, cudaStream_t st, cudaEvent_t placed) {
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeLaunchCompletionEvent;
+  at[0].val.launchCompletionEvent.event = placed;
+  at[0].val.launchCompletionEvent.flags = 0;
+  cudaLaunchConfig_t lc{};
+  lc.gridDim = dim3((unsigned)grid);
+  lc.blockDim = dim3((unsigned)kConfigs[c].threads);
+  lc.stream = st;
+  lc.attrs = at;
+  lc.numAttrs = placed ? 1 : 0;
+#define NBGB_ENS_LAUNCH(T, I, P)                                                                 \
+  NBGB_CUDA(cudaLaunchKernelEx(&lc, ens_direct_kernel<T, I, P>, items, n_items, counter, pm, ax, \
+                               ay, az, eps2, G, err))
   switch (c) {
     case 0: NBGB_ENS_LAUNCH(128, 4, false); break;
     case 1: NBGB_ENS_LAUNCH(128, 2, false); break;
@@ -388,6 +405,8 @@ struct nbgb_ensemble {
   int tune_cnt[kNumConfigs] = {};
   double tuned_load = 0.0;
   cudaEvent_t ev_kd = nullptr;
+  cudaEvent_t ev_placed = nullptr;  // every block of the tick's direct kernel is on an SM
+  int direct_occ[kNumConfigs] = {};  // blocks per SM of each direct configuration
   // direct-kernel timing ring
   cudaEvent_t tev0[kTimingRing] = {}, tev1[kTimingRing] = {};
   bool tev_used[kTimingRing] = {};
@@ -796,15 +815,8 @@ static void run_tick(nbgb_ensemble* e) {
     NBGB_LAUNCH_CHECK();
   }
   NBGB_CUDA(cudaEventRecord(e->ev_kd, e->main));
-  // 2. all Barnes-Hut systems: one batched pass on the side stream
   const bool bh_work = e->bh_n > 0;
-  if (bh_work) {
-    NBGB_CUDA(cudaStreamWaitEvent(e->bh_stream, e->ev_kd, 0));
-    graph_kernels = run_bh_pass(e);
-    NBGB_CUDA(cudaEventRecord(e->ev_bh, e->bh_stream));
-    e->bh_stable++;
-  }
-  // 3. direct systems: persistent work-queue kernel (always timed)
+  // 2. direct systems: persistent work-queue kernel (always timed)
   if (e->n_items) {
     const int k = e->tev_next % kTimingRing;
     harvest(e, k);
@@ -821,15 +833,27 @@ static void run_tick(nbgb_ensemble* e) {
     // warps, not issue slots) without crowding it out, and still finishes
     // before the walk (serving bench: 5.79 ms per tick vs 5.98 at full
     // occupancy; 2 per SM 5.86, one per two SMs 5.83).  Alone, full occupancy.
-    const int grid = bh_work ? num_sms() : num_sms() * config_occupancy(e->config);
+    // The build waits until these CTAs have their places: with its blocks on the
+    // SMs first, all 152 could end up on 16 of them (a tick 1.49 ms instead of
+    // 0.78, a burst of 24 systems 31 ms instead of 19.4).
+    const int grid = bh_work ? num_sms() : num_sms() * e->direct_occ[e->config];
     launch_config(e->config, grid, e->d_items.ptr, e->n_items, e->d_counter.ptr, e->pm.ptr,
                   e->ax.ptr, e->ay.ptr, e->az.ptr, e->cfg.softening * e->cfg.softening, e->cfg.G,
-                  e->d_err.ptr, e->main);
+                  e->d_err.ptr, e->main, bh_work ? e->ev_placed : nullptr);
     NBGB_CUDA(cudaEventRecord(e->tev1[k], e->main));
     e->tev_used[k] = true;
     e->tev_next++;
     if (e->tuning) e->tune_tick++;
     e->st.direct_interactions += inter;
+  }
+  // 3. all Barnes-Hut systems: one batched pass on the side stream
+  if (bh_work) {
+    NBGB_CUDA(cudaStreamWaitEvent(e->bh_stream, e->ev_kd, 0));
+    // (a matter of places only: the data is ordered by ev_kd)
+    if (e->n_items) NBGB_CUDA(cudaStreamWaitEvent(e->bh_stream, e->ev_placed, 0));
+    graph_kernels = run_bh_pass(e);
+    NBGB_CUDA(cudaEventRecord(e->ev_bh, e->bh_stream));
+    e->bh_stable++;
   }
   if (bh_work) NBGB_CUDA(cudaStreamWaitEvent(e->main, e->ev_bh, 0));
   // 4. bookkeeping and retirement
@@ -935,7 +959,9 @@ nbgb_status nbgb_ensemble_create(const nbgb_ensemble_config* cfg, nbgb_ensemble*
       NBGB_CUDA(cudaEventCreate(&e->wev0[k]));
       NBGB_CUDA(cudaEventCreate(&e->wev1[k]));
     }
+    for (int k = 0; k < kNumConfigs; ++k) e->direct_occ[k] = config_occupancy(k);
     NBGB_CUDA(cudaEventCreateWithFlags(&e->ev_kd, cudaEventDisableTiming));
+    NBGB_CUDA(cudaEventCreateWithFlags(&e->ev_placed, cudaEventDisableTiming));
     NBGB_CUDA(cudaEventCreateWithFlags(&e->ev_bh, cudaEventDisableTiming));
     e->d_bh_inter.ensure(1);
     NBGB_CUDA(cudaMemset(e->d_bh_inter.ptr, 0, sizeof(unsigned long long)));
@@ -964,6 +990,7 @@ nbgb_status nbgb_ensemble_destroy(nbgb_ensemble* e) {
       cudaEventDestroy(e->wev1[k]);
     }
     cudaEventDestroy(e->ev_kd);
+    cudaEventDestroy(e->ev_placed);
     if (e->stage_evt) cudaEventDestroy(e->stage_evt);
     cudaStreamDestroy(e->main);
     delete e;
