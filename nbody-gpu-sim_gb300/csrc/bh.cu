@@ -91,7 +91,14 @@ __device__ __forceinline__ float ord2f(uint32_t u) {
 // last block derives the boxes.  Min/max are exact, so the result equals the
 // reference's computeBoundingBoxKernel (:78-122).  mm holds [6][nseg] maxima of
 // order-preserving integers (minima as the maxima of their complements) and a
-// block counter, all zero before the launch.
+// block counter, all zero before the launch and left zero for the next; the last
+// block also clears the counters that the rest of the build starts from (a
+// memset each would cost as much as a small kernel).
+struct ZeroList {
+  uint32_t* p[3];
+  uint32_t words[3];
+};
+
 __device__ __forceinline__ void seg_box(const uint32_t* mm, int nseg, int s, BBox* box,
                                         uint32_t* err) {
   BBox o;
@@ -117,7 +124,7 @@ __device__ __forceinline__ void seg_box(const uint32_t* mm, int nseg, int s, BBo
 
 __global__ void seg_bounds_kernel(const float4* __restrict__ pm, SegView sv, int64_t n, int nseg,
                                   uint32_t* __restrict__ mm, BBox* __restrict__ box,
-                                  uint32_t* err) {
+                                  ZeroList zero, uint32_t* err) {
   __shared__ float s_red[32][6];
   __shared__ int s_same;
   __shared__ bool s_last;
@@ -180,6 +187,11 @@ __global__ void seg_bounds_kernel(const float4* __restrict__ pm, SegView sv, int
   if (!s_last) return;
   __threadfence();
   for (int s = threadIdx.x; s < nseg; s += blockDim.x) seg_box(mm, nseg, s, box, err);
+  __syncthreads();
+  for (int i = threadIdx.x; i < 6 * nseg + 1; i += blockDim.x) mm[i] = 0;
+#pragma unroll
+  for (int z = 0; z < 3; ++z)
+    for (uint32_t i = threadIdx.x; i < zero.words[z]; i += blockDim.x) zero.p[z][i] = 0;
 }
 
 // High path key of every body in concatenated order (values = indices).
@@ -280,268 +292,6 @@ __global__ void morton_scatter_kernel(const float4* __restrict__ spm,
     keys[i] = morton_of(spm[k], b);
     idx[i] = i;
   }
-}
-
-// Common levels of sorted bodies i and j (low keys are written, and read, only
-// where the high keys agree).
-__device__ __forceinline__ int common_levels(const u64* hi, const u64* lo, int64_t i, int64_t j) {
-  const u64 h0 = hi[i], h1 = hi[j];
-  if (h0 != h1) return (__clzll(h0 ^ h1) - 1) / 3;  // bit 63 unused
-  const u64 l0 = lo[i], l1 = lo[j];
-  if (l0 != l1) return kHiLevels + (__clzll(l0 ^ l1) - 31) / 3;  // bits 63..33 unused
-  return kMaxDepth;
-}
-
-// l_k (0 across a segment boundary) and per-body node counts: internal +
-// leaf, + the root at the first body of a segment.
-__global__ void lcp_count_kernel(const int32_t* __restrict__ kseg, const u64* __restrict__ hi,
-                                 const u64* __restrict__ lo, int64_t n, uint8_t* __restrict__ lcp,
-                                 uint32_t* __restrict__ cnt) {
-  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n;
-       k += (int64_t)gridDim.x * blockDim.x) {
-    const bool first = (k == 0) || kseg[k - 1] != kseg[k];
-    const bool last = (k + 1 == n) || kseg[k + 1] != kseg[k];
-    const int lk = last ? 0 : common_levels(hi, lo, k, k + 1);
-    const int lp = first ? 0 : common_levels(hi, lo, k - 1, k);
-    if (k + 1 < n) lcp[k] = (uint8_t)lk;
-    const int fd = first ? 1 : lp + 1;
-    const int top = last ? 0 : min(lk, kMaxDepth - 1);
-    uint32_t c = (uint32_t)max(0, top - fd + 1);
-    const bool leaf_start = first || (lp < kMaxDepth);
-    c += leaf_start ? 1u : 0u;
-    if (first) c += 1u;  // the segment's root
-    cnt[k] = c;
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0) cnt[n] = 0;
-}
-
-// Range end of the depth-d node that contains sorted body k: the largest j of
-// the same segment with common_levels(key_k, key_j) >= d.  Keys are sorted
-// and segments contiguous, so the predicate is monotone in j: gallop, then
-// bisect (Karras-style, O(log range)).
-__device__ __forceinline__ bool same_prefix(const int32_t* kseg, const u64* hi, const u64* lo,
-                                            int32_t s0, int64_t k, int64_t j, int d) {
-  return kseg[j] == s0 && common_levels(hi, lo, k, j) >= d;
-}
-
-__device__ __forceinline__ int64_t range_end(const int32_t* __restrict__ kseg,
-                                             const u64* __restrict__ hi, const u64* __restrict__ lo,
-                                             int64_t n, int64_t k, int d) {
-  const int32_t s0 = kseg[k];
-  int64_t good = k, step = 1;
-  while (k + step < n && same_prefix(kseg, hi, lo, s0, k, k + step, d)) {
-    good = k + step;
-    step <<= 1;
-  }
-  int64_t bad = (k + step < n) ? k + step : n;
-  while (bad - good > 1) {
-    const int64_t mid = good + ((bad - good) >> 1);
-    if (same_prefix(kseg, hi, lo, s0, k, mid, d))
-      good = mid;
-    else
-      bad = mid;
-  }
-  return good;
-}
-
-struct EmitArgs {
-  const int32_t* kseg;
-  const uint8_t* lcp;
-  const u64* hi;
-  const u64* lo;
-  const uint32_t* nstart;
-  const float4* spm;
-  const BBox* box;
-  const int64_t* base;  // segment s occupies sorted positions [base[s], base[s+1])
-  int64_t n;
-  int64_t cap;
-  Node* nodes;
-  int32_t* parent;
-  int32_t* visit;
-  int32_t* seg_root;
-  int32_t* seg_end;
-  int32_t* seg_depth;
-  int32_t* leaf_of;  // per sorted body: the leaf node it starts, or -1
-  uint32_t* err;
-};
-
-__global__ void emit_nodes_kernel(EmitArgs a) {
-  const uint32_t total = a.nstart[a.n];
-  if ((int64_t)total > a.cap) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) raise_error(a.err, kErrTreeCapacity);
-    return;
-  }
-  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < a.n;
-       k += (int64_t)gridDim.x * blockDim.x) {
-    const int32_t s = a.kseg[k];
-    const bool first = (k == 0) || a.kseg[k - 1] != s;
-    const bool last = (k + 1 == a.n) || a.kseg[k + 1] != s;
-    const int lk = last ? 0 : (int)a.lcp[k];
-    const int lp = first ? 0 : (int)a.lcp[k - 1];
-    const int fd = first ? 1 : lp + 1;
-    const int top = last ? 0 : min(lk, kMaxDepth - 1);
-    uint32_t idx = a.nstart[k];
-    const float4 p = a.spm[k];
-    const BBox b = a.box[s];
-    if (first) {
-      const int64_t send = a.base[s + 1];  // one past the segment's last position
-      const uint32_t skip = (send < a.n) ? a.nstart[send] : total;
-      a.nodes[idx].geom = make_float4(b.center[0], b.center[1], b.center[2], b.half);
-      a.nodes[idx].info = make_int4((int)skip, 0, (int)k, (int)(send - k));
-      a.parent[idx] = -1;
-      a.visit[idx] = 0;
-      a.seg_root[s] = (int32_t)idx;
-      a.seg_end[s] = (int32_t)skip;
-      ++idx;
-    }
-    // internal nodes of depth fd..top: slots claimed here (owner = k in
-    // parent[]); their cubes are written below on the way down to k's leaf
-    // (every owned depth lies above it), the rest by internal_nodes_kernel,
-    // one thread per node
-    const int n_int = max(0, top - fd + 1);
-    const uint32_t int0 = idx;
-    for (int j = 0; j < n_int; ++j) a.parent[idx + j] = (int32_t)k;
-    idx += n_int;
-    const bool leaf_start = first || (lp < kMaxDepth);
-    int md = -1;
-    if (!leaf_start) a.leaf_of[k] = -1;
-    if (leaf_start) {
-      const int ld = min(kMaxDepth, max(lp, lk) + 1);
-      float cx = b.center[0], cy = b.center[1], cz = b.center[2], h = b.half;
-      for (int lev = 1; lev <= ld; ++lev) {
-        const uint32_t o = (p.x >= cx ? 1u : 0u) | (p.y >= cy ? 2u : 0u) | (p.z >= cz ? 4u : 0u);
-        const float hs = __fmul_rn(h, 0.5f);
-        cx = __fadd_rn(cx, (o & 1u) ? hs : -hs);
-        cy = __fadd_rn(cy, (o & 2u) ? hs : -hs);
-        cz = __fadd_rn(cz, (o & 4u) ? hs : -hs);
-        h = hs;
-        if (lev >= fd && lev <= top) a.nodes[int0 + (lev - fd)].geom = make_float4(cx, cy, cz, h);
-      }
-      int64_t e = k;
-      while (e + 1 < a.n && a.kseg[e + 1] == s && (int)a.lcp[e] >= kMaxDepth) ++e;
-      a.nodes[idx].geom = make_float4(cx, cy, cz, h);
-      a.nodes[idx].info = make_int4((int)(idx + 1), (ld << 8) | 1, (int)k, (int)(e - k + 1));
-      a.parent[idx] = -1;
-      a.visit[idx] = 0;
-      a.leaf_of[k] = (int32_t)idx;
-      // reference max_depth_: depth of the inserting body's last loop level
-      md = (ld == kMaxDepth && e > k) ? kMaxDepth : ld - 1;
-    }
-    // per-segment maximum: reduced over the lanes of the same segment, one
-    // atomic per group and only while it can still raise the stored value
-    const unsigned peers = __match_any_sync(__activemask(), s);
-    const int gmax = __reduce_max_sync(peers, md);
-    if ((int)(threadIdx.x & 31) == __ffs(peers) - 1 && gmax > __ldcg(&a.seg_depth[s]))
-      atomicMax(&a.seg_depth[s], gmax);
-  }
-}
-
-// Internal nodes, one thread per node: the owner body k (the first body of
-// the node's range) and the depth follow from k's slot numbering, the range
-// end from a search over the sorted keys (the cube was written by
-// emit_nodes_kernel on k's path).
-__global__ void internal_nodes_kernel(EmitArgs a) {
-  const uint32_t total = a.nstart[a.n];
-  if ((int64_t)total > a.cap) return;
-  for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < (int64_t)total;
-       q += (int64_t)gridDim.x * blockDim.x) {
-    const int32_t k32 = a.parent[q];
-    if (k32 < 0) continue;  // a root or a leaf
-    const int64_t k = k32;
-    const int32_t s = a.kseg[k];
-    const bool first = (k == 0) || a.kseg[k - 1] != s;
-    const int fd = first ? 1 : (int)a.lcp[k - 1] + 1;
-    const int d = fd + (int)(q - (int64_t)a.nstart[k]) - (first ? 1 : 0);
-    const int64_t e = range_end(a.kseg, a.hi, a.lo, a.n, k, d);
-    const uint32_t skip = (e + 1 < a.n) ? a.nstart[e + 1] : total;
-    a.nodes[q].info = make_int4((int)skip, d << 8, (int)k, (int)(e - k + 1));
-    a.visit[q] = 0;
-  }
-}
-
-// Where link_kernel writes the group walk's groups.
-struct GroupSink {
-  const uint32_t* body;  // path-sorted position -> concatenated body index
-  const int32_t* seg_of;
-  int4* groups;          // first body, count, segment: classes 0 and 1
-  int4* groups2;         // classes 2 and 3
-  GroupCounters* gc;
-  int gmax;              // largest group (32 or 64 bodies)
-  int64_t gcap;          // groups capacity
-  const uint32_t* body_cost;           // last walk's cost per body
-  const unsigned long long* cost_acc;  // last walk's total cost, groups
-};
-
-// Parent links and child counts (children of P: P+1, skip(P+1), ... < skip(P)).
-// With GROUPS it also emits the group walk's groups: roots with at most
-// gmax bodies; below larger nodes, runs of consecutive children with at
-// most gmax bodies in total (merged only when the parent holds at most
-// kGroupMergeMax bodies: sibling cells of a large sparse node can lie far
-// apart); depth-32 leaves larger than a group are split.  Every body
-// belongs to exactly one group, and a group is one contiguous range of
-// path-sorted bodies.  Groups go to four cost classes (GroupCounters) by
-// the last walk's cost of their first body's group: classes 0 and 1 to the
-// front and back of groups, 2 and 3 to those of groups2; the walk takes
-// class 0 first, so the longest groups start early and its last tasks are
-// short ones.
-template <bool GROUPS>
-__global__ void link_kernel(const Node* __restrict__ nodes, const uint32_t* __restrict__ nstart,
-                            int64_t n, int64_t cap, int32_t* __restrict__ parent,
-                            int32_t* __restrict__ nchild, GroupSink gs) {
-  const uint32_t total = nstart[n];
-  if ((int64_t)total > cap) return;
-  const int gmax = gs.gmax;
-  unsigned long long mean = ~0ull;  // no estimates before the first walk
-  if (GROUPS && gs.cost_acc[1]) mean = gs.cost_acc[0] / gs.cost_acc[1];
-  auto emit = [&](int f, int c) {
-    const uint32_t b = gs.body[f];
-    const unsigned long long e = gs.body_cost[b];
-    const int cls = mean == ~0ull ? 3 : (e > 2 * mean ? 0 : (e > mean ? 1 : (2 * e > mean ? 2 : 3)));
-    const uint32_t k = atomicAdd(&gs.gc->nclass[cls], 1u);
-    int4* arr = cls < 2 ? gs.groups : gs.groups2;
-    const int64_t g = (cls & 1) ? gs.gcap - 1 - (int64_t)k : (int64_t)k;
-    arr[g] = make_int4(f, c, gs.seg_of[b], 0);
-  };
-  for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < (int64_t)total;
-       p += (int64_t)gridDim.x * blockDim.x) {
-    const int4 ip = nodes[p].info;  // skip, depth << 8 | leaf, first, count
-    if (ip.y & 1) {
-      nchild[p] = 0;
-      if (GROUPS && ip.w > gmax)
-        for (int f = 0; f < ip.w; f += gmax) emit(ip.z + f, min(gmax, ip.w - f));
-      continue;
-    }
-    if (GROUPS && (ip.y >> 8) == 0 && ip.w <= gmax) emit(ip.z, ip.w);  // a small root
-    const bool grp = GROUPS && ip.w > gmax, merge = ip.w <= kGroupMergeMax;
-    int c = (int)p + 1, nc = 0, gf = 0, gn = 0;
-    while (c < ip.x) {
-      parent[c] = (int)p;
-      ++nc;
-      const int4 ci = nodes[c].info;
-      if (grp) {
-        if (ci.w > gmax) {
-          if (gn) emit(gf, gn);
-          gn = 0;
-        } else if (gn && merge && gn + ci.w <= gmax) {
-          gn += ci.w;
-        } else {
-          if (gn) emit(gf, gn);
-          gf = ci.z;
-          gn = ci.w;
-        }
-      }
-      c = ci.x;
-    }
-    if (grp && gn) emit(gf, gn);
-    nchild[p] = nc;
-  }
-}
-
-// Arrival counter increment with acquire-release ordering at GPU scope.
-__device__ __forceinline__ int arrive_acq_rel(int32_t* p) {
-  int old;
-  asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(old) : "l"(p) : "memory");
-  return old;
 }
 
 // --------------------------------------------- reference-identical tree --
@@ -771,65 +521,6 @@ __global__ void ref_tree_kernel(RefTreeArgs a) {
   a.seg_depth[0] = max_depth;
 }
 
-constexpr int kComThreads = 64;
-
-// Leaves: mass/com as the reference's allocateLeaf + mergeParticleIntoLeaf
-// (force_barnes_hut.cu:355-389); then the last-arriving child of each node
-// computes that node from all its children in octant order (:514-538).
-__global__ void com_kernel(Node* __restrict__ nodes, const float4* __restrict__ spm,
-                           const uint32_t* __restrict__ nstart, int64_t n, int64_t cap,
-                           const int32_t* __restrict__ parent, const int32_t* __restrict__ nchild,
-                           int32_t* __restrict__ visit, const int32_t* __restrict__ leaf_of) {
-  const uint32_t total = nstart[n];
-  if ((int64_t)total > cap) return;
-  // one thread per sorted body; the bodies that start a leaf carry it
-  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n;
-       k += (int64_t)gridDim.x * blockDim.x) {
-    const int32_t p = leaf_of[k];
-    if (p < 0) continue;
-    const int4 ip = nodes[p].info;
-    float4 b0 = spm[ip.z];
-    float m = b0.w, cx = b0.x, cy = b0.y, cz = b0.z;
-    for (int j = 1; j < ip.w; ++j) {
-      const float4 q = spm[ip.z + j];
-      const float t = __fadd_rn(m, q.w);
-      cx = __fdiv_rn(__fadd_rn(__fmul_rn(cx, m), __fmul_rn(q.x, q.w)), t);
-      cy = __fdiv_rn(__fadd_rn(__fmul_rn(cy, m), __fmul_rn(q.y, q.w)), t);
-      cz = __fdiv_rn(__fadd_rn(__fmul_rn(cz, m), __fmul_rn(q.z, q.w)), t);
-      m = t;
-    }
-    nodes[p].com = make_float4(cx, cy, cz, m);
-    int node = parent[p];
-    nodes[p].walk = walk_record(ip, nodes[p].geom.w, m, has_next_sibling(nodes, ip.x, node));
-    while (node >= 0) {
-      // release: this child's centre of mass is visible to the sibling that
-      // arrives last; acquire: the last one sees every sibling's
-      if (arrive_acq_rel(&visit[node]) != nchild[node] - 1) break;
-      const int4 in = nodes[node].info;
-      float tm = 0.f, sx = 0.f, sy = 0.f, sz = 0.f;
-      int c = node + 1;
-      while (c < in.x) {
-        const float4 q = __ldcg(&nodes[c].com);
-        tm = __fadd_rn(tm, q.w);
-        sx = __fadd_rn(sx, __fmul_rn(q.x, q.w));
-        sy = __fadd_rn(sy, __fmul_rn(q.y, q.w));
-        sz = __fadd_rn(sz, __fmul_rn(q.z, q.w));
-        c = nodes[c].info.x;
-      }
-      float4 r = make_float4(0.f, 0.f, 0.f, tm);
-      if (tm > 0.0f) {
-        r.x = __fdiv_rn(sx, tm);
-        r.y = __fdiv_rn(sy, tm);
-        r.z = __fdiv_rn(sz, tm);
-      }
-      __stcg(&nodes[node].com, r);
-      const int up = parent[node];
-      nodes[node].walk = walk_record(in, nodes[node].geom.w, r.w, has_next_sibling(nodes, in.x, up));
-      node = up;
-    }
-  }
-}
-
 static unsigned grid1d(int64_t n, int threads = 256) {
   return (unsigned)std::max<int64_t>(
       1, std::min<int64_t>(ceil_div(std::max<int64_t>(n, 1), threads), (int64_t)num_sms() * 32));
@@ -845,7 +536,7 @@ size_t bh_state_bytes(const BHState* p) {
          h.pidx.bytes() + h.pidx_alt.bytes() + h.sk.bytes() + h.sk_alt.bytes() + h.kseg.bytes() +
          h.psort_ws.bytes() + h.hist.bytes() + h.scan_ws.bytes() + h.lcp.bytes() + h.ncnt.bytes() + h.nstart.bytes() +
          h.scalars.bytes() + h.nodes.bytes() +
-         h.node_parent.bytes() + h.node_nchild.bytes() + h.node_visit.bytes() +
+         h.node_parent.bytes() +
          h.leaf_of.bytes() + h.ref_nodes.bytes() + h.ref_pos.bytes() + h.spm.bytes() +
          h.walk_ctr.bytes() + h.groups.bytes() + h.groups2.bytes() + h.body_cost.bytes() + h.cost_acc.bytes() +
          h.group_ctr.bytes() + h.group_ovf.bytes();
@@ -909,6 +600,14 @@ void bh_set_segments(BHState& h, const int64_t* off, const int64_t* n_per, int n
   NBGB_LAUNCH_CHECK();
 }
 
+// The bounds kernel's maxima: zero when allocated, and left zero by the kernel.
+static uint32_t* seg_minmax_zeroed(BHState& h, cudaStream_t st) {
+  const size_t old = h.seg_minmax.cap;
+  uint32_t* mm = grow(h.seg_minmax, (size_t)h.nseg * 6 + 1);
+  if (h.seg_minmax.cap != old) NBGB_CUDA(cudaMemsetAsync(mm, 0, h.seg_minmax.bytes(), st));
+  return mm;
+}
+
 // Builds the trees of all segments (positions and masses read from `pm` at
 // each segment's offset).
 void bh_build(BHState& h, const float4* pm, cudaStream_t st, uint32_t* err, bool groups,
@@ -922,10 +621,15 @@ void bh_build(BHState& h, const float4* pm, cudaStream_t st, uint32_t* err, bool
   const size_t R = (size_t)h.reserve;  // per-body buffers are sized for the reserve
   SegView sv{h.seg_off_p, h.seg_base_p, h.seg_of.ptr, grow(h.box, (size_t)nseg)};
   // 1. per-segment bounds and root cubes
-  uint32_t* mm = grow(h.seg_minmax, (size_t)nseg * 6 + 1);
-  NBGB_CUDA(cudaMemsetAsync(mm, 0, ((size_t)nseg * 6 + 1) * sizeof(uint32_t), st));
+  uint32_t* mm = seg_minmax_zeroed(h, st);
+  const ZeroList zero{
+      {reinterpret_cast<uint32_t*>(grow(h.psort_ws, path_sort_ws_bytes())),
+       reinterpret_cast<uint32_t*>(grow(h.seg_depth, (size_t)nseg + 2)),
+       reinterpret_cast<uint32_t*>(grow(h.group_ctr, sizeof(GroupCounters)))},
+      {h.sort_buckets > 0 ? (uint32_t)path_sort_zero_words() : 0u, (uint32_t)nseg + 2,
+       (uint32_t)(sizeof(GroupCounters) / sizeof(uint32_t))}};
   seg_bounds_kernel<<<(unsigned)ceil_div(n, 1024), 256, 0, st>>>(pm, sv, n, nseg, mm, h.box.ptr,
-                                                                 err);
+                                                                 zero, err);
   NBGB_LAUNCH_CHECK();
   // 2. keys and order
   uint32_t* hist = grow(h.hist, radix_hist_elems((int64_t)R));
@@ -1015,64 +719,8 @@ void bh_build(BHState& h, const float4* pm, cudaStream_t st, uint32_t* err, bool
     h.built = true;
     return;
   }
-  // 3.-4. node counts, numbering, emission
-  stage_mark(timer, "barnes_hut.nodes");
-  uint8_t* lcp = grow(h.lcp, R);
-  uint32_t* nst = grow(h.nstart, R + 1);
-  uint32_t* sc = grow(h.scalars, 2);
-  lcp_count_kernel<<<grid1d(n), 256, 0, st>>>(kseg, hi, lo, n, lcp, cnt);
-  NBGB_LAUNCH_CHECK();
-  scan_exclusive_u32(cnt, nst, n + 1, sws, sc, st);
-  int32_t* sdepth = grow(h.seg_depth, (size_t)nseg);
-  NBGB_CUDA(cudaMemsetAsync(sdepth, 0, (size_t)nseg * sizeof(int32_t), st));
-  const int64_t min_cap = 2 * n + 64 * (int64_t)nseg;
-  if (h.cap < min_cap) h.cap = 3 * n + 64 * (int64_t)nseg;
-  if (h.cap >= kMaxWalkNodes)
-    fail(NBGB_ERR_OVERFLOW, "Barnes-Hut node capacity above 2^30 nodes: too many bodies in one tree build");
-  Node* nodes = grow(h.nodes, (size_t)h.cap);
-  int32_t* par = grow(h.node_parent, (size_t)h.cap);
-  int32_t* nch = grow(h.node_nchild, (size_t)h.cap);
-  int32_t* vis = grow(h.node_visit, (size_t)h.cap);
-  int32_t* leaf_of = grow(h.leaf_of, R);
-  EmitArgs ea{kseg, lcp, hi, lo, nst, spm, h.box.ptr, h.seg_base_p, n, h.cap, nodes, par,
-              vis, grow(h.seg_root, (size_t)nseg), grow(h.seg_end, (size_t)nseg), sdepth,
-              leaf_of, err};
-  emit_nodes_kernel<<<grid1d(n), 256, 0, st>>>(ea);
-  NBGB_LAUNCH_CHECK();
-  internal_nodes_kernel<<<grid1d(h.cap), 256, 0, st>>>(ea);
-  NBGB_LAUNCH_CHECK();
-  if (groups) {
-    h.group_max = group_max > 0 ? group_max : bh_group_max(n);
-    uint32_t* bc_old = h.body_cost.ptr;
-    uint32_t* bc = grow(h.body_cost, R);
-    if (bc != bc_old) NBGB_CUDA(cudaMemsetAsync(bc, 0, h.body_cost.cap * sizeof(uint32_t), st));
-    unsigned long long* acc_old = h.cost_acc.ptr;
-    unsigned long long* acc = grow(h.cost_acc, 2);
-    if (acc != acc_old) NBGB_CUDA(cudaMemsetAsync(acc, 0, 2 * sizeof(unsigned long long), st));
-    int4* gr = grow(h.groups, R);
-    int4* gr2 = h.groups2.ensure(h.groups.cap);
-    GroupSink gs{h.body, h.seg_of.ptr, gr, gr2,
-                 reinterpret_cast<GroupCounters*>(grow(h.group_ctr, sizeof(GroupCounters))),
-                 h.group_max, (int64_t)h.groups.cap, bc, acc};
-    NBGB_CUDA(cudaMemsetAsync(gs.gc, 0, sizeof(GroupCounters), st));
-    link_kernel<true><<<grid1d(h.cap), 256, 0, st>>>(nodes, nst, n, h.cap, par, nch, gs);
-    NBGB_LAUNCH_CHECK();
-    // the coming walk adds up its own costs
-    NBGB_CUDA(cudaMemsetAsync(acc, 0, 2 * sizeof(unsigned long long), st));
-  } else {
-    link_kernel<false><<<grid1d(h.cap), 256, 0, st>>>(nodes, nst, n, h.cap, par, nch, GroupSink{});
-  }
-  NBGB_LAUNCH_CHECK();
-  h.groups_ready = groups;
-  // one thread per body that starts a leaf (found through leaf_of, so no
-  // thread idles on an unused node slot): it carries centres of mass up the
-  // tree, so bodies are not chained per thread (one resident wave of threads
-  // striding over the node slots was 0.3 ms per serving tick slower); blocks
-  // of two warps, so that a block waiting for one long climb holds few slots
-  stage_mark(timer, "barnes_hut.com");
-  com_kernel<<<(unsigned)ceil_div(std::max<int64_t>(n, 1), kComThreads), kComThreads, 0, st>>>(
-      nodes, spm, nst, n, h.cap, par, nch, vis, leaf_of);
-  NBGB_LAUNCH_CHECK();
+  // 3.-5. nodes, groups, centres of mass (bh_nodes.cu)
+  bh_nodes(h, groups, group_max, err, timer, st);
   h.built = true;
 }
 
@@ -1101,7 +749,15 @@ void bh_reserve_buffers(BHState& h, bool groups) {
   if (h.cap >= kMaxWalkNodes)
     fail(NBGB_ERR_OVERFLOW, "Barnes-Hut node capacity above 2^30 nodes: too many bodies in one tree build");
   grow(h.box, (size_t)nseg);
-  grow(h.seg_minmax, (size_t)nseg * 6 + 1);
+  {
+    // zero for the bounds kernel, complete before any stream of the caller uses it
+    const size_t old = h.seg_minmax.cap;
+    grow(h.seg_minmax, (size_t)nseg * 6 + 1);
+    if (h.seg_minmax.cap != old) {
+      NBGB_CUDA(cudaMemset(h.seg_minmax.ptr, 0, h.seg_minmax.bytes()));
+      NBGB_CUDA(cudaDeviceSynchronize());
+    }
+  }
   grow(h.hist, radix_hist_elems((int64_t)R));
   grow(h.scan_ws, scan_workspace_elems((int64_t)radix_hist_elems((int64_t)R)) +
                       scan_workspace_elems((int64_t)R + 1));
@@ -1117,15 +773,13 @@ void bh_reserve_buffers(BHState& h, bool groups) {
   }
   grow(h.kseg, R);
   grow(h.spm, R);
-  grow(h.lcp, R);
+  grow(h.lcp, lcp_bytes((int64_t)R));
   grow(h.ncnt, R + 1);
   grow(h.nstart, R + 1);
   grow(h.scalars, 2);
-  grow(h.seg_depth, (size_t)nseg);
+  grow(h.seg_depth, (size_t)nseg + 2);
   grow(h.nodes, (size_t)h.cap);
   grow(h.node_parent, (size_t)h.cap);
-  grow(h.node_nchild, (size_t)h.cap);
-  grow(h.node_visit, (size_t)h.cap);
   grow(h.leaf_of, R);
   grow(h.seg_root, (size_t)nseg);
   grow(h.seg_end, (size_t)nseg);

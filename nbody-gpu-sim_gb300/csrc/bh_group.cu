@@ -516,8 +516,7 @@ void bh_group_walk(BHState& h, const BHWalkParams& p, float* ax, float* ay, floa
   int4* groups = h.groups.ptr;
   GroupCounters* gc = reinterpret_cast<GroupCounters*>(h.group_ctr.ptr);
   int* ovf = grow(h.group_ovf, (size_t)kOvfChunks * kOvfChunk);
-  // the walk's task and overflow counters (the group count stays)
-  NBGB_CUDA(cudaMemsetAsync(&gc->task, 0, 2 * sizeof(uint32_t), st));
+  // the walk's task and overflow counters were cleared by the build
   GroupWalkArgs g;
   g.nodes = h.nodes.ptr;
   g.spm = h.spm.ptr;

@@ -72,13 +72,13 @@ struct BHState {
   DevBuf<int32_t> kseg;          // segment of sorted position k
   DevBuf<uint32_t> hist, scan_ws;
   DevBuf<char> psort_ws;         // path sort: ranks, counts, splitters
-  DevBuf<uint8_t> lcp;
-  DevBuf<uint32_t> ncnt;    // n + 1
+  DevBuf<uint8_t> lcp;      // common levels of neighbours, and minima over 32, 1024, ... of them
+  DevBuf<uint32_t> ncnt;    // n + 1 (sort scratch)
   DevBuf<uint32_t> nstart;  // n + 1
   DevBuf<uint32_t> scalars; // [0] total nodes
   HostPinned<uint32_t> h_scalars;
   DevBuf<Node> nodes;
-  DevBuf<int32_t> node_parent, node_nchild, node_visit;
+  DevBuf<int32_t> node_parent;
   DevBuf<int32_t> leaf_of;  // per sorted body: the leaf it starts, or -1
   DevBuf<char> ref_nodes;   // reference-identical build: the reference's node array
   DevBuf<int32_t> ref_pos;  // reference-identical build: original index -> sorted position
@@ -172,5 +172,10 @@ void bh_reference_walk(BHState& h, const BHWalkParams& p, float* ax, float* ay, 
                        int32_t* counts, unsigned long long* inter_total, cudaStream_t st);
 // Stack entries the walks use (bh_set_group_stack_limit).
 int bh_group_stack_limit();
+
+// Nodes, groups and centres of mass of the sorted bodies (bh_nodes.cu).
+void bh_nodes(BHState& h, bool groups, int group_max, uint32_t* err, StageTimer* timer,
+              cudaStream_t st);
+size_t lcp_bytes(int64_t n);
 
 }  // namespace nbgb

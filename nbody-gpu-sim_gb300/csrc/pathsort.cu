@@ -41,7 +41,7 @@ struct __align__(16) SplitKey {
 };
 
 struct PsWork {
-  // zeroed for each sort
+  // zero before each sort (the bounds kernel clears it)
   uint32_t rank[kPsMaxSamples];
   uint32_t count[kPsMaxBuckets];
   uint32_t done[kPsMaxSamples / 256 + 4];  // CTAs done: per 256 samples; [last] counting
@@ -53,6 +53,7 @@ struct PsWork {
 };
 
 size_t path_sort_ws_bytes() { return sizeof(PsWork); }
+size_t path_sort_zero_words() { return offsetof(PsWork, offset) / sizeof(uint32_t); }
 
 int path_sort_buckets(const int64_t* n_per, int nseg, int32_t* first) {
   int64_t n = 0;
@@ -438,7 +439,6 @@ void path_sort(const float4* pm, const SegView& sv, const int32_t* first, int nb
                         : std::max(4, std::min(kPsMaxOver, 2048 / nb));
   a.w = reinterpret_cast<PsWork*>(b.ws);
   a.b = b;
-  NBGB_CUDA(cudaMemsetAsync(a.w, 0, offsetof(PsWork, offset), st));
   const int ns = nb * a.over;
   const dim3 g((unsigned)ceil_div(ns, 256), (unsigned)ceil_div(ns, kPsChunk));
   ps_sample_kernel<<<(unsigned)ceil_div(ns, 64), 64, 0, st>>>(a);

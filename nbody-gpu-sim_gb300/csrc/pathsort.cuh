@@ -29,6 +29,7 @@ struct PathSortBuffers {
 };
 
 size_t path_sort_ws_bytes();
+size_t path_sort_zero_words();  // leading words of ws that are zero before a sort
 // first: path_sort_buckets' table on the device, nb their number (above 0).
 void path_sort(const float4* pm, const SegView& sv, const int32_t* first, int nb, int64_t n,
                int nseg, const PathSortBuffers& b, StageTimer* timer, cudaStream_t st);
