@@ -1,8 +1,8 @@
 // bh_group.cu -- the Barnes-Hut group walk (NBGB_FLAG_GROUP_WALK): one
-// interaction list per group of at most 32 or 64 nearby bodies, built by one
-// warp that tests 32 nodes at a time and evaluated by all its lanes.  Groups
-// come from the tree build (link_kernel in bh.cu), filed in cost classes
-// learned from the previous walk.
+// interaction list per group of at most 32 or 64 nearby bodies, built by one,
+// two or four warps that test 32 nodes each at a time and evaluated by all their
+// lanes.  Groups come from the tree build (groups_kernel in bh_nodes.cu), filed
+// in cost classes learned from the previous walk.
 #include <algorithm>
 #include <atomic>
 
@@ -14,7 +14,7 @@ namespace nbgb {
 // ---------------------------------------------------------- group walk --
 // Barnes-Hut with a per-group opening test: the bodies of one small subtree
 // (or of consecutive small sibling subtrees, at most 64 bodies) share one
-// interaction list, built by one warp that tests 32 nodes at a time.  A cell
+// interaction list, built by warps that test 32 nodes at a time.  A cell
 // is accepted for the whole group when its cube does not touch the group's
 // bounding box and size2 < theta2 (d_min^2 + eps^2), d_min being the distance
 // from the cell's centre of mass to the box: every accepted cell passes the
@@ -63,6 +63,12 @@ __device__ __forceinline__ uint32_t ord_of(float f) {
 }
 __device__ __forceinline__ float float_of(uint32_t o) {
   return __uint_as_float((o & 0x80000000u) ? (o & 0x7fffffffu) : ~o);
+}
+
+__device__ __forceinline__ void f2_sum(f2 v, float& s) {
+  float lo, hi;
+  f2_split(v, lo, hi);
+  s = lo + hi;
 }
 
 // One pair of list entries (packed x, y, z, m) added to one target.
@@ -150,17 +156,41 @@ __device__ __forceinline__ void group_eval2(const float* ex, const float* ey, co
 // TWO: groups of up to 64 bodies (two targets per lane above 32; 80
 // registers, 3 blocks per SM); otherwise groups of up to 32 (64 registers,
 // 4 blocks per SM).
-template <int CNT, bool ZERO_EPS, bool TWO>
+// K: warps per group.  A group's walk is a chain of dependent steps (pop nodes,
+// load, test, push), about 1.5 us each, so few groups leave the GPU waiting.
+// K warps share one stack: each tests 32 of the 32 K nodes of a step and lists
+// and evaluates what it accepts in a ring of its own; their sums are added in
+// the warps' order at the end.  The interactions are the same, the chain is
+// K times shorter, and two barriers a step are the price.
+template <int CNT, bool ZERO_EPS, bool TWO, int K>
 __global__ void __launch_bounds__(kGWarps * 32, TWO ? 3 : 4) bh_group_walk_kernel(GroupWalkArgs a) {
+  static_assert(K == 1 || !TWO, "several warps per group: groups of at most 32 bodies");
   constexpr bool COUNT = CNT == 2;
   __shared__ int s_stack[kGWarps][kGStack];
   __shared__ __align__(16) float s_ring[kGWarps][4][kGRing];
   __shared__ __align__(16) float4 s_box[kGWarps][2];  // group box: centre, half sizes
+  __shared__ uint32_t s_team[kGWarps];  // what a warp tells the others of its group
   const uint32_t total = a.nstart[a.n];
   if ((int64_t)total > a.cap) return;  // the tree build failed and said so
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const unsigned full = 0xffffffffu, lt = (1u << lane) - 1u;
-  int* stk = s_stack[wid];
+  const int tw = wid & (K - 1), tid = tw * 32 + lane;  // warp and thread of the group's K warps
+  uint32_t* team = s_team + (wid - tw);
+  int* stk = s_stack[wid - tw];  // one stack for the group
+  const int limit = K * a.stack_limit;
+  auto sync = [&] {  // the group's K warps
+    if (K == 1)
+      __syncwarp();
+    else
+      asm volatile("bar.sync %0, %1;" ::"r"(1 + wid / K), "n"(32 * K) : "memory");
+  };
+  auto lead = [&](uint32_t v) {  // the value that the group's first lane has
+    if (K == 1) return __shfl_sync(full, v, 0);
+    sync();
+    if (tid == 0) team[0] = v;
+    sync();
+    return *(volatile uint32_t*)team;
+  };
   float* ex = s_ring[wid][0];
   float* ey = s_ring[wid][1];
   float* ez = s_ring[wid][2];
@@ -173,8 +203,8 @@ __global__ void __launch_bounds__(kGWarps * 32, TWO ? 3 : 4) bh_group_walk_kerne
   int* ovf = nullptr;  // this warp's overflow chunk, taken on first use
   while (true) {
     uint32_t t32 = 0;
-    if (lane == 0) t32 = atomicAdd(&a.gc->task, 1u);
-    const uint32_t t = __shfl_sync(full, t32, 0);
+    if (tid == 0) t32 = atomicAdd(&a.gc->task, 1u);
+    const uint32_t t = lead(t32);
     if (t >= ngroups) break;
     const int4 g = t < c0     ? a.groups[t]
                    : t < c01  ? a.groups[a.gcap - 1 - (int64_t)(t - c0)]
@@ -237,40 +267,48 @@ __global__ void __launch_bounds__(kGWarps * 32, TWO ? 3 : 4) bh_group_walk_kerne
     };
     int sp = 1, gsp = 0;
     bool failed = false;
-    if (lane == 0) stk[0] = a.seg_root[g.z];
-    __syncwarp();
+    if (tid == 0) stk[0] = a.seg_root[g.z];
+    sync();
     while (sp > 0 || gsp > 0) {
       if (sp == 0) {  // refill from the overflow chunk
-        const int m = min(gsp, a.stack_limit / 2);
-        for (int j = lane; j < m; j += 32) stk[j] = ovf[gsp - m + j];
+        const int m = min(gsp, limit / 2);
+        for (int j = tid; j < m; j += 32 * K) stk[j] = ovf[gsp - m + j];
         gsp -= m;
         sp = m;
-        __syncwarp();
+        sync();
       }
-      if (sp > a.stack_limit - 32) {  // a step adds at most 32: spill the oldest half
-        const int half = a.stack_limit / 2;
+      if (sp > limit - 32 * K) {  // a step adds at most 32 per warp: spill the oldest half
+        const int half = limit / 2;
         if (!ovf) {
           uint32_t c32 = 0;
-          if (lane == 0) c32 = atomicAdd(&a.gc->ovf, 1u);
-          const uint32_t c = __shfl_sync(full, c32, 0);
+          if (tid == 0) c32 = atomicAdd(&a.gc->ovf, 1u);
+          const uint32_t c = lead(c32);
           if (c < (uint32_t)kOvfChunks) ovf = a.ovf + (size_t)c * kOvfChunk;
         }
         if (!ovf || gsp + half > kOvfChunk) {
           failed = true;
           break;
         }
-        for (int j = lane; j < half; j += 32) ovf[gsp + j] = stk[j];
-        __syncwarp();
-        for (int j = lane; j < sp - half; j += 32) stk[j] = stk[half + j];
+        for (int j = tid; j < half; j += 32 * K) ovf[gsp + j] = stk[j];
+        sync();
+        // (half is at least 32 * K, and at most half + 32 * K entries move)
+        for (int j = tid; j - tid < sp - half; j += 32 * K) {
+          const int v = j < sp - half ? stk[half + j] : 0;
+          sync();
+          if (j < sp - half) stk[j] = v;
+        }
         gsp += half;
         sp -= half;
-        __syncwarp();
+        sync();
       }
-      const int m = min(sp, 32);
+      // the warps take the top nodes in turn, so that few nodes are shared out
+      // too; once entries have spilled a step takes 32 in all, which bounds what
+      // comes on top of them as with one warp
+      const int m = min(sp, K > 1 && gsp > 0 ? 32 : 32 * K);
       sp -= m;
-      const bool have = lane < m;
-      const int node = have ? stk[sp + lane] : 0;
-      __syncwarp();
+      const bool have = lane * K + tw < m;
+      const int node = have ? stk[sp + lane * K + tw] : 0;
+      if (K == 1) __syncwarp();
       f2 cm_xy = f2_make(0.f, 0.f), cm_zw = cm_xy, g_xy = cm_xy, g_zw = cm_xy;
       int4 w = make_int4((int)kWalkZero, 0, 0, 0);
       if (have) {
@@ -308,9 +346,25 @@ __global__ void __launch_bounds__(kGWarps * 32, TWO ? 3 : 4) bh_group_walk_kerne
       }
       // next siblings below first children, so the walk goes depth first
       const unsigned bs = __ballot_sync(full, next), bo = __ballot_sync(full, open);
-      if (next) stk[sp + __popc(bs & lt)] = (int)(wx & (kWalkZero - 1u));
-      if (open) stk[sp + __popc(bs) + __popc(bo & lt)] = node + 1;
-      sp += __popc(bs) + __popc(bo);
+      int ps = sp, po = sp + __popc(bs);  // this warp's places
+      sp = po + __popc(bo);
+      if (K > 1) {
+        if (lane == 0) team[tw] = (uint32_t)(__popc(bs) | __popc(bo) << 16);
+        sync();  // also: every warp has read its nodes
+        uint32_t before = 0, all = 0;
+#pragma unroll
+        for (int v = 0; v < K; ++v) {
+          const uint32_t c = *(volatile uint32_t*)&team[v];
+          before += v < tw ? c : 0u;
+          all += c;
+        }
+        po = ps + (int)(all & 0xffffu);
+        sp = po + (int)(all >> 16);
+        ps += (int)(before & 0xffffu);
+        po += (int)(before >> 16);
+      }
+      if (next) stk[ps + __popc(bs & lt)] = (int)(wx & (kWalkZero - 1u));
+      if (open) stk[po + __popc(bo & lt)] = node + 1;
       const unsigned be = __ballot_sync(full, entry);
       if (entry) {
         const int slot = (int)((wr + __popc(be & lt)) & (kGRing - 1));
@@ -391,6 +445,7 @@ __global__ void __launch_bounds__(kGWarps * 32, TWO ? 3 : 4) bh_group_walk_kerne
           }
         }
       }
+      if (K > 1) sync();  // the step's nodes are on the stack
     }
     if (failed) {
       if (lane == 0) raise_error(a.err, kErrWalkStack);
@@ -425,29 +480,50 @@ __global__ void __launch_bounds__(kGWarps * 32, TWO ? 3 : 4) bh_group_walk_kerne
     if (COUNT)
       selfmask = (uint64_t)__reduce_or_sync(full, (uint32_t)selfmask) |
                  ((uint64_t)__reduce_or_sync(full, (uint32_t)(selfmask >> 32)) << 32);
+    float fx, fy, fz, hx, hy, hz;
+    f2_sum(ax2, fx);
+    f2_sum(ay2, fy);
+    f2_sum(az2, fz);
+    f2_sum(bx2, hx);
+    f2_sum(by2, hy);
+    f2_sum(bz2, hz);
+    if (K > 1) {  // the warps' sums, in order, through their rings
+      float* r = s_ring[wid][0];
+      if (tw > 0) {
+        r[lane] = fx;
+        r[32 + lane] = fy;
+        r[64 + lane] = fz;
+        if (lane == 0) {
+          r[96] = __uint_as_float(wr);
+          r[97] = __uint_as_float((uint32_t)selfmask);
+        }
+      }
+      sync();
+      if (tw > 0) continue;
+      for (int v = 1; v < K; ++v) {
+        const float* q = s_ring[wid + v][0];
+        fx += q[lane];
+        fy += q[32 + lane];
+        fz += q[64 + lane];
+        wr += __float_as_uint(q[96]);
+        selfmask |= __float_as_uint(q[97]);
+      }
+    }
     const int cnt_lane = (int)wr - (int)((selfmask >> tl) & 1u);
     const int cnt_lane2 = (int)wr - (int)((selfmask >> (32 + tl2)) & 1u);
     const bool owner = valid && rr == 0, owner2 = valid2 && rr2 == 0;
     if (owner) {
-      float sx0, sx1, sy0, sy1, sz0, sz1;
-      f2_split(ax2, sx0, sx1);
-      f2_split(ay2, sy0, sy1);
-      f2_split(az2, sz0, sz1);
       const int64_t i = a.sv.arena(a.body[k]);
-      a.ax[i] = a.G * (sx0 + sx1);
-      a.ay[i] = a.G * (sy0 + sy1);
-      a.az[i] = a.G * (sz0 + sz1);
+      a.ax[i] = a.G * fx;
+      a.ay[i] = a.G * fy;
+      a.az[i] = a.G * fz;
       if (COUNT && a.counts) a.counts[i] = cnt_lane;
     }
     if (owner2) {
-      float sx0, sx1, sy0, sy1, sz0, sz1;
-      f2_split(bx2, sx0, sx1);
-      f2_split(by2, sy0, sy1);
-      f2_split(bz2, sz0, sz1);
       const int64_t i = a.sv.arena(a.body[k2]);
-      a.ax[i] = a.G * (sx0 + sx1);
-      a.ay[i] = a.G * (sy0 + sy1);
-      a.az[i] = a.G * (sz0 + sz1);
+      a.ax[i] = a.G * hx;
+      a.ay[i] = a.G * hy;
+      a.az[i] = a.G * hz;
       if (COUNT && a.counts) a.counts[i] = cnt_lane2;
     }
     {  // this group's cost, for the order of the next build's groups
@@ -471,33 +547,38 @@ __global__ void __launch_bounds__(kGWarps * 32, TWO ? 3 : 4) bh_group_walk_kerne
   }
 }
 
-template <int CNT, bool ZERO_EPS, bool TWO>
-static int group_walk_occupancy() {
+// Bodies below which a group gets four, two warps (the walk in us, Plummer
+// sphere, theta 0.5, with 1, 2, 4 warps per group: 20 K bodies 247, 162, 121;
+// 50 K 312, 194, 213; 100 K 322, 303, 398; 200 K 527, 592, 798).  Groups of up
+// to 64 bodies, which calculators use from 262,144 bodies on and ensembles
+// always, have one (1M bodies 2154, 2530, 3443).
+constexpr int64_t kGroupWarps4Max = 40000;
+constexpr int64_t kGroupWarps2Max = 115000;
+
+template <int CNT, bool ZERO_EPS, bool TWO, int K>
+static void launch_group_walk_t(const GroupWalkArgs& g, int64_t n, cudaStream_t st) {
   static const int occ = [] {
     int b = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, bh_group_walk_kernel<CNT, ZERO_EPS, TWO>,
-                                                  kGWarps * 32,
-                                                  0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, bh_group_walk_kernel<CNT, ZERO_EPS, TWO, K>,
+                                                  kGWarps * 32, 0);
     return std::max(b, 1);
   }();
-  return occ;
-}
-
-template <int CNT, bool ZERO_EPS, bool TWO>
-static void launch_group_walk_t(const GroupWalkArgs& g, int64_t n, cudaStream_t st) {
-  // persistent warps: one resident wave, never more warps than bodies
-  const int64_t blocks = std::max<int64_t>(
-      1, std::min<int64_t>(ceil_div(n, kGWarps),
-                           (int64_t)num_sms() * group_walk_occupancy<CNT, ZERO_EPS, TWO>()));
-  bh_group_walk_kernel<CNT, ZERO_EPS, TWO><<<(unsigned)blocks, kGWarps * 32, 0, st>>>(g);
+  // persistent warps: one resident wave, never more groups in flight than bodies
+  const int64_t blocks =
+      std::max<int64_t>(1, std::min<int64_t>(ceil_div(n, kGWarps / K), (int64_t)num_sms() * occ));
+  bh_group_walk_kernel<CNT, ZERO_EPS, TWO, K><<<(unsigned)blocks, kGWarps * 32, 0, st>>>(g);
 }
 
 template <int CNT, bool ZERO_EPS>
 static void launch_group_walk(const GroupWalkArgs& g, int64_t n, bool two, cudaStream_t st) {
   if (two)
-    launch_group_walk_t<CNT, ZERO_EPS, true>(g, n, st);
+    launch_group_walk_t<CNT, ZERO_EPS, true, 1>(g, n, st);
+  else if (n < kGroupWarps4Max)
+    launch_group_walk_t<CNT, ZERO_EPS, false, 4>(g, n, st);
+  else if (n < kGroupWarps2Max)
+    launch_group_walk_t<CNT, ZERO_EPS, false, 2>(g, n, st);
   else
-    launch_group_walk_t<CNT, ZERO_EPS, false>(g, n, st);
+    launch_group_walk_t<CNT, ZERO_EPS, false, 1>(g, n, st);
 }
 
 // Shared stack entries the group walk uses before spilling to global memory

@@ -123,7 +123,9 @@ constexpr int kGWarps = 8;            // warps (groups in flight) per block
 constexpr int kGStack = 512;          // per-warp shared stack (nodes to test)
 constexpr int kGRing = 64;            // per-warp ring of pending list entries
 constexpr int kGSmallRun = 16;        // bucket / leaf bodies listed lane-parallel up to this
-constexpr int kOvfChunk = 8704;       // per-warp stack overflow: 32 x 8 siblings x 34 levels
+// A group's stack overflow: 32 x 8 siblings x 34 levels on top of what the first
+// spill moved (half of four warps' shared entries and one step).
+constexpr int kOvfChunk = 8704 + 2 * kGStack + 128;
 constexpr int kOvfChunks = 256;       // overflow chunks per launch
 constexpr float kBoxWiden = 0x1.000004p0f;  // 1 + 2^-22: covers the half sizes' rounding
 
