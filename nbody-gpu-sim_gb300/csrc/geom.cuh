@@ -14,8 +14,16 @@ struct BBox {
   int valid;        // all bounds finite
 };
 
+// The box of a spatial hash build, in mapped host memory.
+struct HostBox {
+  float min[3];
+  float max[3];
+  int valid;  // all bounds finite
+};
+
 int bbox_blocks(int64_t n);  // partials needs bbox_blocks(n) * 6 floats
-void launch_bbox(const float4* pm, int64_t n, float* partials, BBox* box, uint32_t* err,
-                 cudaStream_t st);
+// counter: zero before the first launch, left zero by each.
+void launch_bbox(const float4* pm, int64_t n, float* partials, uint32_t* counter, HostBox* out,
+                 uint32_t* err, cudaStream_t st);
 
 }  // namespace nbgb

@@ -1,19 +1,18 @@
-// hash.cu -- spatial hash: stable counting sort by cell + 27-cell cutoff
+// hash.cu -- spatial hash: stable counting order by cell + 27-cell cutoff
 // gather (K7).
 //
 // Replaces SpatialHashGrid::build / computeForces and
 // SpatialHashCalculator::computeForces (src/cuda/force_spatial_hash.cu:241-388):
 //  * bbox on the device (geom.cu), padded by 0.001f on the host with the
 //    reference's float operations, dims = (int)ceilf((max-min)/cell) + 1,
-//    1e8-cell cap (:232-260).  One 40-byte device-to-host read per build
-//    (the reference does 12 allocations and 12 synchronous copies).
+//    1e8-cell cap (:232-260).  The kernel writes the box to mapped host memory,
+//    one stream synchronisation per build (the reference does 12 allocations and 12 synchronous copies).
 //  * cell id = clamp(floor((p - min) / cell)) with IEEE division, linear
 //    x + y*gx + z*gx*gy (:29-50); the effective cell size is
 //    max(cell_size, cutoff) (:382).
-//  * the reference's atomics-based count/scan/scatter (:53-81,292-308) is a
-//    stable radix sort of (cell id, particle index): same cell_start /
-//    cell_end, and within a cell ascending particle index (the reference's
-//    within-cell order is whatever its atomics produced).
+//  * count / scan / place (:53-81,292-308) with the same cell_start / cell_end,
+//    and then each cell's bodies in ascending index (the reference's within-cell
+//    order is whatever its atomics produced).
 //  * positions+masses are gathered into cell order (two bodies per 32-byte
 //    record), so the force kernel streams contiguous memory per neighbour row.
 //  * force: targets in cell order; 27 neighbours dz, dy, dx; skip j == i;
@@ -35,10 +34,11 @@ namespace nbgb {
 
 struct HashState {
   DevBuf<float> bbox_part;
-  DevBuf<BBox> box;
-  HostPinned<BBox> h_box;
-  DevBuf<uint32_t> keys, keys_alt, vals, vals_alt;
-  DevBuf<uint32_t> hist, scan_ws;
+  DevBuf<uint32_t> box_ctr;  // zero between builds
+  HostPinned<HostBox> h_box;
+  DevBuf<uint32_t> placed;      // bodies by cell, in any order within it
+  DevBuf<uint32_t> cells, idx;  // cell and index of the bodies in cell order
+  DevBuf<uint32_t> scan_ws;
   DevBuf<int32_t> particle_cell;
   DevBuf<uint32_t> cell_start;  // total_cells + 1
   DevBuf<float4> sorted_pm;
@@ -48,10 +48,7 @@ struct HashState {
   float bmin[3] = {0, 0, 0};
   float cell = 0.f;
   int64_t total = 0;
-  bool in_alt = false;
   bool built = false;  // the last build finished (the inspection calls read its buffers)
-  const uint32_t* sorted_cells() const { return in_alt ? keys_alt.ptr : keys.ptr; }
-  const uint32_t* sorted_idx() const { return in_alt ? vals_alt.ptr : vals.ptr; }
 };
 
 void hash_state_delete(HashState* p) { delete p; }
@@ -62,40 +59,56 @@ struct GridArgs {
   int dims[3];
 };
 
-__global__ void hash_assign_kernel(const float4* __restrict__ pm, int64_t n, GridArgs g,
-                                   int32_t* __restrict__ particle_cell,
-                                   uint32_t* __restrict__ keys, uint32_t* __restrict__ vals) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    float4 p = pm[i];
-    int cx = (int)floorf(__fdiv_rn(__fsub_rn(p.x, g.bmin[0]), g.cell));
-    int cy = (int)floorf(__fdiv_rn(__fsub_rn(p.y, g.bmin[1]), g.cell));
-    int cz = (int)floorf(__fdiv_rn(__fsub_rn(p.z, g.bmin[2]), g.cell));
-    cx = max(0, min(cx, g.dims[0] - 1));
-    cy = max(0, min(cy, g.dims[1] - 1));
-    cz = max(0, min(cz, g.dims[2] - 1));
-    int32_t id = cx + cy * g.dims[0] + cz * g.dims[0] * g.dims[1];
-    particle_cell[i] = id;
-    keys[i] = (uint32_t)id;
-    vals[i] = (uint32_t)i;
+__device__ __forceinline__ int32_t cell_of(float4 p, const GridArgs& g) {
+  int cx = (int)floorf(__fdiv_rn(__fsub_rn(p.x, g.bmin[0]), g.cell));
+  int cy = (int)floorf(__fdiv_rn(__fsub_rn(p.y, g.bmin[1]), g.cell));
+  int cz = (int)floorf(__fdiv_rn(__fsub_rn(p.z, g.bmin[2]), g.cell));
+  cx = max(0, min(cx, g.dims[0] - 1));
+  cy = max(0, min(cy, g.dims[1] - 1));
+  cz = max(0, min(cz, g.dims[2] - 1));
+  return cx + cy * g.dims[0] + cz * g.dims[0] * g.dims[1];
+}
+
+// Cell order by counting: count the bodies per cell with atomics, scan, place,
+// and put each cell's bodies in ascending order.  Two random 4-byte accesses per
+// body bound it (4M bodies 164 us; a radix sort of the cell ids, the cell starts
+// by binary search and the records took 258).  The atomics hand out the places
+// within a cell in any order, which the last kernel makes good.
+__global__ void hash_count_kernel(const float4* __restrict__ pm, int64_t n, GridArgs g,
+                                  int32_t* __restrict__ particle_cell,
+                                  uint32_t* __restrict__ count, uint32_t* __restrict__ place) {
+  const int64_t step = (int64_t)gridDim.x * blockDim.x;
+  const int lane = threadIdx.x & 31;
+#pragma unroll 4
+  for (int64_t w = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x - lane); w < n; w += step) {
+    const int64_t i = w + lane;
+    const bool on = i < n;
+    const int32_t id = on ? cell_of(pm[i], g) : 0;
+    const unsigned mask = __ballot_sync(0xffffffffu, on);
+    const int32_t id0 = __shfl_sync(0xffffffffu, id, 0);
+    uint32_t at = 0;
+    if (__all_sync(0xffffffffu, !on || id == id0)) {
+      // one cell: one atomic (a whole system in one cell would queue at it)
+      if (lane == 0) at = atomicAdd(&count[id], (uint32_t)__popc(mask));
+      at = __shfl_sync(0xffffffffu, at, 0) + lane;
+    } else if (on) {
+      at = atomicAdd(&count[id], 1u);
+    }
+    if (on) {
+      particle_cell[i] = id;
+      place[i] = at;
+    }
   }
 }
 
-// start[c] = number of particles with cell < c (lower bound in the sorted
-// cell ids), c in [0, total]; end[c] = start[c + 1].
-__global__ void hash_cell_start_kernel(const uint32_t* __restrict__ sorted_cells, int64_t n,
-                                       int64_t total, uint32_t* __restrict__ start) {
-  for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c <= total;
-       c += (int64_t)gridDim.x * blockDim.x) {
-    int64_t lo = 0, hi = n;
-    while (lo < hi) {
-      int64_t mid = (lo + hi) >> 1;
-      if ((int64_t)sorted_cells[mid] < c)
-        lo = mid + 1;
-      else
-        hi = mid;
-    }
-    start[c] = (uint32_t)lo;
+__global__ void hash_place_kernel(const int32_t* __restrict__ particle_cell,
+                                  const uint32_t* __restrict__ place,
+                                  const uint32_t* __restrict__ start, int64_t n,
+                                  uint32_t* __restrict__ idx) {
+  const int64_t step = (int64_t)gridDim.x * blockDim.x;
+#pragma unroll 4
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += step) {
+    idx[start[particle_cell[i]] + place[i]] = (uint32_t)i;
   }
 }
 
@@ -104,27 +117,95 @@ __global__ void hash_cell_start_kernel(const uint32_t* __restrict__ sorted_cells
 // coordinate is put where its squared distance overflows to infinity, outside
 // every cutoff (in the test d^2 < rc^2 a NaN never passes).  An odd last half
 // is filled the same way, without mass.
-__device__ __forceinline__ float4 gather_body(const float4* pm, const uint32_t* idx, int64_t k,
-                                              int64_t n) {
-  float4 p = make_float4(3.0e38f, 0.f, 0.f, 0.f);
-  if (k < n) {
-    const float4 q = pm[idx[k]];
-    if (q.x == q.x && q.y == q.y && q.z == q.z)
-      p = q;
-    else
-      p.w = q.w;
-  }
-  return p;
+__device__ __forceinline__ float4 gather_record(float4 q) {
+  return q.x == q.x && q.y == q.y && q.z == q.z ? q : make_float4(3.0e38f, 0.f, 0.f, q.w);
 }
 
-__global__ void hash_gather_kernel(const float4* __restrict__ pm, const uint32_t* __restrict__ idx,
-                                   int64_t n, float4* __restrict__ out) {
-  for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; 2 * p < n;
-       p += (int64_t)gridDim.x * blockDim.x) {
-    const float4 u = gather_body(pm, idx, 2 * p, n), v = gather_body(pm, idx, 2 * p + 1, n);
-    out[2 * p] = make_float4(u.x, v.x, u.y, v.y);
-    out[2 * p + 1] = make_float4(u.z, v.z, u.w, v.w);
+// The bodies of each cell in ascending order, and their records: a body's place
+// is the number of smaller indices in its cell.  In a cell of at most kHashCrowd
+// bodies each thread compares its own.  A block meets at most two larger cells,
+// its first and its last slot's; there every index of the cell is looked up among
+// the block's sorted ones, so a cell of c bodies costs c * c / kHashCrowd lookups
+// and not c * c compares (60 K bodies in one cell 74 us against 926).
+constexpr int kHashCrowd = 256;  // threads (and slots) per block, too
+
+__global__ void __launch_bounds__(kHashCrowd) hash_order_kernel(
+    const float4* __restrict__ pm, GridArgs g, const uint32_t* __restrict__ idx,
+    const uint32_t* __restrict__ start, int64_t n, uint32_t* __restrict__ cells,
+    uint32_t* __restrict__ sorted_idx, float* __restrict__ out) {
+  __shared__ uint32_t s_idx[kHashCrowd], s_sorted[kHashCrowd];
+  __shared__ uint32_t s_hist[2][kHashCrowd + 1];
+  __shared__ uint32_t s_cell[2][2];  // first and last slot's cell: start, end
+  const int tid = threadIdx.x;
+  const int64_t p0 = blockIdx.x * (int64_t)kHashCrowd, p = p0 + tid;
+  const int64_t p1 = imin64(p0 + kHashCrowd, n);
+  float4 b = make_float4(3.0e38f, 0.f, 0.f, 0.f);
+  uint32_t i = 0, s = 0, e = 0, r = 0;
+  if (p < n) {
+    i = idx[p];
+    b = pm[i];
+    const int32_t id = cell_of(b, g);
+    b = gather_record(b);
+    cells[p] = (uint32_t)id;
+    s = start[id];
+    e = start[id + 1];
   }
+  const bool crowd = e - s > (uint32_t)kHashCrowd;
+  if (!crowd)
+    for (uint32_t q = s; q < e; ++q) r += idx[q] < i ? 1u : 0u;
+  if (__syncthreads_or(crowd)) {
+    s_idx[tid] = i;
+    if (p == p0 || p == p1 - 1) {
+      const int w = p == p0 ? 0 : 1;
+      s_cell[w][0] = s;
+      s_cell[w][1] = e;
+      if (p0 == p1 - 1) s_cell[1][0] = s_cell[1][1] = 0;
+    }
+    __syncthreads();
+    for (int w = 0; w < 2; ++w) {
+      const uint32_t cs = s_cell[w][0], ce = s_cell[w][1];
+      if (ce - cs <= (uint32_t)kHashCrowd || (w == 1 && cs == s_cell[0][0])) continue;
+      // the block's slots [a, z) of this cell, sorted
+      const int a = cs > (uint32_t)p0 ? (int)(cs - (uint32_t)p0) : 0;
+      const int z = (int)imin64((int64_t)ce, p1) - (int)p0;
+      const bool mine = tid >= a && tid < z;
+      int own = 0;
+      if (mine) {
+        for (int q = a; q < z; ++q) own += s_idx[q] < i ? 1 : 0;
+        s_sorted[own] = i;
+      } else {
+        s_sorted[z - a + (tid < a ? tid : tid - (z - a))] = 0xffffffffu;
+      }
+      s_hist[0][tid] = 0;
+      __syncthreads();
+#pragma unroll 4
+      for (uint32_t q = cs + tid; q < ce; q += kHashCrowd) {
+        const uint32_t v = idx[q];
+        int at = 0;  // sorted entries not above v
+#pragma unroll
+        for (int h = kHashCrowd / 2; h > 0; h >>= 1) at += s_sorted[at + h - 1] <= v ? h : 0;
+        at += s_sorted[at] <= v ? 1 : 0;
+        if (at < kHashCrowd) atomicAdd(&s_hist[0][at], 1u);
+      }
+      __syncthreads();
+      int f = 0;
+      for (int o = 1; o < kHashCrowd; o <<= 1) {
+        s_hist[f ^ 1][tid] = s_hist[f][tid] + (tid >= o ? s_hist[f][tid - o] : 0u);
+        f ^= 1;
+        __syncthreads();
+      }
+      if (mine) r = s_hist[f][own];
+      __syncthreads();
+    }
+  }
+  if (p > n || (p == n && !(n & 1))) return;  // an odd last half is filled, too
+  const int64_t at = p < n ? (int64_t)s + r : p;
+  if (p < n) sorted_idx[at] = i;
+  float* o = out + (at >> 1) * 8 + (at & 1);
+  o[0] = b.x;
+  o[2] = b.y;
+  o[4] = b.z;
+  o[6] = b.w;
 }
 
 // The 27-cell gather.  Cells cx-1 .. cx+1 of a neighbour row are consecutive
@@ -256,10 +337,12 @@ void hash_forces(nbgb_calculator* c, const float4* pm, int64_t n, float* ax, flo
   uint32_t* err = c->err.ensure(1);
   // 1. bounding box -> host (sizes the grid)
   float* part = h.bbox_part.ensure((size_t)bbox_blocks(n) * 6);
-  BBox* box = h.box.ensure(1);
-  launch_bbox(pm, n, part, box, err, st);
-  BBox* hb = h.h_box.ensure(1);
-  NBGB_CUDA(cudaMemcpyAsync(hb, box, sizeof(BBox), cudaMemcpyDeviceToHost, st));
+  if (!h.box_ctr.ptr) {
+    h.box_ctr.ensure(1);
+    NBGB_CUDA(cudaMemsetAsync(h.box_ctr.ptr, 0, sizeof(uint32_t), st));
+  }
+  HostBox* hb = h.h_box.ensure(1);
+  launch_bbox(pm, n, part, h.box_ctr.ptr, hb, err, st);
   NBGB_CUDA(cudaStreamSynchronize(st));
   if (!hb->valid) fail(NBGB_ERR_INVALID_ARG, "Validation Error: non-finite particle position");
   const float cell = std::max(c->params.cell_size, c->params.cutoff);
@@ -287,30 +370,25 @@ void hash_forces(nbgb_calculator* c, const float4* pm, int64_t n, float* ax, flo
   // 2. assign cells
   stage_mark(timer, "spatial_hash.assign");
   int32_t* pc = h.particle_cell.ensure((size_t)n);
-  uint32_t* keys = h.keys.ensure((size_t)n);
-  uint32_t* vals = h.vals.ensure((size_t)n);
-  uint32_t* keys_alt = h.keys_alt.ensure((size_t)n);
-  uint32_t* vals_alt = h.vals_alt.ensure((size_t)n);
-  hash_assign_kernel<<<grid1d(n), 256, 0, st>>>(pm, n, g, pc, keys, vals);
-  NBGB_LAUNCH_CHECK();
-  // 3. stable sort by cell id
-  stage_mark(timer, "spatial_hash.sort");
-  int bits = 1;
-  while (bits < 32 && ((int64_t)1 << bits) < total) ++bits;
-  const int end_bit = ((bits + 7) / 8) * 8;
-  uint32_t* hist = h.hist.ensure(radix_hist_elems(n));
-  uint32_t* sws = h.scan_ws.ensure(scan_workspace_elems((int64_t)radix_hist_elems(n)) +
-                                   scan_workspace_elems(total + 1));
-  radix_sort_pairs<uint32_t>(keys, keys_alt, vals, vals_alt, n, 0, end_bit, hist, sws, st,
-                             &h.in_alt, c->err.ensure(1));
-  // 4. cell starts
-  stage_mark(timer, "spatial_hash.cells");
+  uint32_t* placed = h.placed.ensure((size_t)n);
+  uint32_t* cells = h.cells.ensure((size_t)n);
+  uint32_t* idx = h.idx.ensure((size_t)n);
+  uint32_t* place = idx;  // free until the last kernel fills it
   uint32_t* start = h.cell_start.ensure((size_t)total + 1);
-  hash_cell_start_kernel<<<grid1d(total + 1), 256, 0, st>>>(h.sorted_cells(), n, total, start);
-  NBGB_LAUNCH_CHECK();
-  // 5. payload in cell order
   float4* spm = h.sorted_pm.ensure((size_t)n + 1);
-  hash_gather_kernel<<<grid1d((n + 1) / 2), 256, 0, st>>>(pm, h.sorted_idx(), n, spm);
+  uint32_t* sws = h.scan_ws.ensure(scan_workspace_elems(total + 1));
+  NBGB_CUDA(cudaMemsetAsync(start, 0, ((size_t)total + 1) * sizeof(uint32_t), st));
+  hash_count_kernel<<<grid1d(n), 256, 0, st>>>(pm, n, g, pc, start, place);
+  NBGB_LAUNCH_CHECK();
+  // 3. cell starts and places
+  stage_mark(timer, "spatial_hash.sort");
+  scan_exclusive_u32(start, start, total + 1, sws, nullptr, st);
+  hash_place_kernel<<<grid1d(n), 256, 0, st>>>(pc, place, start, n, placed);
+  NBGB_LAUNCH_CHECK();
+  // 4.-5. order within the cells, and records in that order
+  stage_mark(timer, "spatial_hash.cells");
+  hash_order_kernel<<<(unsigned)ceil_div(n + 1, kHashCrowd), kHashCrowd, 0, st>>>(
+      pm, g, placed, start, n, cells, idx, reinterpret_cast<float*>(spm));
   NBGB_LAUNCH_CHECK();
   // 6. cutoff gather
   stage_mark(timer, "spatial_hash.forces");
@@ -320,7 +398,7 @@ void hash_forces(nbgb_calculator* c, const float4* pm, int64_t n, float* ax, flo
   const auto force = [&](auto cnt, auto sub) {
     constexpr int S = decltype(sub)::value, T = S == 1 ? 256 : 32;
     hash_force_kernel<decltype(cnt)::value, S>
-        <<<(unsigned)ceil_div(n, T), T * S, 0, st>>>(spm, h.sorted_cells(), h.sorted_idx(), start,
+        <<<(unsigned)ceil_div(n, T), T * S, 0, st>>>(spm, cells, idx, start,
                                                      n, g, rc * rc, eps * eps, c->params.G, ax,
                                                      ay, az, counts);
   };
@@ -373,7 +451,7 @@ nbgb_status nbgb_hash_copy_cells(nbgb_calculator* c, int32_t* cell_start, int32_
   if (particle_cells && e == cudaSuccess)
     e = cudaMemcpy(particle_cells, h.particle_cell.ptr, n * 4, cudaMemcpyDeviceToHost);
   if (sorted_indices && e == cudaSuccess)
-    e = cudaMemcpy(sorted_indices, h.sorted_idx(), n * 4, cudaMemcpyDeviceToHost);
+    e = cudaMemcpy(sorted_indices, h.idx.ptr, n * 4, cudaMemcpyDeviceToHost);
   return e == cudaSuccess ? NBGB_OK : NBGB_ERR_CUDA;
 }
 

@@ -27,6 +27,7 @@ namespace nbgb {
 constexpr int kScanThreads = 256;
 constexpr int kScanItems = 16;  // per thread
 constexpr int kScanChunk = kScanThreads * kScanItems;
+constexpr int kScanOneBlock = 16384;  // values that one block scans in one launch
 
 // ---------------------------------------------------------------- scan --
 __global__ void scan_reduce_kernel(const uint32_t* __restrict__ in, int64_t n,
@@ -131,6 +132,11 @@ size_t scan_workspace_elems(int64_t n) { return (size_t)ceil_div(std::max<int64_
 void scan_exclusive_u32(const uint32_t* in, uint32_t* out, int64_t n, uint32_t* ws,
                         uint32_t* total, cudaStream_t st) {
   if (n <= 0) return;
+  if (in == out && n <= kScanOneBlock) {
+    scan_single_block_kernel<<<1, 1024, 0, st>>>(out, n, total);
+    NBGB_LAUNCH_CHECK();
+    return;
+  }
   const int64_t nb = ceil_div(n, kScanChunk);
   scan_reduce_kernel<<<(unsigned)nb, kScanThreads, 0, st>>>(in, n, ws);
   NBGB_LAUNCH_CHECK();
