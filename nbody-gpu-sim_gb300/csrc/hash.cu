@@ -23,6 +23,7 @@
 //    bit-exactly.
 #include <cmath>
 #include <type_traits>
+#include <vector>
 
 #include "common.cuh"
 #include "geom.cuh"
@@ -36,12 +37,15 @@ struct HashState {
   DevBuf<float> bbox_part;
   DevBuf<uint32_t> box_ctr;  // zero between builds
   HostPinned<HostBox> h_box;
-  DevBuf<uint32_t> placed;      // bodies by cell, in any order within it
-  DevBuf<uint32_t> cells, idx;  // cell and index of the bodies in cell order
-  DevBuf<uint32_t> scan_ws;
   DevBuf<int32_t> particle_cell;
-  DevBuf<uint32_t> cell_start;  // total_cells + 1
-  DevBuf<float4> sorted_pm;
+  DevBuf<uint32_t> count;   // bodies per cell (total_cells + 1, the last 0)
+  DevBuf<uint32_t> start;   // a cell's first slot (total_cells + 1): each cell has an
+                            // even number of slots, a last odd one without a body
+  DevBuf<uint32_t> placed;  // slots: bodies in any order within the cell
+  DevBuf<uint32_t> idx;     // slots: bodies in ascending order within the cell
+  DevBuf<uint32_t> cells;   // pairs of slots: their cell
+  DevBuf<float4> pairs;     // pairs of slots: their bodies
+  DevBuf<uint32_t> scan_ws;
   // last build
   int64_t n = 0;
   int dims[3] = {0, 0, 0};
@@ -113,13 +117,14 @@ __global__ void hash_place_kernel(const int32_t* __restrict__ particle_cell,
 }
 
 // Bodies in cell order, two per 32-byte record (x0 x1 y0 y1 z0 z1 m0 m1), so
-// that two candidates arrive as packed FP32x2 operands.  A body with a NaN
-// coordinate is put where its squared distance overflows to infinity, outside
-// every cutoff (in the test d^2 < rc^2 a NaN never passes).  An odd last half
-// is filled the same way, without mass.
-__device__ __forceinline__ float4 gather_record(float4 q) {
-  return q.x == q.x && q.y == q.y && q.z == q.z ? q : make_float4(3.0e38f, 0.f, 0.f, q.w);
-}
+// that two candidates arrive as packed FP32x2 operands.  A cell starts a record:
+// no candidate of a range has to be masked out, and a record's two bodies are
+// targets with the same candidates.  A body with a NaN coordinate is put where its
+// squared distance overflows to infinity, outside every cutoff (in the test
+// d^2 < rc^2 a NaN never passes).  A slot without a body is filled the same way,
+// without mass.
+constexpr uint32_t kNoBody = 0xffffffffu;
+constexpr float kFarAway = 3.0e38f;  // (bodies are within 1e30, where the box's bounds start)
 
 // The bodies of each cell in ascending order, and their records: a body's place
 // is the number of smaller indices in its cell.  In a cell of at most kHashCrowd
@@ -130,36 +135,47 @@ __device__ __forceinline__ float4 gather_record(float4 q) {
 constexpr int kHashCrowd = 256;  // threads (and slots) per block, too
 
 __global__ void __launch_bounds__(kHashCrowd) hash_order_kernel(
-    const float4* __restrict__ pm, GridArgs g, const uint32_t* __restrict__ idx,
-    const uint32_t* __restrict__ start, int64_t n, uint32_t* __restrict__ cells,
-    uint32_t* __restrict__ sorted_idx, float* __restrict__ out) {
+    const float4* __restrict__ pm, int64_t n, GridArgs g, int64_t total,
+    const uint32_t* __restrict__ placed,
+    const uint32_t* __restrict__ count, const uint32_t* __restrict__ start,
+    uint32_t* __restrict__ cells, uint32_t* __restrict__ idx, float* __restrict__ out) {
   __shared__ uint32_t s_idx[kHashCrowd], s_sorted[kHashCrowd];
   __shared__ uint32_t s_hist[2][kHashCrowd + 1];
   __shared__ uint32_t s_cell[2][2];  // first and last slot's cell: start, end
   const int tid = threadIdx.x;
+  const int64_t slots = start[total];
   const int64_t p0 = blockIdx.x * (int64_t)kHashCrowd, p = p0 + tid;
-  const int64_t p1 = imin64(p0 + kHashCrowd, n);
-  float4 b = make_float4(3.0e38f, 0.f, 0.f, 0.f);
-  uint32_t i = 0, s = 0, e = 0, r = 0;
-  if (p < n) {
-    i = idx[p];
+  const int64_t p1 = imin64(p0 + kHashCrowd, slots);
+  if (p0 >= slots) return;
+  float4 b = make_float4(kFarAway, 0.f, 0.f, 0.f);
+  uint32_t i = p < slots ? placed[p] : kNoBody, s = 0, e = 0, r = 0;
+  if (i < n) {
     b = pm[i];
     const int32_t id = cell_of(b, g);
-    b = gather_record(b);
-    cells[p] = (uint32_t)id;
+    if (!(b.x == b.x && b.y == b.y && b.z == b.z)) b = make_float4(kFarAway, 0.f, 0.f, b.w);
+    if (!(p & 1)) cells[p >> 1] = (uint32_t)id;
     s = start[id];
-    e = start[id + 1];
+    e = s + count[id];
+  }
+  // a cell's odd last slot holds nothing: it is not below the end of the cell
+  // that the slot before it belongs to
+  const uint32_t before = __shfl_up_sync(0xffffffffu, e, 1);
+  if (p >= slots || ((p & 1) && p >= before)) {
+    i = kNoBody;
+    s = e = 0;
+    b = make_float4(kFarAway, 0.f, 0.f, 0.f);
   }
   const bool crowd = e - s > (uint32_t)kHashCrowd;
   if (!crowd)
-    for (uint32_t q = s; q < e; ++q) r += idx[q] < i ? 1u : 0u;
+    for (uint32_t q = s; q < e; ++q) r += placed[q] < i ? 1u : 0u;
   if (__syncthreads_or(crowd)) {
     s_idx[tid] = i;
-    if (p == p0 || p == p1 - 1) {
+    // (the block's first slot has a body; its last two slots are of one cell)
+    if (p == p0 || p == p1 - 2) {
       const int w = p == p0 ? 0 : 1;
       s_cell[w][0] = s;
       s_cell[w][1] = e;
-      if (p0 == p1 - 1) s_cell[1][0] = s_cell[1][1] = 0;
+      if (p0 == p1 - 2) s_cell[1][0] = s_cell[1][1] = 0;
     }
     __syncthreads();
     for (int w = 0; w < 2; ++w) {
@@ -180,7 +196,7 @@ __global__ void __launch_bounds__(kHashCrowd) hash_order_kernel(
       __syncthreads();
 #pragma unroll 4
       for (uint32_t q = cs + tid; q < ce; q += kHashCrowd) {
-        const uint32_t v = idx[q];
+        const uint32_t v = placed[q];
         int at = 0;  // sorted entries not above v
 #pragma unroll
         for (int h = kHashCrowd / 2; h > 0; h >>= 1) at += s_sorted[at + h - 1] <= v ? h : 0;
@@ -198,9 +214,9 @@ __global__ void __launch_bounds__(kHashCrowd) hash_order_kernel(
       __syncthreads();
     }
   }
-  if (p > n || (p == n && !(n & 1))) return;  // an odd last half is filled, too
-  const int64_t at = p < n ? (int64_t)s + r : p;
-  if (p < n) sorted_idx[at] = i;
+  if (p >= slots) return;
+  const int64_t at = i != kNoBody ? (int64_t)s + r : p;
+  idx[at] = i;
   float* o = out + (at >> 1) * 8 + (at & 1);
   o[0] = b.x;
   o[2] = b.y;
@@ -209,111 +225,169 @@ __global__ void __launch_bounds__(kHashCrowd) hash_order_kernel(
 }
 
 // The 27-cell gather.  Cells cx-1 .. cx+1 of a neighbour row are consecutive
-// in the sorted bodies, so a target walks 9 ranges, two candidates per packed
-// step and without a branch on the cutoff: with 15 % of the candidates
-// accepted almost every warp took both paths of a branch (24 to 31
-// instructions per candidate, 21 of 32 lanes active).  A rejected candidate's
-// force factor is zero.  The squared distance uses the reference's rounding
-// (packed operations round each half like the scalar ones), so neighbour
-// counts stay bit-exact.
+// records, so a pair of targets walks 9 ranges, two candidates per packed step
+// and without a branch on the cutoff: with 15 % of the candidates accepted almost
+// every warp took both paths of a branch.  A rejected candidate's force factor is
+// zero.  The squared distance uses the reference's rounding (packed operations
+// round each half like the scalar ones), so neighbour counts stay bit-exact.
+// A thread has the two bodies of a record as targets: with one, the candidates'
+// way from L1 to the registers (32 bytes per thread and step, 67 % of that path)
+// was as busy as the issue slots (4M bodies 814 us, now 678).
 //
-// SUB threads share a target's rows (9 / SUB each) where the targets alone do
-// not fill the GPU; their sums are added in row order.
-template <bool COUNT, int SUB>
-__global__ void __launch_bounds__(SUB == 1 ? 256 : 288) hash_force_kernel(
-    const float4* __restrict__ spm, const uint32_t* __restrict__ sorted_cells,
-    const uint32_t* __restrict__ sorted_idx, const uint32_t* __restrict__ start, int64_t n,
-    GridArgs g, float cut2, float eps2, float G, float* __restrict__ ax, float* __restrict__ ay,
+// SUB threads share a pair's records, an equal run of all nine rows' each, where
+// the targets alone do not fill the GPU; their sums are added in order.  ROWS: a
+// thread's run is taken row by row in a tight loop, which pays where rows are long;
+// otherwise it goes on to the next row at once, without waiting for the longest
+// row of the warp (of 8 cells with 24 candidates per row on average).
+template <bool COUNT, int SUB, int T, bool ROWS>
+__global__ void __launch_bounds__(SUB * T) hash_force_kernel(
+    const float4* __restrict__ pairs, const uint32_t* __restrict__ cells,
+    const uint32_t* __restrict__ idx, const uint32_t* __restrict__ start, int64_t total, GridArgs g,
+    float cut2, float eps2, float G, float* __restrict__ ax, float* __restrict__ ay,
     float* __restrict__ az, int32_t* __restrict__ counts) {
-  constexpr int T = SUB == 1 ? 256 : 32;  // targets per block
-  const int t = threadIdx.x % T, sub = threadIdx.x / T;
+  __shared__ uint2 s_row[9][T];  // records of each neighbour row
+  const int t = threadIdx.x % T, sub = threadIdx.x / T;  // pair of the block, its thread
+  const int64_t npairs = start[total] >> 1;
   const int64_t k = (int64_t)blockIdx.x * T + t;
-  const bool valid = k < n;
-  const int64_t kk = valid ? k : n - 1;
-  const float* sf = reinterpret_cast<const float*>(spm);
-  const int64_t me = (kk >> 1) * 8 + (kk & 1);
-  const float px = sf[me], py = sf[me + 2], pz = sf[me + 4];
-  const f2 xi = f2_make(px, px), yi = f2_make(py, py), zi = f2_make(pz, pz);
+  if ((int64_t)blockIdx.x * T >= npairs) return;
+  const bool valid = k < npairs;
+  const uint32_t me = (uint32_t)(valid ? k : npairs - 1);
+  const float4 own0 = pairs[2 * (int64_t)me], own1 = pairs[2 * (int64_t)me + 1];
+  const float px[2] = {own0.x, own0.y};
+  const f2 xi[2] = {f2_make(own0.x, own0.x), f2_make(own0.y, own0.y)};
+  const f2 yi[2] = {f2_make(own0.z, own0.z), f2_make(own0.w, own0.w)};
+  const f2 zi[2] = {f2_make(own1.x, own1.x), f2_make(own1.y, own1.y)};
   const f2 e2 = f2_make(eps2, eps2);
-  const int id = (int)sorted_cells[kk];
+  const int id = (int)cells[me];
   const int gxy = g.dims[0] * g.dims[1];
   const int cz = id / gxy;
   const int rem = id - cz * gxy;
   const int cy = rem / g.dims[0];
   const int cx = rem - cy * g.dims[0];
   const int x0 = max(cx - 1, 0), x1 = min(cx + 1, g.dims[0] - 1) + 1;
-  f2 sx = f2_make(0.f, 0.f), sy = sx, sz = sx;
-  int cnt = 0;
-  // candidates [s, e) of one row; self: the row that holds the target
-  auto row = [&](uint32_t s, uint32_t e, auto self) {
-    for (uint32_t j = s & ~1u; j < e; j += 2) {
-      const float4* rec = spm + j;  // record j / 2: two float4
-      const ulonglong2 xy = __ldg(reinterpret_cast<const ulonglong2*>(rec));
-      const ulonglong2 zm = __ldg(reinterpret_cast<const ulonglong2*>(rec + 1));
-      const f2 dx = f2_sub(f2{xy.x}, xi), dy = f2_sub(f2{xy.y}, yi), dz = f2_sub(f2{zm.x}, zi);
+  f2 sum[2][3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) sum[0][c] = sum[1][c] = f2_make(0.f, 0.f);
+  int cnt[2] = {0, 0};
+  uint32_t len = 0;
+#pragma unroll 1
+  for (int r = sub; r < 9; r += SUB) {
+    const int nz = cz + r / 3 - 1, ny = cy + r % 3 - 1;
+    uint2 se = make_uint2(0, 0);
+    if (nz >= 0 && nz < g.dims[2] && ny >= 0 && ny < g.dims[1]) {
+      const int base = ny * g.dims[0] + nz * gxy;
+      se = make_uint2(start[base + x0] >> 1, start[base + x1] >> 1);
+    }
+    s_row[r][t] = se;
+    len += se.y - se.x;
+  }
+  auto add = [&](uint32_t j) {
+    const ulonglong2* rec = reinterpret_cast<const ulonglong2*>(pairs) + 2 * (uint64_t)j;
+    const ulonglong2 xy = __ldg(rec), zm = __ldg(rec + 1);
+    const bool other = j != me;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const f2 dx = f2_sub(f2{xy.x}, xi[q]), dy = f2_sub(f2{xy.y}, yi[q]),
+               dz = f2_sub(f2{zm.x}, zi[q]);
       const f2 d2 = f2_fma(dz, dz, f2_fma(dy, dy, f2_mul(dx, dx)));
       float dl, dh;
       f2_split(d2, dl, dh);
-      bool ol = dl < cut2 && j >= s, oh = dh < cut2 && j + 1 < e;
-      if constexpr (decltype(self)::value) {
-        ol = ol && (int64_t)j != kk;
-        oh = oh && (int64_t)j + 1 != kk;
-      }
+      const bool ol = dl < cut2 && (q == 1 || other), oh = dh < cut2 && (q == 0 || other);
       const f2 s2 = f2_add(d2, e2);
       f2_split(s2, dl, dh);
-      const f2 r = f2_make(rsqrt_approx(dl), rsqrt_approx(dh));
-      f2 f = f2_mul(f2_mul(f2{zm.y}, r), f2_mul(r, r));
+      const f2 rs = f2_make(rsqrt_approx(dl), rsqrt_approx(dh));
+      f2 f = f2_mul(f2_mul(f2{zm.y}, rs), f2_mul(rs, rs));
       float fl, fh;
       f2_split(f, fl, fh);
       f = f2_make(ol ? fl : 0.f, oh ? fh : 0.f);
-      sx = f2_fma(f, dx, sx);
-      sy = f2_fma(f, dy, sy);
-      sz = f2_fma(f, dz, sz);
-      if (COUNT) cnt += (ol ? 1 : 0) + (oh ? 1 : 0);
+      sum[q][0] = f2_fma(f, dx, sum[q][0]);
+      sum[q][1] = f2_fma(f, dy, sum[q][1]);
+      sum[q][2] = f2_fma(f, dz, sum[q][2]);
+      if (COUNT) cnt[q] += (ol ? 1 : 0) + (oh ? 1 : 0);
     }
   };
-#pragma unroll 1
-  for (int r = sub * (9 / SUB); r < (sub + 1) * (9 / SUB); ++r) {
-    const int nz = cz + r / 3 - 1, ny = cy + r % 3 - 1;
-    if (nz < 0 || nz >= g.dims[2] || ny < 0 || ny >= g.dims[1]) continue;
-    const int base = ny * g.dims[0] + nz * gxy;
-    const uint32_t s = start[base + x0], e = start[base + x1];
-    if (r == 4)
-      row(s, e, std::true_type{});
-    else
-      row(s, e, std::false_type{});
-  }
-  float v[3], hi;
-  f2_split(sx, v[0], hi);
-  v[0] += hi;
-  f2_split(sy, v[1], hi);
-  v[1] += hi;
-  f2_split(sz, v[2], hi);
-  v[2] += hi;
+  uint32_t lo = 0, hi = len;
   if constexpr (SUB > 1) {
-    __shared__ float s_sum[SUB - 1][3][T];
-    __shared__ int s_cnt[COUNT ? SUB - 1 : 1][T];
+    __syncthreads();
+    len = 0;
+#pragma unroll
+    for (int r = 0; r < 9; ++r) len += s_row[r][t].y - s_row[r][t].x;
+    // records [lo, hi) of all nine rows
+    lo = (uint32_t)((uint64_t)len * sub / SUB);
+    hi = (uint32_t)((uint64_t)len * (sub + 1) / SUB);
+  }
+  if constexpr (!ROWS) {
+    // row after row without waiting for the warp's longer rows
+    uint2 se = make_uint2(0, 0);
+    int r = -1;
+    uint32_t left = hi - lo;
+    if (SUB > 1) {
+      while (left > 0) {
+        se = s_row[++r][t];
+        if (lo < se.y - se.x) break;
+        lo -= se.y - se.x;
+      }
+      se.x += lo;
+    }
+#pragma unroll 1
+    for (; left > 0; --left) {
+      while (se.x == se.y) se = s_row[++r][t];
+      add(se.x++);
+    }
+  } else {
+#pragma unroll 1
+    for (int r = 0; r < 9 && hi > 0; ++r) {
+      const uint2 se = s_row[r][t];
+      const uint32_t l = se.y - se.x, a = min(lo, l), b = min(hi, l);
+      for (uint32_t j = se.x + a; j < se.x + b; ++j) add(j);
+      lo -= a;
+      hi -= b;
+    }
+  }
+  float v[2][3];
+#pragma unroll
+  for (int q = 0; q < 2; ++q)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      float hi;
+      f2_split(sum[q][c], v[q][c], hi);
+      v[q][c] += hi;
+    }
+  if constexpr (SUB > 1) {
+    __shared__ float s_sum[SUB - 1][6][T];
+    __shared__ int s_cnt[COUNT ? SUB - 1 : 1][2][T];
     if (sub > 0) {
 #pragma unroll
-      for (int c = 0; c < 3; ++c) s_sum[sub - 1][c][t] = v[c];
-      if (COUNT) s_cnt[sub - 1][t] = cnt;
+      for (int c = 0; c < 6; ++c) s_sum[sub - 1][c][t] = v[c / 3][c % 3];
+      if (COUNT) {
+        s_cnt[sub - 1][0][t] = cnt[0];
+        s_cnt[sub - 1][1][t] = cnt[1];
+      }
     }
     __syncthreads();
     if (sub > 0) return;
 #pragma unroll
     for (int q = 0; q < SUB - 1; ++q) {
 #pragma unroll
-      for (int c = 0; c < 3; ++c) v[c] += s_sum[q][c][t];
-      if (COUNT) cnt += s_cnt[q][t];
+      for (int c = 0; c < 6; ++c) v[c / 3][c % 3] += s_sum[q][c][t];
+      if (COUNT) {
+        cnt[0] += s_cnt[q][0][t];
+        cnt[1] += s_cnt[q][1][t];
+      }
     }
   }
   if (!valid) return;
-  const uint32_t i = sorted_idx[k];
-  const bool nan = px == 3.0e38f;  // a NaN position has no neighbours
-  ax[i] = nan ? 0.f : G * v[0];
-  ay[i] = nan ? 0.f : G * v[1];
-  az[i] = nan ? 0.f : G * v[2];
-  if (COUNT) counts[i] = nan ? 0 : cnt;
+  const uint2 who = reinterpret_cast<const uint2*>(idx)[me];
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    const uint32_t i = q ? who.y : who.x;
+    if (i == kNoBody) continue;
+    const bool nan = px[q] == kFarAway;  // a NaN position has no neighbours
+    ax[i] = nan ? 0.f : G * v[q][0];
+    ay[i] = nan ? 0.f : G * v[q][1];
+    az[i] = nan ? 0.f : G * v[q][2];
+    if (COUNT) counts[i] = nan ? 0 : cnt[q];
+  }
 }
 
 static unsigned grid1d(int64_t n, int threads = 256) {
@@ -321,10 +395,17 @@ static unsigned grid1d(int64_t n, int threads = 256) {
       1, std::min<int64_t>(ceil_div(std::max<int64_t>(n, 1), threads), (int64_t)num_sms() * 32));
 }
 
-// One thread per target of the gather from this many bodies on, below it nine
-// (one per neighbour row): N = 1M at 8 bodies per cell 209 against 226 us,
-// N = 200 K 55 against 53, N = 60 K at 114 bodies per cell 343 against 126.
-constexpr int64_t kHashOneThreadMin = 400000;
+// How the gather's work is split (in us, uniform cubes):
+//  threads per pair  at 8 bodies per cell 30 K: 9 take 14, 4 take 18, 1 takes 43;
+//                    400 K: 90, 80, 93; 1M: 215, 186, 176;
+//                    at 64 and more per cell 60 K bodies: 16 take 116, 9 take 121;
+//                    500 K: 516, 460
+//  rows or one run   of records per thread: 60 K at 114 per cell 121 against 128, 1M
+//                    at 200 per cell 2462 against 2691; 1M at 8 per cell 291
+//                    against 215.
+constexpr int64_t kHashDense = 24;         // bodies per cell on average
+constexpr int64_t kHashSplitMax = 131072;  // bodies
+constexpr int64_t kHashWholeMin = 524288;  // bodies
 
 void hash_forces(nbgb_calculator* c, const float4* pm, int64_t n, float* ax, float* ay,
                  float* az) {
@@ -370,45 +451,56 @@ void hash_forces(nbgb_calculator* c, const float4* pm, int64_t n, float* ax, flo
   // 2. assign cells
   stage_mark(timer, "spatial_hash.assign");
   int32_t* pc = h.particle_cell.ensure((size_t)n);
-  uint32_t* placed = h.placed.ensure((size_t)n);
-  uint32_t* cells = h.cells.ensure((size_t)n);
-  uint32_t* idx = h.idx.ensure((size_t)n);
+  uint32_t* count = h.count.ensure((size_t)total + 1);
+  uint32_t* start = h.start.ensure((size_t)total + 1);
+  const size_t slots = (size_t)(n + std::min(n, total));  // at most
+  uint32_t* placed = h.placed.ensure(slots);
+  uint32_t* idx = h.idx.ensure(slots);
+  uint32_t* cells = h.cells.ensure(slots / 2 + 1);
+  float4* pairs = h.pairs.ensure(slots + 1);
   uint32_t* place = idx;  // free until the last kernel fills it
-  uint32_t* start = h.cell_start.ensure((size_t)total + 1);
-  float4* spm = h.sorted_pm.ensure((size_t)n + 1);
   uint32_t* sws = h.scan_ws.ensure(scan_workspace_elems(total + 1));
-  NBGB_CUDA(cudaMemsetAsync(start, 0, ((size_t)total + 1) * sizeof(uint32_t), st));
-  hash_count_kernel<<<grid1d(n), 256, 0, st>>>(pm, n, g, pc, start, place);
+  NBGB_CUDA(cudaMemsetAsync(count, 0, ((size_t)total + 1) * sizeof(uint32_t), st));
+  hash_count_kernel<<<grid1d(n), 256, 0, st>>>(pm, n, g, pc, count, place);
   NBGB_LAUNCH_CHECK();
   // 3. cell starts and places
   stage_mark(timer, "spatial_hash.sort");
-  scan_exclusive_u32(start, start, total + 1, sws, nullptr, st);
+  scan_exclusive_even_u32(count, start, total + 1, sws, st);
   hash_place_kernel<<<grid1d(n), 256, 0, st>>>(pc, place, start, n, placed);
   NBGB_LAUNCH_CHECK();
   // 4.-5. order within the cells, and records in that order
   stage_mark(timer, "spatial_hash.cells");
-  hash_order_kernel<<<(unsigned)ceil_div(n + 1, kHashCrowd), kHashCrowd, 0, st>>>(
-      pm, g, placed, start, n, cells, idx, reinterpret_cast<float*>(spm));
+  hash_order_kernel<<<(unsigned)ceil_div((int64_t)slots, kHashCrowd), kHashCrowd, 0, st>>>(
+      pm, n, g, total, placed, count, start, cells, idx, reinterpret_cast<float*>(pairs));
   NBGB_LAUNCH_CHECK();
   // 6. cutoff gather
   stage_mark(timer, "spatial_hash.forces");
   const float eps = c->params.softening, rc = c->params.cutoff;
-  const bool count = (c->params.flags & NBGB_FLAG_COUNT_INTERACTIONS) != 0;
-  int32_t* counts = count ? c->counts.ensure((size_t)n) : nullptr;
-  const auto force = [&](auto cnt, auto sub) {
-    constexpr int S = decltype(sub)::value, T = S == 1 ? 256 : 32;
-    hash_force_kernel<decltype(cnt)::value, S>
-        <<<(unsigned)ceil_div(n, T), T * S, 0, st>>>(spm, cells, idx, start,
-                                                     n, g, rc * rc, eps * eps, c->params.G, ax,
-                                                     ay, az, counts);
+  const bool counting = (c->params.flags & NBGB_FLAG_COUNT_INTERACTIONS) != 0;
+  int32_t* counts = counting ? c->counts.ensure((size_t)n) : nullptr;
+  const auto force = [&](auto cnt, auto sub, auto rows) {
+    constexpr int S = decltype(sub)::value, T = S == 1 ? 128 : S == 4 ? 64 : 32;
+    hash_force_kernel<decltype(cnt)::value, S, T, decltype(rows)::value>
+        <<<(unsigned)ceil_div((int64_t)(slots / 2), T), T * S, 0, st>>>(
+            pairs, cells, idx, start, total, g, rc * rc, eps * eps, c->params.G, ax, ay, az,
+            counts);
   };
   const auto pick = [&](auto cnt) {
-    if (n >= kHashOneThreadMin)
-      force(cnt, std::integral_constant<int, 1>{});
-    else
-      force(cnt, std::integral_constant<int, 9>{});
+    using std::integral_constant;
+    if (n >= kHashDense * total) {
+      if (n < kHashSplitMax)
+        force(cnt, integral_constant<int, 16>{}, std::true_type{});
+      else
+        force(cnt, integral_constant<int, 9>{}, std::true_type{});
+    } else if (n < kHashSplitMax) {
+      force(cnt, integral_constant<int, 9>{}, std::false_type{});
+    } else if (n < kHashWholeMin) {
+      force(cnt, integral_constant<int, 4>{}, std::false_type{});
+    } else {
+      force(cnt, integral_constant<int, 1>{}, std::false_type{});
+    }
   };
-  if (count)
+  if (counting)
     pick(std::true_type{});
   else
     pick(std::false_type{});
@@ -443,16 +535,32 @@ nbgb_status nbgb_hash_copy_cells(nbgb_calculator* c, int32_t* cell_start, int32_
   HashState& h = *c->hash;
   if (cudaStreamSynchronize(c->stream) != cudaSuccess) return NBGB_ERR_CUDA;
   const size_t tot = (size_t)h.total, n = (size_t)h.n;
+  std::vector<uint32_t> cnt, idx;
+  try {
+    cnt.resize(tot);
+    idx.resize(sorted_indices ? n + std::min(n, tot) : 0);
+  } catch (...) {
+    return NBGB_ERR_OOM;
+  }
   cudaError_t e = cudaSuccess;
-  if (cell_start && e == cudaSuccess)
-    e = cudaMemcpy(cell_start, h.cell_start.ptr, tot * 4, cudaMemcpyDeviceToHost);
-  if (cell_end && e == cudaSuccess)
-    e = cudaMemcpy(cell_end, h.cell_start.ptr + 1, tot * 4, cudaMemcpyDeviceToHost);
+  if ((cell_start || cell_end || sorted_indices) && e == cudaSuccess)
+    e = cudaMemcpy(cnt.data(), h.count.ptr, tot * 4, cudaMemcpyDeviceToHost);
+  if (sorted_indices && e == cudaSuccess)
+    e = cudaMemcpy(idx.data(), h.idx.ptr, idx.size() * 4, cudaMemcpyDeviceToHost);
   if (particle_cells && e == cudaSuccess)
     e = cudaMemcpy(particle_cells, h.particle_cell.ptr, n * 4, cudaMemcpyDeviceToHost);
-  if (sorted_indices && e == cudaSuccess)
-    e = cudaMemcpy(sorted_indices, h.idx.ptr, n * 4, cudaMemcpyDeviceToHost);
-  return e == cudaSuccess ? NBGB_OK : NBGB_ERR_CUDA;
+  if (e != cudaSuccess) return NBGB_ERR_CUDA;
+  // the slots without a body left out
+  size_t at = 0, slot = 0;
+  for (size_t c = 0; c < tot; ++c) {
+    if (cell_start) cell_start[c] = (int32_t)at;
+    if (sorted_indices)
+      for (uint32_t k = 0; k < cnt[c]; ++k) sorted_indices[at + k] = (int32_t)idx[slot + k];
+    at += cnt[c];
+    slot += (cnt[c] + 1u) & ~1u;
+    if (cell_end) cell_end[c] = (int32_t)at;
+  }
+  return NBGB_OK;
 }
 
 }  // extern "C"

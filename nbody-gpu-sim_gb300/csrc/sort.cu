@@ -30,6 +30,13 @@ constexpr int kScanChunk = kScanThreads * kScanItems;
 constexpr int kScanOneBlock = 16384;  // values that one block scans in one launch
 
 // ---------------------------------------------------------------- scan --
+// EVEN: the inputs rounded up to even numbers.
+template <bool EVEN>
+__device__ __forceinline__ uint32_t scan_in(uint32_t v) {
+  return EVEN ? (v + 1u) & ~1u : v;
+}
+
+template <bool EVEN>
 __global__ void scan_reduce_kernel(const uint32_t* __restrict__ in, int64_t n,
                                    uint32_t* __restrict__ block_sums) {
   __shared__ uint32_t s[kScanThreads / 32];
@@ -37,7 +44,7 @@ __global__ void scan_reduce_kernel(const uint32_t* __restrict__ in, int64_t n,
   uint32_t acc = 0;
   for (int k = 0; k < kScanItems; ++k) {
     int64_t i = base + (int64_t)k * kScanThreads + threadIdx.x;
-    if (i < n) acc += in[i];
+    if (i < n) acc += scan_in<EVEN>(in[i]);
   }
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
   if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = acc;
@@ -50,7 +57,8 @@ __global__ void scan_reduce_kernel(const uint32_t* __restrict__ in, int64_t n,
 }
 
 // Exclusive scan of `n` values by one block (n up to a few hundred thousand).
-__global__ void scan_single_block_kernel(uint32_t* __restrict__ data, int64_t n,
+template <bool EVEN>
+__global__ void scan_single_block_kernel(const uint32_t* in, uint32_t* data, int64_t n,
                                          uint32_t* __restrict__ total) {
   __shared__ uint32_t s_carry;
   __shared__ uint32_t s_warp[32];
@@ -59,7 +67,7 @@ __global__ void scan_single_block_kernel(uint32_t* __restrict__ data, int64_t n,
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   for (int64_t base = 0; base < n; base += blockDim.x) {
     int64_t i = base + threadIdx.x;
-    uint32_t v = (i < n) ? data[i] : 0u;
+    uint32_t v = (i < n) ? scan_in<EVEN>(in[i]) : 0u;
     uint32_t x = v;
     for (int o = 1; o < 32; o <<= 1) {
       uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
@@ -86,6 +94,7 @@ __global__ void scan_single_block_kernel(uint32_t* __restrict__ data, int64_t n,
   if (total && threadIdx.x == 0) *total = s_carry;
 }
 
+template <bool EVEN>
 __global__ void scan_apply_kernel(const uint32_t* __restrict__ in, int64_t n,
                                   const uint32_t* __restrict__ block_offsets,
                                   uint32_t* __restrict__ out) {
@@ -96,7 +105,7 @@ __global__ void scan_apply_kernel(const uint32_t* __restrict__ in, int64_t n,
   // kScanItems consecutive items.
   for (int k = 0; k < kScanItems; ++k) {
     int64_t i = base + (int64_t)k * kScanThreads + threadIdx.x;
-    s_vals[k * kScanThreads + threadIdx.x] = (i < n) ? in[i] : 0u;
+    s_vals[k * kScanThreads + threadIdx.x] = (i < n) ? scan_in<EVEN>(in[i]) : 0u;
   }
   __syncthreads();
   uint32_t local[kScanItems];
@@ -129,21 +138,32 @@ __global__ void scan_apply_kernel(const uint32_t* __restrict__ in, int64_t n,
 
 size_t scan_workspace_elems(int64_t n) { return (size_t)ceil_div(std::max<int64_t>(n, 1), kScanChunk) + 1; }
 
-void scan_exclusive_u32(const uint32_t* in, uint32_t* out, int64_t n, uint32_t* ws,
-                        uint32_t* total, cudaStream_t st) {
+template <bool EVEN>
+static void scan_exclusive(const uint32_t* in, uint32_t* out, int64_t n, uint32_t* ws,
+                           uint32_t* total, cudaStream_t st) {
   if (n <= 0) return;
-  if (in == out && n <= kScanOneBlock) {
-    scan_single_block_kernel<<<1, 1024, 0, st>>>(out, n, total);
+  if (n <= kScanOneBlock) {
+    scan_single_block_kernel<EVEN><<<1, 1024, 0, st>>>(in, out, n, total);
     NBGB_LAUNCH_CHECK();
     return;
   }
   const int64_t nb = ceil_div(n, kScanChunk);
-  scan_reduce_kernel<<<(unsigned)nb, kScanThreads, 0, st>>>(in, n, ws);
+  scan_reduce_kernel<EVEN><<<(unsigned)nb, kScanThreads, 0, st>>>(in, n, ws);
   NBGB_LAUNCH_CHECK();
-  scan_single_block_kernel<<<1, 1024, 0, st>>>(ws, nb, total);
+  scan_single_block_kernel<false><<<1, 1024, 0, st>>>(ws, ws, nb, total);
   NBGB_LAUNCH_CHECK();
-  scan_apply_kernel<<<(unsigned)nb, kScanThreads, 0, st>>>(in, n, ws, out);
+  scan_apply_kernel<EVEN><<<(unsigned)nb, kScanThreads, 0, st>>>(in, n, ws, out);
   NBGB_LAUNCH_CHECK();
+}
+
+void scan_exclusive_u32(const uint32_t* in, uint32_t* out, int64_t n, uint32_t* ws,
+                        uint32_t* total, cudaStream_t st) {
+  scan_exclusive<false>(in, out, n, ws, total, st);
+}
+
+void scan_exclusive_even_u32(const uint32_t* in, uint32_t* out, int64_t n, uint32_t* ws,
+                             cudaStream_t st) {
+  scan_exclusive<true>(in, out, n, ws, nullptr, st);
 }
 
 // ----------------------------------------------------------- radix sort --

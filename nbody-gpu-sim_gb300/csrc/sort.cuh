@@ -17,6 +17,9 @@ size_t radix_hist_elems(int64_t n);
 // total (device pointer, may be null) receives the sum of all n inputs.
 void scan_exclusive_u32(const uint32_t* in, uint32_t* out, int64_t n, uint32_t* ws,
                         uint32_t* total, cudaStream_t st);
+// The same of the inputs rounded up to even numbers.
+void scan_exclusive_even_u32(const uint32_t* in, uint32_t* out, int64_t n, uint32_t* ws,
+                             cudaStream_t st);
 
 // Stable LSD radix sort of (keys, vals) on bits [begin_bit, end_bit), 8 bits
 // per pass, ping-ponging with the *_alt buffers.  *result_in_alt tells which

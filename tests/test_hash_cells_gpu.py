@@ -4,8 +4,8 @@ Cell ids, cell starts, the ascending index list and neighbour counts equal the
 oracle's bit for bit; forces agree within 1e-5 (p99, vector relative), as in
 tests/test_hash_gpu.py.  Covered: cells of fewer, as many and more bodies than a
 block has slots, next to each other and astride blocks; all bodies in one
-place; cell tables on both sides of the one-block scan; the body count from which
-one thread takes a target, with odd counts; and bodies with a NaN position.
+place; cell tables on both sides of the one-block scan; the lines between the
+ways the gather's work is split; positions far from the origin and NaN positions.
 """
 from __future__ import annotations
 
@@ -70,9 +70,27 @@ def test_table_sizes(nb, orc, side):
     _check(nb, orc, _uniform(3001, side, seed=int(side)))
 
 
-@pytest.mark.parametrize("n", [399999, 400000, 400001])
-def test_gather_lines(nb, orc, n):
-    _check(nb, orc, _cube(n, seed=n), targets=np.random.default_rng(1).choice(n, 20000, replace=False))
+# on both sides of each line of the gather's split
+@pytest.mark.parametrize("n,per_cell", [(131071, 8), (131072, 8), (524287, 8), (524289, 8),
+                                        (20001, 22), (20001, 60), (131071, 60), (131073, 60)])
+def test_split_lines(nb, orc, n, per_cell):
+    s = _cube(n, density=per_cell / 8.0, seed=n)
+    _check(nb, orc, s, targets=np.random.default_rng(2).choice(n, 10000, replace=False))
+
+
+@pytest.mark.parametrize("at", [-1.0e29, 1.0e29])
+def test_far_from_the_origin(nb, at):
+    # an empty slot's offset must not overflow: three bodies in one place, one beside
+    s = {"x": np.full(4, at, np.float32), "y": np.array([0, 0, 0, 1], np.float32),
+         "z": np.zeros(4, np.float32), "m": np.ones(4, np.float32)}
+    (ax, ay, az), _, nbrs = _run(nb, s)
+    assert nbrs.tolist() == [3, 3, 3, 3]
+    assert np.all(ax == 0.0) and np.all(az == 0.0)
+    f = 1.0 / (1.0 + 1e-4) ** 1.5
+    np.testing.assert_allclose(ay, [f, f, f, -3 * f], rtol=1e-5)
+    (ax, ay, az), _, nbrs = _run(nb, {k: v[:3] for k, v in s.items()})
+    assert nbrs.tolist() == [2, 2, 2]
+    assert np.all(ax == 0.0) and np.all(ay == 0.0) and np.all(az == 0.0)
 
 
 @pytest.mark.parametrize("n", [2001, 400001])
