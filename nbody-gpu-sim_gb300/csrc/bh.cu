@@ -611,7 +611,7 @@ static uint32_t* seg_minmax_zeroed(BHState& h, cudaStream_t st) {
 // Builds the trees of all segments (positions and masses read from `pm` at
 // each segment's offset).
 void bh_build(BHState& h, const float4* pm, cudaStream_t st, uint32_t* err, bool groups,
-              int group_max, bool ref_tree, StageTimer* timer) {
+              int group_max, bool ref_tree, StageTimer* timer, uint32_t* total) {
   stage_mark(timer, "barnes_hut.bounds");
   h.built = false;  // until every kernel of this build is enqueued
   h.groups_ready = false;
@@ -720,7 +720,7 @@ void bh_build(BHState& h, const float4* pm, cudaStream_t st, uint32_t* err, bool
     return;
   }
   // 3.-5. nodes, groups, centres of mass (bh_nodes.cu)
-  bh_nodes(h, groups, group_max, err, timer, st);
+  bh_nodes(h, groups, group_max, err, timer, total, st);
   h.built = true;
 }
 
@@ -823,34 +823,44 @@ void bh_forces(nbgb_calculator* c, const float4* pm, int64_t n, float* ax, float
   const bool groups = (c->params.flags & NBGB_FLAG_GROUP_WALK) != 0;
   StageTimer* timer = stage_timer(c);
   if (!sync) bh_reserve_async(h);
-  for (int attempt = 0; attempt < 2; ++attempt) {
-    // asynchronously the reference's tree is always replayed; synchronously
-    // the canonical tree is built first and replaced only where it can differ
-    bh_build(h, pm, st, err, groups, c->params.group_size, ref_tree && !sync, timer);
-    if (!sync) break;  // capacity overflow surfaces through the device error word
-    // The node count is data dependent: read it back and regrow once if the
-    // capacity was too small (the kernels skipped their work in that case).
-    uint32_t* hs = h.h_scalars.ensure(2);
-    NBGB_CUDA(cudaMemcpyAsync(hs, h.scalars.ptr, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-    NBGB_CUDA(cudaStreamSynchronize(st));
-    if ((int64_t)hs[0] <= h.cap) {
-      // The reference stops splitting once node_count + 33 >= 2N.  Its node
-      // count only grows during the insertion and ends at the canonical
-      // count when the budget never fires, so a canonical count below
-      // 2N - 33 proves that it never fires and the trees are the same.
-      if (ref_tree && (int64_t)hs[0] + kMaxDepth + 1 >= 2 * n)
-        bh_build(h, pm, st, err, groups, c->params.group_size, true, timer);
-      break;
-    }
-    c->err.take();  // the skipped kernels' capacity bit (the stream is idle)
-    h.cap = (int64_t)hs[0] + (int64_t)hs[0] / 8 + 64;
-  }
-  BHWalkParams wp{c->params.G, c->params.softening, c->params.theta, c->params.leaf_capacity,
-                  (c->params.flags & NBGB_FLAG_GROUP_WALK) ? 1 : 0};
+  const BHWalkParams wp{c->params.G, c->params.softening, c->params.theta, c->params.leaf_capacity,
+                        groups ? 1 : 0};
   const bool count = (c->params.flags & NBGB_FLAG_COUNT_INTERACTIONS) != 0;
   int32_t* counts = count ? c->counts.ensure((size_t)n) : nullptr;
-  stage_mark(timer, "barnes_hut.walk");
-  bh_walk(h, wp, ax, ay, az, counts, nullptr, err, st);
+  auto walk = [&] {
+    stage_mark(timer, "barnes_hut.walk");
+    bh_walk(h, wp, ax, ay, az, counts, nullptr, err, st);
+  };
+  // asynchronously the reference's tree is always replayed; synchronously
+  // the canonical tree is built first and replaced only where it can differ
+  uint32_t* total = sync ? h.h_scalars.ensure(2) : nullptr;
+  bh_build(h, pm, st, err, groups, c->params.group_size, ref_tree && !sync, timer, total);
+  if (!sync) {  // capacity overflow surfaces through the device error word
+    walk();
+    return;
+  }
+  // The node count is data dependent: the build writes it to mapped host memory,
+  // too, and if the capacity was too small the build's later kernels and the walk
+  // have skipped their work; then once more with the capacity it takes.  The walk
+  // does not wait for the host to look (14 us at 20 K bodies).
+  if (!ref_tree) walk();
+  NBGB_CUDA(cudaStreamSynchronize(st));
+  const int64_t nodes = (int64_t)*(volatile uint32_t*)total;
+  if (nodes > h.cap) {
+    c->err.take();  // the skipped kernels' capacity bit (the stream is idle)
+    h.cap = nodes + nodes / 8 + 64;
+    bh_build(h, pm, st, err, groups, c->params.group_size, false, timer, total);
+    if (!ref_tree) walk();
+  }
+  // The reference stops splitting once node_count + 33 >= 2N.  Its node
+  // count only grows during the insertion and ends at the canonical
+  // count when the budget never fires, so a canonical count below
+  // 2N - 33 proves that it never fires and the trees are the same.
+  if (ref_tree) {
+    if (nodes + kMaxDepth + 1 >= 2 * n)
+      bh_build(h, pm, st, err, groups, c->params.group_size, true, timer, nullptr);
+    walk();
+  }
 }
 
 // ------------------------------------------------------------- export --

@@ -57,8 +57,10 @@ void bh_reserve_buffers(BHState& h, bool groups);
 // ref_tree: the reference's insertion tree (node budget included) instead of
 // the canonical one; one segment of at most 65,536 bodies, no groups.
 // timer: stage marks for NBGB_FLAG_STAGE_TIMINGS (or null).
+// total: mapped host memory that receives a canonical tree's node count (or null).
 void bh_build(BHState& h, const float4* pm, cudaStream_t st, uint32_t* err, bool groups,
-              int group_max = 0, bool ref_tree = false, StageTimer* timer = nullptr);
+              int group_max = 0, bool ref_tree = false, StageTimer* timer = nullptr,
+              uint32_t* total = nullptr);
 // Accelerations of all segments, written at each segment's offset into
 // ax/ay/az.  counts (per arena index) and inter_total (running sum) are
 // optional; err receives device error bits (group walk stack overflow).

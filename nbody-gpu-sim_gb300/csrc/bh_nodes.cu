@@ -123,6 +123,7 @@ struct NodeArgs {
   uint32_t* done;     // blocks counted (zero before)
   uint32_t* nstart;
   uint32_t* total;    // nodes
+  uint32_t* total_host;  // the same in mapped host memory (or null)
   const float4* spm;
   const BBox* box;
   const int64_t* base;  // segment s occupies sorted positions [base[s], base[s+1])
@@ -234,6 +235,7 @@ __global__ void __launch_bounds__(kNodeBlock) lcp_count_kernel(NodeArgs a) {
   if (tid == 0) {
     a.nstart[a.n] = run;
     *a.total = run;
+    if (a.total_host) *a.total_host = run;
   }
   // minima over 32^2 .. and the padding of every level
   int64_t m = (a.n + 31) / 32;  // entries of the level below
@@ -813,7 +815,7 @@ static unsigned grid1d(int64_t n, int threads = 256) {
 }
 
 void bh_nodes(BHState& h, bool groups, int group_max, uint32_t* err, StageTimer* timer,
-              cudaStream_t st) {
+              uint32_t* total, cudaStream_t st) {
   stage_mark(timer, "barnes_hut.nodes");
   const int64_t n = h.n;
   const int nseg = h.nseg;
@@ -833,6 +835,7 @@ void bh_nodes(BHState& h, bool groups, int group_max, uint32_t* err, StageTimer*
   a.done = reinterpret_cast<uint32_t*>(depth + nseg);
   a.nstart = grow(h.nstart, R + 1);
   a.total = grow(h.scalars, 2);
+  a.total_host = total;
   a.spm = h.spm.ptr;
   a.box = h.box.ptr;
   a.base = h.seg_base_p;

@@ -177,7 +177,7 @@ int bh_group_stack_limit();
 
 // Nodes, groups and centres of mass of the sorted bodies (bh_nodes.cu).
 void bh_nodes(BHState& h, bool groups, int group_max, uint32_t* err, StageTimer* timer,
-              cudaStream_t st);
+              uint32_t* total, cudaStream_t st);
 size_t lcp_bytes(int64_t n);
 
 }  // namespace nbgb
