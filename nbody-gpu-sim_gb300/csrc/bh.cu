@@ -95,8 +95,8 @@ __device__ __forceinline__ float ord2f(uint32_t u) {
 // block also clears the counters that the rest of the build starts from (a
 // memset each would cost as much as a small kernel).
 struct ZeroList {
-  uint32_t* p[3];
-  uint32_t words[3];
+  uint32_t* p[4];
+  uint32_t words[4];
 };
 
 __device__ __forceinline__ void seg_box(const uint32_t* mm, int nseg, int s, BBox* box,
@@ -125,6 +125,7 @@ __device__ __forceinline__ void seg_box(const uint32_t* mm, int nseg, int s, BBo
 __global__ void seg_bounds_kernel(const float4* __restrict__ pm, SegView sv, int64_t n, int nseg,
                                   uint32_t* __restrict__ mm, BBox* __restrict__ box,
                                   ZeroList zero, uint32_t* err) {
+  chain_begin();
   __shared__ float s_red[32][6];
   __shared__ int s_same;
   __shared__ bool s_last;
@@ -190,7 +191,7 @@ __global__ void seg_bounds_kernel(const float4* __restrict__ pm, SegView sv, int
   __syncthreads();
   for (int i = threadIdx.x; i < 6 * nseg + 1; i += blockDim.x) mm[i] = 0;
 #pragma unroll
-  for (int z = 0; z < 3; ++z)
+  for (int z = 0; z < 4; ++z)
     for (uint32_t i = threadIdx.x; i < zero.words[z]; i += blockDim.x) zero.p[z][i] = 0;
 }
 
@@ -252,6 +253,7 @@ __device__ __forceinline__ bool tie_less(const float4& pa, uint32_t a, const flo
 __global__ void tie_order_kernel(SegView sv, int64_t n, const int32_t* __restrict__ kseg,
                                  const u64* __restrict__ hi, uint32_t* __restrict__ body,
                                  u64* __restrict__ lo, float4* __restrict__ spm) {
+  chain_begin();
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k + 1 < n;
        k += (int64_t)gridDim.x * blockDim.x) {
     if (k > 0 && hi[k - 1] == hi[k] && kseg[k - 1] == kseg[k]) continue;
@@ -625,12 +627,12 @@ void bh_build(BHState& h, const float4* pm, cudaStream_t st, uint32_t* err, bool
   const ZeroList zero{
       {reinterpret_cast<uint32_t*>(grow(h.psort_ws, path_sort_ws_bytes())),
        reinterpret_cast<uint32_t*>(grow(h.seg_depth, (size_t)nseg + 2)),
-       reinterpret_cast<uint32_t*>(grow(h.group_ctr, sizeof(GroupCounters)))},
+       reinterpret_cast<uint32_t*>(grow(h.group_ctr, sizeof(GroupCounters))),
+       grow(h.walk_ctr, 2)},
       {h.sort_buckets > 0 ? (uint32_t)path_sort_zero_words() : 0u, (uint32_t)nseg + 2,
-       (uint32_t)(sizeof(GroupCounters) / sizeof(uint32_t))}};
-  seg_bounds_kernel<<<(unsigned)ceil_div(n, 1024), 256, 0, st>>>(pm, sv, n, nseg, mm, h.box.ptr,
-                                                                 zero, err);
-  NBGB_LAUNCH_CHECK();
+       (uint32_t)(sizeof(GroupCounters) / sizeof(uint32_t)), 2}};
+  launch_chained(seg_bounds_kernel, (unsigned)ceil_div(n, 1024), 256, 0, st, pm, sv, n, nseg, mm,
+                 h.box.ptr, zero, err);
   // 2. keys and order
   uint32_t* hist = grow(h.hist, radix_hist_elems((int64_t)R));
   uint32_t* sws = grow(h.scan_ws, scan_workspace_elems((int64_t)radix_hist_elems((int64_t)R)) +
@@ -677,8 +679,7 @@ void bh_build(BHState& h, const float4* pm, cudaStream_t st, uint32_t* err, bool
     NBGB_LAUNCH_CHECK();
   }
   h.body = body;
-  tie_order_kernel<<<grid1d(n), 256, 0, st>>>(sv, n, kseg, hi, body, lo, spm);
-  NBGB_LAUNCH_CHECK();
+  launch_chained(tie_order_kernel, grid1d(n), 256, 0, st, sv, n, kseg, hi, body, lo, spm);
   h.keys_valid = false;  // Morton (key, index) pairs are produced on demand
   if (ref_tree) {
     if (nseg != 1 || n > kRefTreeMaxBodies)

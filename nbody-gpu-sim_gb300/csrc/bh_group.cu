@@ -164,6 +164,7 @@ __device__ __forceinline__ void group_eval2(const float* ex, const float* ey, co
 // K times shorter, and two barriers a step are the price.
 template <int CNT, bool ZERO_EPS, bool TWO, int K>
 __global__ void __launch_bounds__(kGWarps * 32, TWO ? 3 : 4) bh_group_walk_kernel(GroupWalkArgs a) {
+  chain_begin();
   static_assert(K == 1 || !TWO, "several warps per group: groups of at most 32 bodies");
   constexpr bool COUNT = CNT == 2;
   __shared__ int s_stack[kGWarps][kGStack];
@@ -566,7 +567,8 @@ static void launch_group_walk_t(const GroupWalkArgs& g, int64_t n, cudaStream_t 
   // persistent warps: one resident wave, never more groups in flight than bodies
   const int64_t blocks =
       std::max<int64_t>(1, std::min<int64_t>(ceil_div(n, kGWarps / K), (int64_t)num_sms() * occ));
-  bh_group_walk_kernel<CNT, ZERO_EPS, TWO, K><<<(unsigned)blocks, kGWarps * 32, 0, st>>>(g);
+  launch_chained(bh_group_walk_kernel<CNT, ZERO_EPS, TWO, K>, (unsigned)blocks, kGWarps * 32, 0, st,
+                 g);
 }
 
 template <int CNT, bool ZERO_EPS>
@@ -644,7 +646,6 @@ void bh_group_walk(BHState& h, const BHWalkParams& p, float* ax, float* ay, floa
     else
       launch_group_walk<0, false>(g, n, two, st);
   }
-  NBGB_LAUNCH_CHECK();
 }
 
 }  // namespace nbgb

@@ -184,6 +184,7 @@ __device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t* s_w, uint32
 // l_k, its minima over 32 bodies, and the nodes that each block's bodies start;
 // the last block turns those into offsets and completes the minima.
 __global__ void __launch_bounds__(kNodeBlock) lcp_count_kernel(NodeArgs a) {
+  chain_begin();
   __shared__ uint8_t s_l[kNodeBlock + 1];  // l_{k0-1} ..
   __shared__ uint32_t s_w[kNodeBlock / 32];
   __shared__ bool s_last;
@@ -272,6 +273,7 @@ __global__ void __launch_bounds__(kNodeBlock) lcp_count_kernel(NodeArgs a) {
 // parent[] of a new node holds its body (a leaf: complemented) until
 // nodes_kernel has the rest.
 __global__ void __launch_bounds__(kNodeBlock) emit_nodes_kernel(NodeArgs a) {
+  chain_begin();
   __shared__ uint32_t s_w[kNodeBlock / 32];
   const uint32_t total = a.nstart[a.n];
   if ((int64_t)total > a.cap) {
@@ -341,6 +343,7 @@ __global__ void __launch_bounds__(kNodeBlock) emit_nodes_kernel(NodeArgs a) {
 // One thread per node: the internal nodes' records (range end) and every
 // node's parent.
 __global__ void nodes_kernel(NodeArgs a) {
+  chain_begin();
   const uint32_t total = a.nstart[a.n];
   if ((int64_t)total > a.cap) return;
   for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < (int64_t)total;
@@ -403,6 +406,7 @@ struct GroupSink {
 // tasks are short ones.
 __global__ void groups_kernel(const Node* __restrict__ nodes, const uint32_t* __restrict__ nstart,
                               int64_t n, int64_t cap, GroupSink gs) {
+  chain_begin();
   const uint32_t total = nstart[n];
   if ((int64_t)total > cap) return;
   const int gmax = gs.gmax;
@@ -480,6 +484,7 @@ struct ComArgs {
   int group;        // blocks per CTA of com_top_kernel
   int8_t* inner2;   // per CTA of com_top_kernel: least l within its bodies
   uint32_t* done;   // its finished CTAs (zero before)
+  unsigned long long* cost_acc;  // cleared: the coming walk adds up its own (or null)
 };
 
 // l_k as a node depth: -1 between segments, which share no node.
@@ -526,8 +531,10 @@ struct ComShared {
 };
 
 __global__ void __launch_bounds__(kComBodies) com_kernel(ComArgs a) {
+  chain_begin();
   __shared__ ComShared s;
   __shared__ int s_min[kComBodies / 32];
+  if (a.cost_acc && blockIdx.x == 0 && threadIdx.x < 2) a.cost_acc[threadIdx.x] = 0;
   const uint32_t total = a.nstart[a.n];
   if ((int64_t)total > a.cap) return;
   Node* nodes = a.nodes;
@@ -780,6 +787,7 @@ __device__ void com_edges(const ComArgs& a, TopShared& s, int E, int left, int r
 }
 
 __global__ void __launch_bounds__(kTopThreads) com_top_kernel(ComArgs a) {
+  chain_begin();
   extern __shared__ __align__(16) unsigned char top_smem[];
   TopShared& s = *reinterpret_cast<TopShared*>(top_smem);
   __shared__ bool s_last;
@@ -848,12 +856,11 @@ void bh_nodes(BHState& h, bool groups, int group_max, uint32_t* err, StageTimer*
   a.leaf_of = grow(h.leaf_of, R);
   a.err = err;
   const unsigned blocks = (unsigned)ceil_div(n, kNodeBlock);
-  lcp_count_kernel<<<blocks, kNodeBlock, 0, st>>>(a);
-  NBGB_LAUNCH_CHECK();
-  emit_nodes_kernel<<<blocks, kNodeBlock, 0, st>>>(a);
-  NBGB_LAUNCH_CHECK();
-  nodes_kernel<<<grid1d(h.cap), 256, 0, st>>>(a);
-  NBGB_LAUNCH_CHECK();
+  launch_chained(lcp_count_kernel, blocks, kNodeBlock, 0, st, a);
+  launch_chained(emit_nodes_kernel, blocks, kNodeBlock, 0, st, a);
+  launch_chained(nodes_kernel, grid1d(h.cap), 256, 0, st, a);
+  ComArgs c;
+  c.cost_acc = nullptr;
   if (groups) {
     h.group_max = group_max > 0 ? group_max : bh_group_max(n);
     uint32_t* bc_old = h.body_cost.ptr;
@@ -867,14 +874,11 @@ void bh_nodes(BHState& h, bool groups, int group_max, uint32_t* err, StageTimer*
     GroupSink gs{h.body, h.kseg.ptr, gr, gr2,
                  reinterpret_cast<GroupCounters*>(grow(h.group_ctr, sizeof(GroupCounters))),
                  h.group_max, (int64_t)h.groups.cap, bc, acc};
-    groups_kernel<<<grid1d(h.cap), 256, 0, st>>>(a.nodes, a.nstart, n, h.cap, gs);
-    NBGB_LAUNCH_CHECK();
-    // the coming walk adds up its own costs
-    NBGB_CUDA(cudaMemsetAsync(acc, 0, 2 * sizeof(unsigned long long), st));
+    launch_chained(groups_kernel, grid1d(h.cap), 256, 0, st, a.nodes, a.nstart, n, h.cap, gs);
+    c.cost_acc = acc;
   }
   h.groups_ready = groups;
   stage_mark(timer, "barnes_hut.com");
-  ComArgs c;
   c.nodes = a.nodes;
   c.spm = a.spm;
   c.nstart = a.nstart;
@@ -893,13 +897,11 @@ void bh_nodes(BHState& h, bool groups, int group_max, uint32_t* err, StageTimer*
   c.inner = reinterpret_cast<int8_t*>(h.hist.ptr);  // the node counts are free by now
   c.inner2 = c.inner + units;
   c.done = a.done + 1;
-  com_kernel<<<(unsigned)units, kComBodies, 0, st>>>(c);
-  NBGB_LAUNCH_CHECK();
+  launch_chained(com_kernel, (unsigned)units, kComBodies, 0, st, c);
   if (units > 1) {
     NBGB_CUDA(cudaFuncSetAttribute(com_top_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)sizeof(TopShared)));
-    com_top_kernel<<<(unsigned)ctas, kTopThreads, sizeof(TopShared), st>>>(c);
-    NBGB_LAUNCH_CHECK();
+    launch_chained(com_top_kernel, (unsigned)ctas, kTopThreads, sizeof(TopShared), st, c);
   }
 }
 

@@ -1,6 +1,7 @@
 // common.cuh -- shared helpers for the nbgb CUDA kernels (sm_103a only).
 #pragma once
 
+#include <utility>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -49,6 +50,34 @@ inline thread_local int64_t t_launches = 0;
     ++::nbgb::t_launches;                                                                \
     ::nbgb::cuda_check(cudaGetLastError(), "kernel launch", __FILE__, __LINE__);         \
   } while (0)
+
+// Chained launches: the kernel's blocks may take their places while the stream's
+// previous kernel still runs, and wait in chain_begin() until it has finished and
+// its writes are visible (programmatic dependent launch).  Every kernel of a chain
+// begins with chain_begin(), so a kernel that has finished implies that all before
+// it have.  A launch on an idle stream costs 2.1 us from one kernel's end to the
+// next one's start, a chained one hides most of it.
+__device__ __forceinline__ void chain_begin() {
+  cudaTriggerProgrammaticLaunchCompletion();  // the next kernel's blocks may be placed
+  cudaGridDependencySynchronize();
+}
+
+template <typename... P, typename... A>
+inline void launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
+                           cudaStream_t st, A&&... args) {
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t lc{};
+  lc.gridDim = grid;
+  lc.blockDim = block;
+  lc.dynamicSmemBytes = smem;
+  lc.stream = st;
+  lc.attrs = at;
+  lc.numAttrs = 1;
+  NBGB_CUDA(cudaLaunchKernelEx(&lc, kernel, P(std::forward<A>(args))...));
+  NBGB_LAUNCH_CHECK();
+}
 
 // ---------------------------------------------------------------------------
 // Device error word.  Kernels never trap: a bounded wait that runs out, or a

@@ -52,6 +52,7 @@ __global__ void __launch_bounds__(kBoxThreads) bbox_kernel(const float4* __restr
                                                            uint32_t* __restrict__ counter,
                                                            HostBox* __restrict__ out,
                                                            uint32_t* err) {
+  chain_begin();
   __shared__ float s[kBoxThreads / 32][6];
   __shared__ bool s_last;
   float mn[3] = {1e30f, 1e30f, 1e30f}, mx[3] = {-1e30f, -1e30f, -1e30f};
@@ -111,8 +112,7 @@ int bbox_blocks(int64_t n) {
 
 void launch_bbox(const float4* pm, int64_t n, float* partials, uint32_t* counter, HostBox* out,
                  uint32_t* err, cudaStream_t st) {
-  bbox_kernel<<<bbox_blocks(n), kBoxThreads, 0, st>>>(pm, n, partials, counter, out, err);
-  NBGB_LAUNCH_CHECK();
+  launch_chained(bbox_kernel, bbox_blocks(n), kBoxThreads, 0, st, pm, n, partials, counter, out, err);
 }
 
 }  // namespace nbgb

@@ -81,6 +81,7 @@ __device__ __forceinline__ int32_t cell_of(float4 p, const GridArgs& g) {
 __global__ void hash_count_kernel(const float4* __restrict__ pm, int64_t n, GridArgs g,
                                   int32_t* __restrict__ particle_cell,
                                   uint32_t* __restrict__ count, uint32_t* __restrict__ place) {
+  chain_begin();
   const int64_t step = (int64_t)gridDim.x * blockDim.x;
   const int lane = threadIdx.x & 31;
 #pragma unroll 4
@@ -109,6 +110,7 @@ __global__ void hash_place_kernel(const int32_t* __restrict__ particle_cell,
                                   const uint32_t* __restrict__ place,
                                   const uint32_t* __restrict__ start, int64_t n,
                                   uint32_t* __restrict__ idx) {
+  chain_begin();
   const int64_t step = (int64_t)gridDim.x * blockDim.x;
 #pragma unroll 4
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += step) {
@@ -139,6 +141,7 @@ __global__ void __launch_bounds__(kHashCrowd) hash_order_kernel(
     const uint32_t* __restrict__ placed,
     const uint32_t* __restrict__ count, const uint32_t* __restrict__ start,
     uint32_t* __restrict__ cells, uint32_t* __restrict__ idx, float* __restrict__ out) {
+  chain_begin();
   __shared__ uint32_t s_idx[kHashCrowd], s_sorted[kHashCrowd];
   __shared__ uint32_t s_hist[2][kHashCrowd + 1];
   __shared__ uint32_t s_cell[2][2];  // first and last slot's cell: start, end
@@ -245,6 +248,7 @@ __global__ void __launch_bounds__(SUB * T) hash_force_kernel(
     const uint32_t* __restrict__ idx, const uint32_t* __restrict__ start, int64_t total, GridArgs g,
     float cut2, float eps2, float G, float* __restrict__ ax, float* __restrict__ ay,
     float* __restrict__ az, int32_t* __restrict__ counts) {
+  chain_begin();
   __shared__ uint2 s_row[9][T];  // records of each neighbour row
   const int t = threadIdx.x % T, sub = threadIdx.x / T;  // pair of the block, its thread
   const int64_t npairs = start[total] >> 1;
@@ -461,18 +465,16 @@ void hash_forces(nbgb_calculator* c, const float4* pm, int64_t n, float* ax, flo
   uint32_t* place = idx;  // free until the last kernel fills it
   uint32_t* sws = h.scan_ws.ensure(scan_workspace_elems(total + 1));
   NBGB_CUDA(cudaMemsetAsync(count, 0, ((size_t)total + 1) * sizeof(uint32_t), st));
-  hash_count_kernel<<<grid1d(n), 256, 0, st>>>(pm, n, g, pc, count, place);
-  NBGB_LAUNCH_CHECK();
+  launch_chained(hash_count_kernel, grid1d(n), 256, 0, st, pm, n, g, pc, count, place);
   // 3. cell starts and places
   stage_mark(timer, "spatial_hash.sort");
   scan_exclusive_even_u32(count, start, total + 1, sws, st);
-  hash_place_kernel<<<grid1d(n), 256, 0, st>>>(pc, place, start, n, placed);
-  NBGB_LAUNCH_CHECK();
+  launch_chained(hash_place_kernel, grid1d(n), 256, 0, st, pc, place, start, n, placed);
   // 4.-5. order within the cells, and records in that order
   stage_mark(timer, "spatial_hash.cells");
-  hash_order_kernel<<<(unsigned)ceil_div((int64_t)slots, kHashCrowd), kHashCrowd, 0, st>>>(
-      pm, n, g, total, placed, count, start, cells, idx, reinterpret_cast<float*>(pairs));
-  NBGB_LAUNCH_CHECK();
+  launch_chained(hash_order_kernel, (unsigned)ceil_div((int64_t)slots, kHashCrowd), kHashCrowd, 0,
+                 st, pm, n, g, total, placed, count, start, cells, idx,
+                 reinterpret_cast<float*>(pairs));
   // 6. cutoff gather
   stage_mark(timer, "spatial_hash.forces");
   const float eps = c->params.softening, rc = c->params.cutoff;
@@ -480,10 +482,9 @@ void hash_forces(nbgb_calculator* c, const float4* pm, int64_t n, float* ax, flo
   int32_t* counts = counting ? c->counts.ensure((size_t)n) : nullptr;
   const auto force = [&](auto cnt, auto sub, auto rows) {
     constexpr int S = decltype(sub)::value, T = S == 1 ? 128 : S == 4 ? 64 : 32;
-    hash_force_kernel<decltype(cnt)::value, S, T, decltype(rows)::value>
-        <<<(unsigned)ceil_div((int64_t)(slots / 2), T), T * S, 0, st>>>(
-            pairs, cells, idx, start, total, g, rc * rc, eps * eps, c->params.G, ax, ay, az,
-            counts);
+    launch_chained(hash_force_kernel<decltype(cnt)::value, S, T, decltype(rows)::value>,
+                   (unsigned)ceil_div((int64_t)(slots / 2), T), T * S, 0, st, pairs, cells, idx,
+                   start, total, g, rc * rc, eps * eps, c->params.G, ax, ay, az, counts);
   };
   const auto pick = [&](auto cnt) {
     using std::integral_constant;
@@ -504,7 +505,6 @@ void hash_forces(nbgb_calculator* c, const float4* pm, int64_t n, float* ax, flo
     pick(std::true_type{});
   else
     pick(std::false_type{});
-  NBGB_LAUNCH_CHECK();
   h.built = true;
 }
 

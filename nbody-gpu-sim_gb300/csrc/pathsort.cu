@@ -117,6 +117,7 @@ __device__ __forceinline__ SplitKey sample_key(const PsArgs& a, int i) {
 }
 
 __global__ void ps_sample_kernel(PsArgs a) {
+  chain_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < a.nb * a.over) a.w->sample[i] = sample_key(a, i);
 }
@@ -129,6 +130,7 @@ __device__ __forceinline__ u128 wide(const SplitKey& k) {
 
 // A segment with one bucket may draw a body twice; its splitter is not used.
 __global__ void __launch_bounds__(256) ps_rank_kernel(PsArgs a) {
+  chain_begin();
   __shared__ u128 s_k[kPsChunk];
   __shared__ bool s_last;
   const int ns = a.nb * a.over;
@@ -172,6 +174,7 @@ __device__ __forceinline__ int last_not_above(const u64* hi, const uint32_t* idx
 
 // Keys, buckets and bucket counts; the last CTA scans the counts.
 __global__ void __launch_bounds__(256) ps_count_kernel(PsArgs a) {
+  chain_begin();
   extern __shared__ __align__(16) unsigned char ps_smem[];
   u64* s_hi = reinterpret_cast<u64*>(ps_smem);                    // [nb]
   uint32_t* s_idx = reinterpret_cast<uint32_t*>(s_hi + a.nb);     // [nb]
@@ -238,6 +241,7 @@ __global__ void __launch_bounds__(256) ps_count_kernel(PsArgs a) {
 // reservation per CTA and bucket.
 template <int ITEMS>
 __global__ void __launch_bounds__(256) ps_scatter_kernel(PsArgs a) {
+  chain_begin();
   __shared__ uint32_t s_cnt[kPsMaxBuckets], s_base[kPsMaxBuckets];
   for (int b = threadIdx.x; b < a.nb; b += 256) s_cnt[b] = 0;
   __syncthreads();
@@ -376,6 +380,7 @@ __device__ __forceinline__ void sort_bucket(int m, const u64* key, const uint32_
 }
 
 __global__ void __launch_bounds__(512) ps_local_kernel(PsArgs a) {
+  chain_begin();
   extern __shared__ __align__(16) unsigned char ps_smem[];
   u64* s_hi = reinterpret_cast<u64*>(ps_smem);                      // [kPsCap]
   uint32_t* s_idx = reinterpret_cast<uint32_t*>(s_hi + kPsCap);     // [kPsCap]
@@ -441,25 +446,20 @@ void path_sort(const float4* pm, const SegView& sv, const int32_t* first, int nb
   a.b = b;
   const int ns = nb * a.over;
   const dim3 g((unsigned)ceil_div(ns, 256), (unsigned)ceil_div(ns, kPsChunk));
-  ps_sample_kernel<<<(unsigned)ceil_div(ns, 64), 64, 0, st>>>(a);
-  NBGB_LAUNCH_CHECK();
-  ps_rank_kernel<<<g, 256, 0, st>>>(a);
-  NBGB_LAUNCH_CHECK();
+  launch_chained(ps_sample_kernel, (unsigned)ceil_div(ns, 64), 64, 0, st, a);
+  launch_chained(ps_rank_kernel, g, 256, 0, st, a);
   const unsigned gc =
       (unsigned)std::min<int64_t>(ceil_div(n, 256), (int64_t)num_sms() * 4);
-  ps_count_kernel<<<gc, 256, (size_t)nb * 16, st>>>(a);
-  NBGB_LAUNCH_CHECK();
+  launch_chained(ps_count_kernel, gc, 256, (size_t)nb * 16, st, a);
   stage_mark(timer, "barnes_hut.sort");
   if (n < 262144)
-    ps_scatter_kernel<2><<<(unsigned)ceil_div(n, 512), 256, 0, st>>>(a);
+    launch_chained(ps_scatter_kernel<2>, (unsigned)ceil_div(n, 512), 256, 0, st, a);
   else
-    ps_scatter_kernel<8><<<(unsigned)ceil_div(n, 2048), 256, 0, st>>>(a);
-  NBGB_LAUNCH_CHECK();
+    launch_chained(ps_scatter_kernel<8>, (unsigned)ceil_div(n, 2048), 256, 0, st, a);
   constexpr size_t smem = (size_t)kPsCap * 16 + kPsCap / 8;
   NBGB_CUDA(cudaFuncSetAttribute(ps_local_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)smem));
-  ps_local_kernel<<<(unsigned)nb, n / nb <= 512 ? 256 : 512, smem, st>>>(a);
-  NBGB_LAUNCH_CHECK();
+  launch_chained(ps_local_kernel, (unsigned)nb, n / nb <= 512 ? 256 : 512, smem, st, a);
 }
 
 }  // namespace nbgb

@@ -39,6 +39,7 @@ __device__ __forceinline__ uint32_t scan_in(uint32_t v) {
 template <bool EVEN>
 __global__ void scan_reduce_kernel(const uint32_t* __restrict__ in, int64_t n,
                                    uint32_t* __restrict__ block_sums) {
+  chain_begin();
   __shared__ uint32_t s[kScanThreads / 32];
   const int64_t base = (int64_t)blockIdx.x * kScanChunk;
   uint32_t acc = 0;
@@ -60,6 +61,7 @@ __global__ void scan_reduce_kernel(const uint32_t* __restrict__ in, int64_t n,
 template <bool EVEN>
 __global__ void scan_single_block_kernel(const uint32_t* in, uint32_t* data, int64_t n,
                                          uint32_t* __restrict__ total) {
+  chain_begin();
   __shared__ uint32_t s_carry;
   __shared__ uint32_t s_warp[32];
   if (threadIdx.x == 0) s_carry = 0;
@@ -98,6 +100,7 @@ template <bool EVEN>
 __global__ void scan_apply_kernel(const uint32_t* __restrict__ in, int64_t n,
                                   const uint32_t* __restrict__ block_offsets,
                                   uint32_t* __restrict__ out) {
+  chain_begin();
   __shared__ uint32_t s_vals[kScanChunk];
   __shared__ uint32_t s_warp[kScanThreads / 32];
   const int64_t base = (int64_t)blockIdx.x * kScanChunk;
@@ -143,17 +146,13 @@ static void scan_exclusive(const uint32_t* in, uint32_t* out, int64_t n, uint32_
                            uint32_t* total, cudaStream_t st) {
   if (n <= 0) return;
   if (n <= kScanOneBlock) {
-    scan_single_block_kernel<EVEN><<<1, 1024, 0, st>>>(in, out, n, total);
-    NBGB_LAUNCH_CHECK();
+    launch_chained(scan_single_block_kernel<EVEN>, 1, 1024, 0, st, in, out, n, total);
     return;
   }
   const int64_t nb = ceil_div(n, kScanChunk);
-  scan_reduce_kernel<EVEN><<<(unsigned)nb, kScanThreads, 0, st>>>(in, n, ws);
-  NBGB_LAUNCH_CHECK();
-  scan_single_block_kernel<false><<<1, 1024, 0, st>>>(ws, ws, nb, total);
-  NBGB_LAUNCH_CHECK();
-  scan_apply_kernel<EVEN><<<(unsigned)nb, kScanThreads, 0, st>>>(in, n, ws, out);
-  NBGB_LAUNCH_CHECK();
+  launch_chained(scan_reduce_kernel<EVEN>, (unsigned)nb, kScanThreads, 0, st, in, n, ws);
+  launch_chained(scan_single_block_kernel<false>, 1, 1024, 0, st, ws, ws, nb, total);
+  launch_chained(scan_apply_kernel<EVEN>, (unsigned)nb, kScanThreads, 0, st, in, n, ws, out);
 }
 
 void scan_exclusive_u32(const uint32_t* in, uint32_t* out, int64_t n, uint32_t* ws,
