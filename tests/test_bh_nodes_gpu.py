@@ -105,3 +105,25 @@ def test_repeated_builds_of_changing_size(nb):
         for a, b in zip(got, fresh):
             np.testing.assert_array_equal(a, b)
     calc.close()
+
+
+@pytest.mark.parametrize("group", [False, True])
+def test_forces_after_a_capacity_regrow(nb, group):
+    # chains of one-child cells need more nodes than a first call provides: the
+    # walk that followed the failed build wrote nothing that stays
+    s = _clusters(1536, 3, seed=4)
+    n = len(s["x"])
+    calc = nb.BarnesHutCalculator(0.5, group_walk=group)
+    calc.setSofteningParameter(0.01)
+    got = []
+    with nb.ScopedParticleData(n, {"pos_x": s["x"], "pos_y": s["y"], "pos_z": s["z"],
+                                   "mass": s["m"]}) as p:
+        for _ in range(2):
+            calc.computeForces(p.device)
+            p.download()
+            got.append([p.host[f"acc_{a}"].copy() for a in "xyz"])
+    assert calc.tree_stats()[0] > 3 * n + 64
+    calc.close()
+    for a, b in zip(*got):
+        assert np.all(np.isfinite(a)) and np.any(a != 0)
+        np.testing.assert_array_equal(a, b)
