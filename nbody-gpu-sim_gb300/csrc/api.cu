@@ -116,9 +116,23 @@ void check_device_errors(nbgb_calculator* c) {
   }
 }
 
-static void direct_forces(nbgb_calculator* c, const DirectSource& src, int64_t n, float* ax,
-                          float* ay, float* az) {
+static void direct_forces(nbgb_calculator* c, DirectSource src, int64_t n, float* ax, float* ay,
+                          float* az) {
   const DirectPlan p = plan_direct(n);
+  if (p.ring) {  // sources in whole tiles, the last one filled up without mass
+    const int64_t n_pad = ceil_div(n, kDirRingPad) * kDirRingPad;
+    if (!src.pm || n_pad != n) {
+      float4* t = c->tiles.ensure((size_t)n_pad);
+      if (src.pm) {
+        NBGB_CUDA(cudaMemcpyAsync(t, src.pm, (size_t)n * sizeof(float4), cudaMemcpyDeviceToDevice,
+                                  c->stream));
+        NBGB_CUDA(cudaMemsetAsync(t + n, 0, (size_t)(n_pad - n) * sizeof(float4), c->stream));
+      } else {
+        launch_pack_soa(src.x, src.y, src.z, src.m, n, n_pad, t, c->stream);
+      }
+      src.pm = t;
+    }
+  }
   float4* part = nullptr;
   uint32_t* ticket = nullptr;
   if (p.splits > 1) {
@@ -133,7 +147,7 @@ static void direct_forces(nbgb_calculator* c, const DirectSource& src, int64_t n
   const float eps = c->params.softening;
   launch_direct(p, src, n, c->params.G, eps * eps,
                 (c->params.flags & NBGB_FLAG_COMPENSATED) != 0, part, ticket, ax, ay, az,
-                c->stream);
+                c->stream, c->err.ensure(1));
 }
 
 // Direct forces straight from the caller's SoA arrays.  Accelerations that

@@ -16,6 +16,7 @@
 // the slices' sums in plain FP32.
 #include "common.cuh"
 #include "kernels.cuh"
+#include "direct_core.cuh"
 #include "direct_pair.cuh"
 
 namespace nbgb {
@@ -184,6 +185,69 @@ __global__ void __launch_bounds__(kDirThreads, 2) direct_kernel(DirectArgs a) {
   }
 }
 
+// The largest systems: one CTA of 128 threads sums 8 targets per thread, two per
+// packed operation, against 256-source tiles that the bulk-copy engine streams
+// in (direct_core.cuh, the ensembles' engine; sources padded to whole tiles).  Its
+// long inner loop without block barriers sustains up to 2 % more than the kernel
+// above (350,000 bodies 44.0 against 44.5 ms, 1M 391.5 against 401), but its blocks of
+// 1,024 targets and whole tiles split unevenly below (65,536 bodies 1.65 against
+// 1.58 ms, 131,072 6.38 against 6.30, 262,144 24.99 against 24.92).
+template <bool COMP, bool ZERO_SOFT>
+__global__ void __launch_bounds__(kDirHalf) direct_ring_kernel(DirectArgs a) {
+  constexpr int I = 8;
+  __shared__ alignas(128) float4 s_j[kRingStages][kRingTile];
+  __shared__ alignas(8) uint64_t s_bar[kRingStages];
+  TileRing ring{s_j, s_bar, 0};
+  ring_init(ring);
+  const int tid = threadIdx.x;
+  const int64_t tgt_base = (int64_t)blockIdx.x * (kDirHalf * I);
+  const int64_t tile0 = (int64_t)blockIdx.y * (a.jper / kRingTile);
+  const int64_t tile1 = imin64(tile0 + a.jper / kRingTile, a.n_src / kRingTile);
+  const int nt = (int)imax64(tile1 - tile0, 0);
+  float xi[I], yi[I], zi[I];
+#pragma unroll
+  for (int q = 0; q < I; ++q) {
+    const int64_t i = tgt_base + tid + (int64_t)q * kDirHalf;
+    const float4 p = (i < a.n_tgt) ? a.src[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    xi[q] = p.x;
+    yi[q] = p.y;
+    zi[q] = p.z;
+  }
+  float sx[I], sy[I], sz[I];
+  if (!direct_tiles<kDirHalf, I, true, COMP, ZERO_SOFT>(ring, a.src + tile0 * kRingTile, nt, xi, yi,
+                                                        zi, a.eps2, sx, sy, sz, a.err))
+    return;
+#pragma unroll
+  for (int q = 0; q < I; ++q) {
+    const int64_t i = tgt_base + tid + (int64_t)q * kDirHalf;
+    if (i >= a.n_tgt) continue;
+    if (a.splits > 1) {
+      a.partial[(int64_t)blockIdx.y * a.n_tgt_pad + i] = make_float4(sx[q], sy[q], sz[q], 0.f);
+    } else {
+      a.out_x[i] = a.G * sx[q];
+      a.out_y[i] = a.G * sy[q];
+      a.out_z[i] = a.G * sz[q];
+    }
+  }
+}
+
+// Adds the ring kernel's runs in run order.
+__global__ void direct_runs_kernel(DirectArgs a) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < a.n_tgt;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    float rx = 0.f, ry = 0.f, rz = 0.f, fx = 0.f, fy = 0.f, fz = 0.f;
+    for (int s = 0; s < a.splits; ++s) {
+      const float4 p = a.partial[(int64_t)s * a.n_tgt_pad + i];
+      fold<true>(p.x, rx, fx);
+      fold<true>(p.y, ry, fy);
+      fold<true>(p.z, rz, fz);
+    }
+    a.out_x[i] = a.G * (rx + fx);
+    a.out_y[i] = a.G * (ry + fy);
+    a.out_z[i] = a.G * (rz + fz);
+  }
+}
+
 // Targets per thread and source runs for n bodies: the pair with the least
 // estimated time, in SM clocks.  The busiest SM sums k CTAs at 8.65 (one
 // target per thread) or 8.95 interactions per clock together, 7.9 when it has
@@ -193,13 +257,44 @@ __global__ void __launch_bounds__(kDirThreads, 2) direct_kernel(DirectArgs a) {
 // 15 runs; 42 with one target, unsplit), N = 16,384 107 (two, 19 runs; 130
 // with one target, unsplit), N = 131,072 6,262 (two, 19 runs; 6,417 with
 // one); four targets per thread were nowhere faster (6,333 at N = 131,072).
-// Small systems go to steps.cu.
+// Small systems go to steps.cu, those from kDirRingMin bodies on to the ring kernel.
+constexpr int64_t kDirRingMin = 294912;
+
 DirectPlan plan_direct(int64_t n, int max_splits) {
   constexpr double kCtaClocks = 3000.0, kRunClocks = 60.0;
   n = std::max<int64_t>(n, 1);
   const int64_t sms = num_sms();
   DirectPlan best;
   if ((best.small = direct_small_fit(n))) return best;
+  if (n >= kDirRingMin) {
+    // runs so that the CTAs fill whole waves
+    static const int occ = [] {
+      int b = 0;
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, direct_ring_kernel<true, false>, kDirHalf,
+                                                    0);
+      return std::max(b, 1);
+    }();
+    best.ring = true;
+    best.per_thread = 8;
+    best.i_blocks = ceil_div(n, (int64_t)kDirHalf * 8);
+    best.n_tgt_pad = best.i_blocks * kDirHalf * 8;
+    const int64_t tiles = ceil_div(n, (int64_t)kRingTile);
+    double eff = -1.0;
+    for (int64_t s = 1; s <= std::min<int64_t>(max_splits, tiles / 4);
+         ++s) {
+      const double waves = (double)(best.i_blocks * s) / (double)(sms * occ);
+      const double e = waves / std::ceil(waves);
+      const int64_t per = ceil_div(tiles, s);
+      if (s > 1 && ceil_div(tiles, per) != s) continue;
+      if (s == 1 || e > eff + 0.02) {
+        eff = e;
+        best.splits = (int)s;
+        best.jper = per * kRingTile;
+      }
+      if (e >= 0.97) break;
+    }
+    return best;
+  }
   double best_t = 1e300;
   for (int I = 1; I <= 2; ++I) {
     const int64_t T = (int64_t)kDirHalf * I, blocks = ceil_div(n, T);
@@ -251,7 +346,7 @@ static void launch_direct_any(const DirectPlan& p, DirectArgs& a, bool comp, cud
 
 void launch_direct(const DirectPlan& p, const DirectSource& src, int64_t n, float G, float eps2,
                    bool compensated, float4* partial, uint32_t* ticket, float* ox, float* oy,
-                   float* oz, cudaStream_t st) {
+                   float* oz, cudaStream_t st, uint32_t* err) {
   if (n <= 0) return;
   if (p.small) {
     launch_direct_small(src, n, G, eps2, compensated, ox, oy, oz, st);
@@ -272,7 +367,25 @@ void launch_direct(const DirectPlan& p, const DirectSource& src, int64_t n, floa
   a.out_x = ox;
   a.out_y = oy;
   a.out_z = oz;
-  if (src.pm)
+  if (p.ring) {
+    a.err = err;
+    a.n_src = ceil_div(n, (int64_t)kRingTile) * kRingTile;
+    a.n_tgt_pad = p.n_tgt_pad;
+    a.jper = p.jper;
+    a.splits = p.splits;
+    const dim3 grid((unsigned)p.i_blocks, (unsigned)p.splits);
+    if (eps2 > 0.f)
+      compensated ? direct_ring_kernel<true, false><<<grid, kDirHalf, 0, st>>>(a)
+                  : direct_ring_kernel<false, false><<<grid, kDirHalf, 0, st>>>(a);
+    else
+      compensated ? direct_ring_kernel<true, true><<<grid, kDirHalf, 0, st>>>(a)
+                  : direct_ring_kernel<false, true><<<grid, kDirHalf, 0, st>>>(a);
+    NBGB_LAUNCH_CHECK();
+    if (p.splits > 1) {
+      direct_runs_kernel<<<(unsigned)num_sms() * 8, 256, 0, st>>>(a);
+      NBGB_LAUNCH_CHECK();
+    }
+  } else if (src.pm)
     launch_direct_any<false>(p, a, compensated, st);
   else
     launch_direct_any<true>(p, a, compensated, st);

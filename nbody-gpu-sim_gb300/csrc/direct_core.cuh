@@ -1,5 +1,5 @@
 // direct_core.cuh -- the direct-sum tile engine of the ensemble work-queue
-// kernel (ensemble.cu).
+// kernel (ensemble.cu) and of the largest systems (direct.cu).
 //
 // One CTA of THREADS threads computes THREADS*I targets against a run of
 // kRingTile-body j-tiles that the bulk-copy engine streams into a kRingStages
@@ -14,6 +14,7 @@
 namespace nbgb {
 
 constexpr int kRingTile = 256;   // bodies per shared-memory j-tile (4 KB)
+static_assert(kRingTile == kDirRingPad, "padded to whole tiles");
 constexpr int kRingStages = 3;   // bulk-copy pipeline depth
 
 struct TileRing {

@@ -28,6 +28,7 @@ struct DirectArgs {
   float* out_x;
   float* out_y;
   float* out_z;
+  uint32_t* err;     // device error word (ring)
 };
 
 // Bodies of a direct sum: pm (packed), or the SoA arrays when pm is null.
@@ -38,11 +39,12 @@ struct DirectSource {
 
 struct DirectPlan {
   bool small = false;     // the small-system kernel (one CTA set, no runs)
-  int per_thread = 1;     // targets per thread (1 or 2)
+  bool ring = false;      // the tile-ring kernel of the largest systems (packed sources)
+  int per_thread = 1;     // targets per thread (1 or 2; 8 with ring)
   int64_t i_blocks = 0;   // target blocks of kDirHalf * per_thread
   int64_t n_tgt_pad = 0;
   int splits = 1;         // source runs
-  int64_t jper = 0;       // sources per run, a multiple of 16
+  int64_t jper = 0;       // sources per run, a multiple of 16 (ring: of 256)
 };
 
 // Whether a direct sum may read the caller's arrays while it writes the
@@ -53,10 +55,12 @@ constexpr int64_t kDirMaxBlocks = 16384;  // target blocks of a plan with severa
 DirectPlan plan_direct(int64_t n, int max_splits = kDirMaxSplits);
 // Forces on all n bodies of src.  With p.splits > 1: partial holds
 // splits * n_tgt_pad entries, ticket i_blocks counters that are zero before
-// the launch and zero again after it.
+// the launch and zero again after it.  With p.ring: no ticket, and src.pm is given,
+// padded with massless bodies to a multiple of kDirRingPad.
+constexpr int64_t kDirRingPad = 256;
 void launch_direct(const DirectPlan& p, const DirectSource& src, int64_t n, float G, float eps2,
                    bool compensated, float4* partial, uint32_t* ticket, float* ox, float* oy,
-                   float* oz, cudaStream_t st);
+                   float* oz, cudaStream_t st, uint32_t* err = nullptr);
 void launch_pack_soa(const float* x, const float* y, const float* z, const float* m, int64_t n,
                      int64_t n_pad, float4* out, cudaStream_t st);
 

@@ -166,6 +166,7 @@ struct nbgb_calculator {
   int device = 0;
 
   nbgb::DevBuf<float4> pm;        // packed (x, y, z, m) input of the last drop-in call
+  nbgb::DevBuf<float4> tiles;     // direct, largest systems: the bodies in whole tiles
   nbgb::DevBuf<float4> partial;   // direct: finished runs per target block (zero between
                                   // calls), then the partial sums of the source runs
   nbgb::ErrorWord err;            // device error word
