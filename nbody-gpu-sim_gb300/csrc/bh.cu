@@ -1,6 +1,6 @@
-// bh.cu -- Barnes-Hut on the device: path keys, radix sort, octree from
-// sorted keys, bottom-up centre of mass, warp-cooperative walk (K2-K6), for
-// one system or for many independent systems ("segments") in one pass.
+// bh.cu -- Barnes-Hut on the device: bounds, path keys and their order, and the
+// octree from sorted keys (K2-K5), for one system or for many independent
+// systems ("segments") in one pass.
 //
 // Replaces BarnesHutTree::build/computeForces and BarnesHutCalculator
 // (src/cuda/force_barnes_hut.cu:125-583), whose octree is built on the host
@@ -17,10 +17,11 @@
 //   1. per segment, the bounding box and the reference's root cube; every
 //      body's path key = its 32 octants, computed with the reference's float
 //      operations (levels 1..21 in a high 63-bit key, 22..32 in a low key);
-//   2. stable radix sort by the high key, then (several segments) by
-//      segment; bodies sharing segment and high key are put in (low key,
-//      Morton key, index) order, i.e. the reference's insertion order inside
-//      a shared depth-32 cell;
+//   2. order by (segment, high key, index): a sample sort (pathsort.cu), or for
+//      larger sets a stable radix sort by the high key and then by segment;
+//      bodies sharing segment and high key are put in (low key, Morton key,
+//      index) order, i.e. the reference's insertion order inside a shared
+//      depth-32 cell;
 //   3. l_k = common levels of adjacent sorted keys of one segment; body k
 //      starts the internal nodes of depths l_{k-1}+1 .. min(l_k, 31) and
 //      (unless it shares a depth-32 cell with k-1) one leaf of depth
@@ -30,9 +31,9 @@
 //      pre-order (children in octant order): every subtree, and every
 //      segment's tree, is a contiguous index range, and
 //      skip(P) = first node of body end(P)+1;
-//   5. centres of mass bottom-up with per-node arrival counters, summing
-//      children in octant order with the reference's float operations
-//      (:514-538), so masses and centres of mass are bit-identical.
+//   5. centres of mass bottom-up, summing children in octant order with the
+//      reference's float operations (:514-538), so masses and centres of mass
+//      are bit-identical (3.-5. in bh_nodes.cu).
 //
 // The reference walk is in bh_walk.cu, the group walk (one list per group of
 // nearby bodies) in bh_group.cu; the node record, state and shared parameters
