@@ -786,6 +786,7 @@ void bh_reserve_buffers(BHState& h, bool groups) {
   grow(h.seg_root, (size_t)nseg);
   grow(h.seg_end, (size_t)nseg);
   grow(h.walk_ctr, 2);
+  grow(h.group_ctr, sizeof(GroupCounters));  // (cleared by the bounds kernel with either walk)
   if (groups) {
     grow(h.groups, R);
     h.groups2.ensure(h.groups.cap);
@@ -800,7 +801,6 @@ void bh_reserve_buffers(BHState& h, bool groups) {
       NBGB_CUDA(cudaMemset(acc, 0, 2 * sizeof(unsigned long long)));
       NBGB_CUDA(cudaDeviceSynchronize());
     }
-    grow(h.group_ctr, sizeof(GroupCounters));
     grow(h.group_ovf, (size_t)kOvfChunks * kOvfChunk);
   }
 }
