@@ -193,7 +193,10 @@ template <int TL, int I, bool COMP, bool ZS>
 static void launch_steps_t(StepArgs& a, cudaStream_t st) {
   const size_t smem = (size_t)((a.n + 3) & ~3) * 16;
   auto kern = direct_steps_kernel<TL, I, COMP, ZS>;
-  NBGB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // (one limit for all sizes: the attribute is the kernel's, and a smaller one set for a
+  // call in another thread would refuse this one's launch)
+  NBGB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)(kDirectSmallMaxBodies * 16)));
   const unsigned grid = (unsigned)ceil_div(a.n, TL * I);
   if (a.steps) {
     void* args[] = {&a};
