@@ -849,7 +849,6 @@ void bh_forces(nbgb_calculator* c, const float4* pm, int64_t n, float* ax, float
   NBGB_CUDA(cudaStreamSynchronize(st));
   const int64_t nodes = (int64_t)*(volatile uint32_t*)total;
   if (nodes > h.cap) {
-    c->err.take();  // the skipped kernels' capacity bit (the stream is idle)
     h.cap = nodes + nodes / 8 + 64;
     bh_build(h, pm, st, err, groups, c->params.group_size, false, timer, total);
     if (!ref_tree) walk();

@@ -277,7 +277,8 @@ __global__ void __launch_bounds__(kNodeBlock) emit_nodes_kernel(NodeArgs a) {
   __shared__ uint32_t s_w[kNodeBlock / 32];
   const uint32_t total = a.nstart[a.n];
   if ((int64_t)total > a.cap) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) raise_error(a.err, kErrTreeCapacity);
+    // (a host that reads the total builds again; the error word may hold earlier calls' bits)
+    if (blockIdx.x == 0 && threadIdx.x == 0 && !a.total_host) raise_error(a.err, kErrTreeCapacity);
     return;
   }
   const int64_t k = (int64_t)blockIdx.x * kNodeBlock + threadIdx.x;
