@@ -67,7 +67,7 @@ void launch_pack_soa(const float* x, const float* y, const float* z, const float
 // Small systems (steps.cu): the forces of n bodies, or `steps` kick-drift +
 // force steps in one cooperative launch.  exch: 2 n entries; ctr: two
 // counters, zero before and after.
-constexpr int64_t kDirectSmallMaxBodies = 9728;  // 16 bytes per body in shared memory
+constexpr int64_t kDirectSmallMaxBodies = 4864;  // 16 bytes per body in shared memory
 constexpr int32_t kDirectStepsPerLaunch = 256;   // bounds one launch's time
 struct StateArrays {
   double *x, *y, *z, *vx, *vy, *vz;

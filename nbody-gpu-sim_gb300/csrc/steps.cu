@@ -10,11 +10,11 @@
 // targets).  Here every CTA keeps the FP64 state of its T targets in
 // registers for all steps; per step it publishes their positions, passes one
 // grid barrier, copies all bodies to shared memory and sums them, so a step
-// costs one barrier and one read of 16 N bytes.  T = 8, 16, 32 or 64 targets
-// per CTA, the smallest that needs no more CTAs than SMs: fewer targets per
+// costs one barrier and one read of 16 N bytes.  T = 8, 16 or 32 targets per
+// CTA, the smallest that needs no more CTAs than SMs: fewer targets per
 // CTA share the sum over more threads (64 slices of the sources at T = 8).
 // Measured per step in calls of 100 steps: N = 256 2.3 us, 1,024 3.1 (80
-// before the sources were split, 11 as two launches), 4,864 12, 8,192 32.
+// before the sources were split, 11 as two launches), 4,864 12.
 // Force calculators and a system's a(0) run the same kernel (steps = 0, an
 // ordinary launch), so a trajectory does not depend on how its steps are
 // grouped into calls, and the forces of a system are a calculator's, bitwise.
@@ -63,10 +63,11 @@ __device__ __forceinline__ bool grid_barrier(uint32_t* ctr, uint32_t target, uin
   return *s_ok;
 }
 
-// TL target lanes with I targets each; 512 / TL slices of the sources.
-template <int TL, int I, bool COMP, bool ZERO_SOFT>
+// TL targets per CTA; 512 / TL slices of the sources, of at most 304 sources in
+// two plain FP32 sums (even and odd ones).
+template <int TL, bool COMP, bool ZERO_SOFT>
 __global__ void __launch_bounds__(kStepThreads, 1) direct_steps_kernel(StepArgs a) {
-  constexpr int T = TL * I, kSlices = kStepThreads / TL;
+  constexpr int T = TL, kSlices = kStepThreads / TL;
   extern __shared__ __align__(16) float s_body[];  // rows x, y, z, m of n4 floats
   __shared__ float s_red[kStepWarps][3][T];
   __shared__ bool s_ok;
@@ -119,15 +120,9 @@ __global__ void __launch_bounds__(kStepThreads, 1) direct_steps_kernel(StepArgs 
       sm[j] = q.w;
     }
     __syncthreads();
-    f2 xi[I], yi[I], zi[I], ax[I], ay[I], az[I];
-#pragma unroll
-    for (int q = 0; q < I; ++q) {
-      const int i = min(base + tl + q * TL, a.n - 1);
-      xi[q] = f2_make(sx[i], sx[i]);
-      yi[q] = f2_make(sy[i], sy[i]);
-      zi[q] = f2_make(sz[i], sz[i]);
-      ax[q] = ay[q] = az[q] = f2_make(0.f, 0.f);
-    }
+    const int i = min(base + tl, a.n - 1);
+    const f2 xi = f2_make(sx[i], sx[i]), yi = f2_make(sy[i], sy[i]), zi = f2_make(sz[i], sz[i]);
+    f2 ax = f2_make(0.f, 0.f), ay = ax, az = ax;
     const f2 e2 = f2_make(a.eps2, a.eps2);
     // the slices take quads of sources in turn: a warp's slices read
     // neighbouring 16-byte words
@@ -137,22 +132,16 @@ __global__ void __launch_bounds__(kStepThreads, 1) direct_steps_kernel(StepArgs 
       const ulonglong2 Y = *reinterpret_cast<const ulonglong2*>(sy + j);
       const ulonglong2 Z = *reinterpret_cast<const ulonglong2*>(sz + j);
       const ulonglong2 M = *reinterpret_cast<const ulonglong2*>(sm + j);
-#pragma unroll
-      for (int q = 0; q < I; ++q) {
-        pair_step<ZERO_SOFT>(f2{X.x}, f2{Y.x}, f2{Z.x}, f2{M.x}, xi[q], yi[q], zi[q], e2, ax[q],
-                             ay[q], az[q]);
-        pair_step<ZERO_SOFT>(f2{X.y}, f2{Y.y}, f2{Z.y}, f2{M.y}, xi[q], yi[q], zi[q], e2, ax[q],
-                             ay[q], az[q]);
-      }
+      pair_step<ZERO_SOFT>(f2{X.x}, f2{Y.x}, f2{Z.x}, f2{M.x}, xi, yi, zi, e2, ax, ay, az);
+      pair_step<ZERO_SOFT>(f2{X.y}, f2{Y.y}, f2{Z.y}, f2{M.y}, xi, yi, zi, e2, ax, ay, az);
     }
-#pragma unroll
-    for (int q = 0; q < I; ++q) {
-      float s[3] = {f2_sum(ax[q]), f2_sum(ay[q]), f2_sum(az[q])};
+    {
+      float s[3] = {f2_sum(ax), f2_sum(ay), f2_sum(az)};
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
 #pragma unroll
         for (int o = TL; o < 32; o <<= 1) s[c] += __shfl_xor_sync(0xffffffffu, s[c], o);
-        if (lane < TL) s_red[warp][c][tl + q * TL] = s[c];
+        if (lane < TL) s_red[warp][c][tl] = s[c];
       }
     }
     __syncthreads();
@@ -189,15 +178,15 @@ __global__ void __launch_bounds__(kStepThreads, 1) direct_steps_kernel(StepArgs 
   }
 }
 
-template <int TL, int I, bool COMP, bool ZS>
+template <int TL, bool COMP, bool ZS>
 static void launch_steps_t(StepArgs& a, cudaStream_t st) {
   const size_t smem = (size_t)((a.n + 3) & ~3) * 16;
-  auto kern = direct_steps_kernel<TL, I, COMP, ZS>;
+  auto kern = direct_steps_kernel<TL, COMP, ZS>;
   // (one limit for all sizes: the attribute is the kernel's, and a smaller one set for a
   // call in another thread would refuse this one's launch)
   NBGB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(kDirectSmallMaxBodies * 16)));
-  const unsigned grid = (unsigned)ceil_div(a.n, TL * I);
+  const unsigned grid = (unsigned)ceil_div(a.n, TL);
   if (a.steps) {
     void* args[] = {&a};
     NBGB_CUDA(cudaLaunchCooperativeKernel((const void*)kern, dim3(grid), dim3(kStepThreads), args,
@@ -208,35 +197,34 @@ static void launch_steps_t(StepArgs& a, cudaStream_t st) {
   NBGB_LAUNCH_CHECK();
 }
 
-template <int TL, int I>
+template <int TL>
 static void launch_steps_n(StepArgs& a, bool comp, cudaStream_t st) {
   const bool zs = !(a.eps2 > 0.f);
   if (zs)
-    comp ? launch_steps_t<TL, I, true, true>(a, st) : launch_steps_t<TL, I, false, true>(a, st);
+    comp ? launch_steps_t<TL, true, true>(a, st) : launch_steps_t<TL, false, true>(a, st);
   else
-    comp ? launch_steps_t<TL, I, true, false>(a, st) : launch_steps_t<TL, I, false, false>(a, st);
+    comp ? launch_steps_t<TL, true, false>(a, st) : launch_steps_t<TL, false, false>(a, st);
 }
 
-// Sizes for this kernel: up to 32 targets per CTA on at most one CTA per SM,
-// and 64 where that fills three quarters of the SMs.  Between (4,865 .. 7,296
-// bodies on 152 SMs) the source runs of direct_kernel fill the GPU better:
-// N = 6,000 21 us per sum against 24; N = 8,192 33 against 32.
+// Sizes for this kernel: up to 32 targets per CTA on at most one CTA per SM.
+// With 64 targets per CTA it took systems of up to twice that, too: alone 4 to
+// 10 % faster in calls of 20 steps (8,192 bodies 36.0 us per step against 37.5),
+// but its shared memory and its one CTA per SM keep other streams' systems
+// waiting (16 systems of 8,192 bodies on streams of their own 35.2 us per step,
+// 25.0 with the source runs of direct_kernel), and its slices added up to 608
+// sources in plain FP32.
 bool direct_small_fit(int64_t n) {
-  const int64_t sms = num_sms();
-  return n <= std::min(32 * sms, kDirectSmallMaxBodies) ||
-         (n > 48 * sms && n <= std::min(64 * sms, kDirectSmallMaxBodies));
+  return n <= std::min<int64_t>(32 * num_sms(), kDirectSmallMaxBodies);
 }
 
 static void launch_small(StepArgs& a, bool comp, cudaStream_t st) {
   const int64_t sms = num_sms();
   if (a.n <= 8 * sms)
-    launch_steps_n<8, 1>(a, comp, st);
+    launch_steps_n<8>(a, comp, st);
   else if (a.n <= 16 * sms)
-    launch_steps_n<16, 1>(a, comp, st);
-  else if (a.n <= 32 * sms)
-    launch_steps_n<32, 1>(a, comp, st);
+    launch_steps_n<16>(a, comp, st);
   else
-    launch_steps_n<32, 2>(a, comp, st);
+    launch_steps_n<32>(a, comp, st);
 }
 
 void launch_direct_small(const DirectSource& src, int64_t n, float G, float eps2, bool comp,

@@ -14,7 +14,7 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-# 32 targets per CTA (of 152 SMs) above 2,432 bodies, 64 above 7,296
+# the small-system kernel (32 targets per CTA of 152 SMs above 2,432 bodies), and above it
 @pytest.mark.parametrize("sizes", [(4000, 3000), (9728, 7400)])
 def test_small_direct_sums_of_two_sizes(nb, sizes):
     calls = 1500
