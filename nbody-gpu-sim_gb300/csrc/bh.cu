@@ -123,9 +123,8 @@ __device__ __forceinline__ void seg_box(const uint32_t* mm, int nseg, int s, BBo
   box[s] = o;
 }
 
-__global__ void seg_bounds_kernel(const float4* __restrict__ pm, SegView sv, int64_t n, int nseg,
-                                  uint32_t* __restrict__ mm, BBox* __restrict__ box,
-                                  ZeroList zero, uint32_t* err) {
+__global__ void seg_bounds_kernel(const float4* pm, SegView sv, int64_t n, int nseg,
+                                  uint32_t* mm, BBox* box, ZeroList zero, uint32_t* err) {
   chain_begin();
   __shared__ float s_red[32][6];
   __shared__ int s_same;
@@ -139,12 +138,18 @@ __global__ void seg_bounds_kernel(const float4* __restrict__ pm, SegView sv, int
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int s0 = same && nseg > 1 ? sv.seg_of[c0] : 0;
   const int64_t d0 = sv.off[s0] - sv.base[s0];
+  float4 body[4];  // (loaded ahead of the first one's atomics)
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const int64_t q = c0 + (int64_t)r * blockDim.x + threadIdx.x;
+    if (q < c1) body[r] = pm[same ? q + d0 : sv.arena((uint32_t)q)];
+  }
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
     const int64_t q = c0 + (int64_t)r * blockDim.x + threadIdx.x;
     if (q < c1) {
+      const float4 p = body[r];
       if (same) {
-        const float4 p = pm[q + d0];
         v[0] = fminf(v[0], p.x);
         v[1] = fminf(v[1], p.y);
         v[2] = fminf(v[2], p.z);
@@ -152,7 +157,6 @@ __global__ void seg_bounds_kernel(const float4* __restrict__ pm, SegView sv, int
         v[4] = fmaxf(v[4], p.y);
         v[5] = fmaxf(v[5], p.z);
       } else {
-        const float4 p = pm[sv.arena((uint32_t)q)];
         const int s = sv.seg_of[q];
         const float w[6] = {fminf(1e30f, p.x),  fminf(1e30f, p.y),  fminf(1e30f, p.z),
                             fmaxf(-1e30f, p.x), fmaxf(-1e30f, p.y), fmaxf(-1e30f, p.z)};
@@ -251,9 +255,8 @@ __device__ __forceinline__ bool tie_less(const float4& pa, uint32_t a, const flo
 // which also writes their low keys (nobody reads the low key of a body whose
 // high key differs from its neighbours').  A run already in order (e.g.
 // coincident bodies) costs one comparison per body.
-__global__ void tie_order_kernel(SegView sv, int64_t n, const int32_t* __restrict__ kseg,
-                                 const u64* __restrict__ hi, uint32_t* __restrict__ body,
-                                 u64* __restrict__ lo, float4* __restrict__ spm) {
+__global__ void tie_order_kernel(SegView sv, int64_t n, const int32_t* kseg, const u64* hi,
+                                 uint32_t* body, u64* lo, float4* spm) {
   chain_begin();
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k + 1 < n;
        k += (int64_t)gridDim.x * blockDim.x) {

@@ -313,8 +313,8 @@ __global__ void __launch_bounds__(kGWarps * 32, TWO ? 3 : 4) bh_group_walk_kerne
       f2 cm_xy = f2_make(0.f, 0.f), cm_zw = cm_xy, g_xy = cm_xy, g_zw = cm_xy;
       int4 w = make_int4((int)kWalkZero, 0, 0, 0);
       if (have) {
-        ld_node2(&a.nodes[node], cm_xy, cm_zw, g_xy, g_zw);
-        w = __ldg(&a.nodes[node].walk);
+        ld_node2_chained(&a.nodes[node], cm_xy, cm_zw, g_xy, g_zw);
+        w = a.nodes[node].walk;
       }
       float4 cm, ge;
       f2_split(cm_xy, cm.x, cm.y);

@@ -405,7 +405,7 @@ struct GroupSink {
 // 0 and 1 to the front and back of groups, 2 and 3 to those of groups2; the
 // walk takes class 0 first, so the longest groups start early and its last
 // tasks are short ones.
-__global__ void groups_kernel(const Node* __restrict__ nodes, const uint32_t* __restrict__ nstart,
+__global__ void groups_kernel(const Node* nodes, const uint32_t* nstart,
                               int64_t n, int64_t cap, GroupSink gs) {
   chain_begin();
   const uint32_t total = nstart[n];

@@ -147,12 +147,20 @@ struct GroupCounters {
 // has enough groups to fill the GPU.
 inline int bh_group_max(int64_t n) { return n >= kGroup64MinBodies ? kGroupSize : kGroupSmall; }
 
-// Centre of mass and cube of a node in one 256-bit load (read-only path),
-// as the register pairs (com x, y), (com z, mass), (centre x, y), (centre z, half).
+// Centre of mass and cube of a node in one 256-bit load, as the register pairs
+// (com x, y), (com z, mass), (centre x, y), (centre z, half): through the read-only
+// path, and for kernels of a launch chain by an ordinary load that stays behind
+// the chain's wait (chain_begin, also volatile).
 __device__ __forceinline__ void ld_node2(const Node* p, f2& cm_xy, f2& cm_zw, f2& g_xy, f2& g_zw) {
   asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];"
       : "=l"(cm_xy.v), "=l"(cm_zw.v), "=l"(g_xy.v), "=l"(g_zw.v)
       : "l"(p));
+}
+__device__ __forceinline__ void ld_node2_chained(const Node* p, f2& cm_xy, f2& cm_zw, f2& g_xy,
+                                                 f2& g_zw) {
+  asm volatile("ld.global.v4.b64 {%0, %1, %2, %3}, [%4];"
+               : "=l"(cm_xy.v), "=l"(cm_zw.v), "=l"(g_xy.v), "=l"(g_zw.v)
+               : "l"(p));
 }
 
 // Grows a buffer to hold n elements, with 1.5x headroom when it has to

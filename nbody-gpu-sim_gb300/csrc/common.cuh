@@ -55,7 +55,10 @@ inline thread_local int64_t t_launches = 0;
 // previous kernel still runs, and wait in chain_begin() until it has finished and
 // its writes are visible (programmatic dependent launch).  Every kernel of a chain
 // begins with chain_begin(), so a kernel that has finished implies that all before
-// it have.  A launch on an idle stream costs 2.1 us from one kernel's end to the
+// it have.  What earlier kernels wrote is read with ordinary loads: the read-only
+// path (__ldg, ld.global.nc, const __restrict__ parameters) is for data that stays
+// constant while a kernel runs, the wait included, and restrict pointers let the
+// compiler move loads above the wait.  A launch on an idle stream costs 2.1 us from one kernel's end to the
 // next one's start, a chained one hides most of it.
 __device__ __forceinline__ void chain_begin() {
   cudaTriggerProgrammaticLaunchCompletion();  // the next kernel's blocks may be placed

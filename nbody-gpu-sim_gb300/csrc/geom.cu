@@ -47,11 +47,9 @@ __device__ __forceinline__ void block_min_max(float (&mn)[3], float (&mx)[3], fl
 // Memory bound (16 bytes per body): four independent loads per thread and turn.
 // The last block folds the blocks' partials (one thread that folded them took
 // longer than the pass over 4M bodies) and leaves the counter zero.
-__global__ void __launch_bounds__(kBoxThreads) bbox_kernel(const float4* __restrict__ pm, int64_t n,
-                                                           float* __restrict__ part,
-                                                           uint32_t* __restrict__ counter,
-                                                           HostBox* __restrict__ out,
-                                                           uint32_t* err) {
+__global__ void __launch_bounds__(kBoxThreads) bbox_kernel(const float4* pm, int64_t n,
+                                                           float* part, uint32_t* counter,
+                                                           HostBox* out, uint32_t* err) {
   chain_begin();
   __shared__ float s[kBoxThreads / 32][6];
   __shared__ bool s_last;

@@ -78,43 +78,55 @@ __device__ __forceinline__ int32_t cell_of(float4 p, const GridArgs& g) {
 // body bound it (4M bodies 164 us; a radix sort of the cell ids, the cell starts
 // by binary search and the records took 258).  The atomics hand out the places
 // within a cell in any order, which the last kernel makes good.
-__global__ void hash_count_kernel(const float4* __restrict__ pm, int64_t n, GridArgs g,
-                                  int32_t* __restrict__ particle_cell,
-                                  uint32_t* __restrict__ count, uint32_t* __restrict__ place) {
+__global__ void hash_count_kernel(const float4* pm, int64_t n, GridArgs g, int32_t* particle_cell,
+                                  uint32_t* count, uint32_t* place) {
   chain_begin();
   const int64_t step = (int64_t)gridDim.x * blockDim.x;
   const int lane = threadIdx.x & 31;
-#pragma unroll 4
-  for (int64_t w = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x - lane); w < n; w += step) {
-    const int64_t i = w + lane;
-    const bool on = i < n;
-    const int32_t id = on ? cell_of(pm[i], g) : 0;
-    const unsigned mask = __ballot_sync(0xffffffffu, on);
-    const int32_t id0 = __shfl_sync(0xffffffffu, id, 0);
-    uint32_t at = 0;
-    if (__all_sync(0xffffffffu, !on || id == id0)) {
-      // one cell: one atomic (a whole system in one cell would queue at it)
-      if (lane == 0) at = atomicAdd(&count[id], (uint32_t)__popc(mask));
-      at = __shfl_sync(0xffffffffu, at, 0) + lane;
-    } else if (on) {
-      at = atomicAdd(&count[id], 1u);
-    }
-    if (on) {
-      particle_cell[i] = id;
-      place[i] = at;
+  // (four bodies' loads ahead of the first one's stores)
+  for (int64_t w0 = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x - lane); w0 < n; w0 += 4 * step) {
+    float4 p[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+      if (w0 + r * step + lane < n) p[r] = pm[w0 + r * step + lane];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int64_t i = w0 + r * step + lane;
+      const bool on = i < n;
+      const int32_t id = on ? cell_of(p[r], g) : 0;
+      const unsigned mask = __ballot_sync(0xffffffffu, on);
+      if (!mask) break;
+      const int32_t id0 = __shfl_sync(0xffffffffu, id, 0);
+      uint32_t at = 0;
+      if (__all_sync(0xffffffffu, !on || id == id0)) {
+        // one cell: one atomic (a whole system in one cell would queue at it)
+        if (lane == 0) at = atomicAdd(&count[id], (uint32_t)__popc(mask));
+        at = __shfl_sync(0xffffffffu, at, 0) + lane;
+      } else if (on) {
+        at = atomicAdd(&count[id], 1u);
+      }
+      if (on) {
+        particle_cell[i] = id;
+        place[i] = at;
+      }
     }
   }
 }
 
-__global__ void hash_place_kernel(const int32_t* __restrict__ particle_cell,
-                                  const uint32_t* __restrict__ place,
-                                  const uint32_t* __restrict__ start, int64_t n,
-                                  uint32_t* __restrict__ idx) {
+__global__ void hash_place_kernel(const int32_t* particle_cell, const uint32_t* place,
+                                  const uint32_t* start, int64_t n, uint32_t* idx) {
   chain_begin();
   const int64_t step = (int64_t)gridDim.x * blockDim.x;
-#pragma unroll 4
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += step) {
-    idx[start[particle_cell[i]] + place[i]] = (uint32_t)i;
+  for (int64_t i0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i0 < n; i0 += 4 * step) {
+    uint32_t at[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int64_t i = i0 + r * step;
+      if (i < n) at[r] = start[particle_cell[i]] + place[i];
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+      if (i0 + r * step < n) idx[at[r]] = (uint32_t)(i0 + r * step);
   }
 }
 
@@ -137,10 +149,8 @@ constexpr float kFarAway = 3.0e38f;  // (bodies are within 1e30, where the box's
 constexpr int kHashCrowd = 256;  // threads (and slots) per block, too
 
 __global__ void __launch_bounds__(kHashCrowd) hash_order_kernel(
-    const float4* __restrict__ pm, int64_t n, GridArgs g, int64_t total,
-    const uint32_t* __restrict__ placed,
-    const uint32_t* __restrict__ count, const uint32_t* __restrict__ start,
-    uint32_t* __restrict__ cells, uint32_t* __restrict__ idx, float* __restrict__ out) {
+    const float4* pm, int64_t n, GridArgs g, int64_t total, const uint32_t* placed,
+    const uint32_t* count, const uint32_t* start, uint32_t* cells, uint32_t* idx, float* out) {
   chain_begin();
   __shared__ uint32_t s_idx[kHashCrowd], s_sorted[kHashCrowd];
   __shared__ uint32_t s_hist[2][kHashCrowd + 1];
@@ -244,10 +254,9 @@ __global__ void __launch_bounds__(kHashCrowd) hash_order_kernel(
 // row of the warp (of 8 cells with 24 candidates per row on average).
 template <bool COUNT, int SUB, int T, bool ROWS>
 __global__ void __launch_bounds__(SUB * T) hash_force_kernel(
-    const float4* __restrict__ pairs, const uint32_t* __restrict__ cells,
-    const uint32_t* __restrict__ idx, const uint32_t* __restrict__ start, int64_t total, GridArgs g,
-    float cut2, float eps2, float G, float* __restrict__ ax, float* __restrict__ ay,
-    float* __restrict__ az, int32_t* __restrict__ counts) {
+    const float4* pairs, const uint32_t* cells, const uint32_t* idx, const uint32_t* start,
+    int64_t total, GridArgs g, float cut2, float eps2, float G, float* ax, float* ay, float* az,
+    int32_t* counts) {
   chain_begin();
   __shared__ uint2 s_row[9][T];  // records of each neighbour row
   const int t = threadIdx.x % T, sub = threadIdx.x / T;  // pair of the block, its thread
@@ -287,7 +296,7 @@ __global__ void __launch_bounds__(SUB * T) hash_force_kernel(
   }
   auto add = [&](uint32_t j) {
     const ulonglong2* rec = reinterpret_cast<const ulonglong2*>(pairs) + 2 * (uint64_t)j;
-    const ulonglong2 xy = __ldg(rec), zm = __ldg(rec + 1);
+    const ulonglong2 xy = rec[0], zm = rec[1];
     const bool other = j != me;
 #pragma unroll
     for (int q = 0; q < 2; ++q) {

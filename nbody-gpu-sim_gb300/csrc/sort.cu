@@ -37,8 +37,7 @@ __device__ __forceinline__ uint32_t scan_in(uint32_t v) {
 }
 
 template <bool EVEN>
-__global__ void scan_reduce_kernel(const uint32_t* __restrict__ in, int64_t n,
-                                   uint32_t* __restrict__ block_sums) {
+__global__ void scan_reduce_kernel(const uint32_t* in, int64_t n, uint32_t* block_sums) {
   chain_begin();
   __shared__ uint32_t s[kScanThreads / 32];
   const int64_t base = (int64_t)blockIdx.x * kScanChunk;
@@ -60,7 +59,7 @@ __global__ void scan_reduce_kernel(const uint32_t* __restrict__ in, int64_t n,
 // Exclusive scan of `n` values by one block (n up to a few hundred thousand).
 template <bool EVEN>
 __global__ void scan_single_block_kernel(const uint32_t* in, uint32_t* data, int64_t n,
-                                         uint32_t* __restrict__ total) {
+                                         uint32_t* total) {
   chain_begin();
   __shared__ uint32_t s_carry;
   __shared__ uint32_t s_warp[32];
@@ -97,9 +96,9 @@ __global__ void scan_single_block_kernel(const uint32_t* in, uint32_t* data, int
 }
 
 template <bool EVEN>
-__global__ void scan_apply_kernel(const uint32_t* __restrict__ in, int64_t n,
-                                  const uint32_t* __restrict__ block_offsets,
-                                  uint32_t* __restrict__ out) {
+__global__ void scan_apply_kernel(const uint32_t* in, int64_t n,
+                                  const uint32_t* block_offsets,
+                                  uint32_t* out) {
   chain_begin();
   __shared__ uint32_t s_vals[kScanChunk];
   __shared__ uint32_t s_warp[kScanThreads / 32];
