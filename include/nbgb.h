@@ -528,6 +528,13 @@ nbgb_status nbgb_selftest_fail_allocation(int32_t nth);
  * next synchronization instead of returning forces.  Process-wide. */
 nbgb_status nbgb_selftest_group_walk_stack(int32_t entries);
 
+/* Test hook for the small-system steps of nbgb_system_step: cooperative
+ * launches of more than `ctas` CTAs are refused (0: none are), as the driver
+ * refuses them where a process has fewer SMs than the device reports.  The call
+ * then takes its steps one at a time, with the same results bit for bit.
+ * Process-wide; nothing reaches the GPU. */
+nbgb_status nbgb_selftest_cooperative_limit(int32_t ctas);
+
 /* Test hook for nbgb_compute_forces_direct_noalloc: the j-split count the
  * regular direct planner picks for `count` bodies on the current device
  * (*planned_splits) and the count the allocation-free entry point uses after

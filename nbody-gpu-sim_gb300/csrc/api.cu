@@ -297,7 +297,9 @@ static bool system_in_one_launch(const nbgb_system* s) {
   return !s->fp64 && s->calc->method == NBGB_DIRECT_N2 && direct_small_fit(s->n);
 }
 
-static void system_small_steps(nbgb_system* s, int32_t steps, double kick0, double h) {
+// False: the launch was refused and nothing has changed (never with steps = 0,
+// which is an ordinary launch).
+static bool system_small_steps(nbgb_system* s, int32_t steps, double kick0, double h) {
   nbgb_calculator* c = s->calc;
   const float eps = c->params.softening;
   const StateArrays a{s->x.ptr,  s->y.ptr,  s->z.ptr,  s->vx.ptr, s->vy.ptr,
@@ -308,10 +310,11 @@ static void system_small_steps(nbgb_system* s, int32_t steps, double kick0, doub
   StageTimer* t = stage_timer(c);
   if (t) t->st = c->stream;
   stage_mark(t, "direct.forces");
-  launch_direct_steps(a, s->n, steps, kick0, h, h, eps * eps, c->params.G,
-                      (c->params.flags & NBGB_FLAG_COMPENSATED) != 0, ex, s->exch_ctr.ptr,
-                      c->err.ensure(1), c->stream);
+  const bool ok = launch_direct_steps(a, s->n, steps, kick0, h, h, eps * eps, c->params.G,
+                                      (c->params.flags & NBGB_FLAG_COMPENSATED) != 0, ex,
+                                      s->exch_ctr.ptr, c->err.ensure(1), c->stream);
   if (t) t->end();
+  return ok;
 }
 
 // Forces at the current state into the system's acceleration arrays.
@@ -698,7 +701,9 @@ nbgb_status nbgb_system_step(nbgb_system* s, float dt, int32_t steps) {
       const int32_t most = stage_timer(c) ? 1 : kDirectStepsPerLaunch;
       while (k < steps) {
         const int32_t m = std::min(steps - k, most);
-        system_small_steps(s, m, s->pending_half ? 0.5 * s->last_dt + 0.5 * h : 0.5 * h, h);
+        // (refused: the rest one step at a time below, with the same sums)
+        if (!system_small_steps(s, m, s->pending_half ? 0.5 * s->last_dt + 0.5 * h : 0.5 * h, h))
+          break;
         s->pending_half = true;
         s->last_dt = h;
         k += m;

@@ -65,7 +65,8 @@ void launch_pack_soa(const float* x, const float* y, const float* z, const float
                      int64_t n_pad, float4* out, cudaStream_t st);
 
 // Small systems (steps.cu): the forces of n bodies, or `steps` kick-drift +
-// force steps in one cooperative launch.  exch: 2 n entries; ctr: two
+// force steps in one cooperative launch (false: refused, its CTAs cannot all be
+// resident; nothing has been launched).  exch: 2 n entries; ctr: two
 // counters, zero before and after.
 constexpr int64_t kDirectSmallMaxBodies = 4864;  // 16 bytes per body in shared memory
 constexpr int32_t kDirectStepsPerLaunch = 256;   // bounds one launch's time
@@ -77,9 +78,10 @@ struct StateArrays {
 bool direct_small_fit(int64_t n);
 void launch_direct_small(const DirectSource& src, int64_t n, float G, float eps2, bool comp,
                          float* ox, float* oy, float* oz, cudaStream_t st);
-void launch_direct_steps(const StateArrays& s, int64_t n, int32_t steps, double kick0, double kick,
+bool launch_direct_steps(const StateArrays& s, int64_t n, int32_t steps, double kick0, double kick,
                          double dt, float eps2, float G, bool comp, float4* exch, uint32_t* ctr,
                          uint32_t* err, cudaStream_t st);
+void direct_set_cooperative_limit(int ctas);  // test hook: CTAs of a launch (0: no limit)
 
 // Energies: `partials` needs nblocks * 4 doubles; out[0..3] = KE, Px, Py, Pz
 // (kinetic) or out[0] = sum_i m_i phi_i / 2 without G (potential).

@@ -65,3 +65,10 @@ extern "C" nbgb_status nbgb_selftest_group_walk_stack(int32_t entries) {
   bh_set_group_stack_limit(entries);
   return NBGB_OK;
 }
+
+extern "C" nbgb_status nbgb_selftest_cooperative_limit(int32_t ctas) {
+  if (ctas < 0)
+    return set_error(NBGB_ERR_INVALID_ARG, "Validation Error: the CTA limit must be >= 0");
+  direct_set_cooperative_limit(ctas);
+  return set_error(NBGB_OK, std::string());
+}

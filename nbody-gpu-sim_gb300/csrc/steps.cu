@@ -18,6 +18,8 @@
 // Force calculators and a system's a(0) run the same kernel (steps = 0, an
 // ordinary launch), so a trajectory does not depend on how its steps are
 // grouped into calls, and the forces of a system are a calculator's, bitwise.
+#include <atomic>
+
 #include "common.cuh"
 #include "direct_pair.cuh"
 #include "kernels.cuh"
@@ -178,8 +180,14 @@ __global__ void __launch_bounds__(kStepThreads, 1) direct_steps_kernel(StepArgs 
   }
 }
 
+// Cooperative launches of more CTAs than this are refused (0: none; test hook).
+static std::atomic<int> g_cooperative_limit{0};
+void direct_set_cooperative_limit(int ctas) { g_cooperative_limit.store(ctas); }
+
+// False: the CTAs cannot all be resident (a share of the GPU with fewer SMs than
+// the device reports), and nothing was launched.
 template <int TL, bool COMP, bool ZS>
-static void launch_steps_t(StepArgs& a, cudaStream_t st) {
+static bool launch_steps_t(StepArgs& a, cudaStream_t st) {
   const size_t smem = (size_t)((a.n + 3) & ~3) * 16;
   auto kern = direct_steps_kernel<TL, COMP, ZS>;
   // (one limit for all sizes: the attribute is the kernel's, and a smaller one set for a
@@ -189,21 +197,29 @@ static void launch_steps_t(StepArgs& a, cudaStream_t st) {
   const unsigned grid = (unsigned)ceil_div(a.n, TL);
   if (a.steps) {
     void* args[] = {&a};
-    NBGB_CUDA(cudaLaunchCooperativeKernel((const void*)kern, dim3(grid), dim3(kStepThreads), args,
-                                          smem, st));
+    const int limit = g_cooperative_limit.load(std::memory_order_relaxed);
+    const cudaError_t e = limit > 0 && grid > (unsigned)limit
+                              ? cudaErrorCooperativeLaunchTooLarge
+                              : cudaLaunchCooperativeKernel((const void*)kern, dim3(grid),
+                                                            dim3(kStepThreads), args, smem, st);
+    if (e == cudaErrorCooperativeLaunchTooLarge) {
+      cudaGetLastError();
+      return false;
+    }
+    NBGB_CUDA(e);
   } else {  // forces only: the CTAs do not wait on one another
     kern<<<grid, kStepThreads, smem, st>>>(a);
   }
   NBGB_LAUNCH_CHECK();
+  return true;
 }
 
 template <int TL>
-static void launch_steps_n(StepArgs& a, bool comp, cudaStream_t st) {
+static bool launch_steps_n(StepArgs& a, bool comp, cudaStream_t st) {
   const bool zs = !(a.eps2 > 0.f);
   if (zs)
-    comp ? launch_steps_t<TL, true, true>(a, st) : launch_steps_t<TL, false, true>(a, st);
-  else
-    comp ? launch_steps_t<TL, true, false>(a, st) : launch_steps_t<TL, false, false>(a, st);
+    return comp ? launch_steps_t<TL, true, true>(a, st) : launch_steps_t<TL, false, true>(a, st);
+  return comp ? launch_steps_t<TL, true, false>(a, st) : launch_steps_t<TL, false, false>(a, st);
 }
 
 // Sizes for this kernel: up to 32 targets per CTA on at most one CTA per SM.
@@ -217,14 +233,11 @@ bool direct_small_fit(int64_t n) {
   return n <= std::min<int64_t>(32 * num_sms(), kDirectSmallMaxBodies);
 }
 
-static void launch_small(StepArgs& a, bool comp, cudaStream_t st) {
+static bool launch_small(StepArgs& a, bool comp, cudaStream_t st) {
   const int64_t sms = num_sms();
-  if (a.n <= 8 * sms)
-    launch_steps_n<8>(a, comp, st);
-  else if (a.n <= 16 * sms)
-    launch_steps_n<16>(a, comp, st);
-  else
-    launch_steps_n<32>(a, comp, st);
+  if (a.n <= 8 * sms) return launch_steps_n<8>(a, comp, st);
+  if (a.n <= 16 * sms) return launch_steps_n<16>(a, comp, st);
+  return launch_steps_n<32>(a, comp, st);
 }
 
 void launch_direct_small(const DirectSource& src, int64_t n, float G, float eps2, bool comp,
@@ -244,7 +257,7 @@ void launch_direct_small(const DirectSource& src, int64_t n, float G, float eps2
   launch_small(a, comp, st);
 }
 
-void launch_direct_steps(const StateArrays& s, int64_t n, int32_t steps, double kick0, double kick,
+bool launch_direct_steps(const StateArrays& s, int64_t n, int32_t steps, double kick0, double kick,
                          double dt, float eps2, float G, bool comp, float4* exch, uint32_t* ctr,
                          uint32_t* err, cudaStream_t st) {
   StepArgs a{};
@@ -268,7 +281,7 @@ void launch_direct_steps(const StateArrays& s, int64_t n, int32_t steps, double 
   a.G = G;
   a.steps = steps;
   a.kick0 = kick0;
-  launch_small(a, comp, st);
+  return launch_small(a, comp, st);
 }
 
 }  // namespace nbgb
