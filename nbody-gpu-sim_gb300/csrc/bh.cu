@@ -558,7 +558,8 @@ BHState* bh_state_new() { return new BHState(); }
 
 size_t bh_segment_table_bytes(const int64_t* n_per, int nseg) {
   int64_t ntask = 0;
-  for (int s = 0; s < nseg; ++s) ntask += ceil_div(n_per[s], bh_walk_targets(n_per[s]));
+  for (int s = 0; s < nseg; ++s)
+    ntask += ceil_div(n_per[s], bh_walk_targets(bh_walk_class(n_per[s])));
   return ((size_t)nseg * 2 + 1) * sizeof(int64_t) + (size_t)ntask * sizeof(WarpTask) +
          ((size_t)nseg + 1) * sizeof(int32_t);
 }
@@ -584,14 +585,15 @@ void bh_set_segments(BHState& h, const int64_t* off, const int64_t* n_per, int n
     hbase[s] = n;
     n += n_per[s];
   }
-  // the walk's tasks, those of 32 targets first
-  for (const int tw : {32, 16}) {
+  // the walk's tasks by size class
+  for (int cls = 0; cls < kWalkClasses; ++cls) {
+    const int tw = bh_walk_targets(cls);
     for (int s = 0; s < nseg; ++s) {
-      if (bh_walk_targets(n_per[s]) != tw) continue;
+      if (bh_walk_class(n_per[s]) != cls) continue;
       const int64_t end = hbase[s] + n_per[s];
       for (int64_t f = hbase[s]; f < end; f += tw) ht[t++] = WarpTask{f, end, s, 0};
     }
-    if (tw == 32) h.ntasks32 = t;
+    if (cls < kWalkClasses - 1) h.ntasks_upto[cls] = t;
   }
   h.sort_buckets = path_sort_buckets(n_per, nseg, reinterpret_cast<int32_t*>(ht + t));
   hbase[nseg] = n;
@@ -636,9 +638,9 @@ void bh_build(BHState& h, const float4* pm, cudaStream_t st, uint32_t* err, bool
       {reinterpret_cast<uint32_t*>(grow(h.psort_ws, path_sort_ws_bytes())),
        reinterpret_cast<uint32_t*>(grow(h.seg_depth, (size_t)nseg + 2)),
        reinterpret_cast<uint32_t*>(grow(h.group_ctr, sizeof(GroupCounters))),
-       grow(h.walk_ctr, 2)},
+       grow(h.walk_ctr, kWalkLaunches)},
       {h.sort_buckets > 0 ? (uint32_t)path_sort_zero_words() : 0u, (uint32_t)nseg + 2,
-       (uint32_t)(sizeof(GroupCounters) / sizeof(uint32_t)), 2}};
+       (uint32_t)(sizeof(GroupCounters) / sizeof(uint32_t)), (uint32_t)kWalkLaunches}};
   launch_chained(seg_bounds_kernel, (unsigned)ceil_div(n, 1024), 256, 0, st, pm, sv, n, nseg, mm,
                  h.box.ptr, zero, err);
   // 2. keys and order
@@ -792,7 +794,7 @@ void bh_reserve_buffers(BHState& h, bool groups) {
   grow(h.leaf_of, R);
   grow(h.seg_root, (size_t)nseg);
   grow(h.seg_end, (size_t)nseg);
-  grow(h.walk_ctr, 2);
+  grow(h.walk_ctr, kWalkLaunches);
   grow(h.group_ctr, sizeof(GroupCounters));  // (cleared by the bounds kernel with either walk)
   if (groups) {
     grow(h.groups, R);

@@ -10,7 +10,7 @@ struct BHState;
 struct StageTimer;
 
 // Consecutive path-sorted targets of one segment (bh_walk_targets of its
-// size), walked by one warp.
+// class), walked by one warp.
 struct WarpTask {
   int64_t first;  // first sorted position
   int64_t end;    // one past the segment's last sorted position
@@ -28,8 +28,12 @@ struct BHWalkParams {
                       // leaf_capacity bodies list their bodies)
 };
 
-constexpr int64_t kWalk32MinBodies = 32768;
-int bh_walk_targets(int64_t n);
+// Size classes of the reference walk (bh_walk.cu): 0 and 1 the sizes that short
+// walks take in another way, 2 the others with 32 targets per warp, 3 with 16.
+constexpr int kWalkClasses = 4;
+constexpr int kWalkLaunches = 3;  // at most: short walks, 32 targets per warp, 16
+int bh_walk_class(int64_t n);
+constexpr int bh_walk_targets(int cls) { return cls == kWalkClasses - 1 ? 16 : 32; }
 
 BHState* bh_state_new();
 void bh_state_delete(BHState* p);

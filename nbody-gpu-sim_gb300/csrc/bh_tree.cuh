@@ -64,7 +64,9 @@ struct BHState {
   HostPinned<char> h_tables;
   int32_t nseg = 0;
   int64_t ntasks = 0;
-  int64_t ntasks32 = 0;  // the first tasks, of 32 targets; the others have 16
+  // the first tasks: of the largest, of large and of all systems whose tasks have 32
+  // targets (bh_walk_class); the others have 16
+  int64_t ntasks_upto[kWalkClasses - 1] = {0, 0, 0};
   // keys and order
   DevBuf<uint32_t> mkeys, mkeys_alt, midx, midx_alt;  // on-demand Morton sort
   DevBuf<u64> klo, khi, khi_alt;
@@ -83,7 +85,7 @@ struct BHState {
   DevBuf<char> ref_nodes;   // reference-identical build: the reference's node array
   DevBuf<int32_t> ref_pos;  // reference-identical build: original index -> sorted position
   DevBuf<float4> spm;      // bodies in path order
-  DevBuf<uint32_t> walk_ctr;  // next warp task of the walk (32 and 16 targets)
+  DevBuf<uint32_t> walk_ctr;  // next warp task of each launch of the walk
   DevBuf<int4> groups;        // group walk: first body, count, segment; cost classes 0 / 1
                               // from the front / back of groups, 2 / 3 of groups2
   DevBuf<int4> groups2;

@@ -33,9 +33,10 @@ struct WalkArgs {
   const uint32_t* body;
   const uint32_t* nstart;
   SegView sv;
-  const WarpTask* tasks;  // 32 consecutive targets each
+  const WarpTask* tasks;  // up to 32 consecutive targets each
   int64_t ntasks;
   const int32_t* seg_root;
+  const int32_t* seg_end;
   int64_t n;
   int64_t cap;
   float theta2;
@@ -575,37 +576,169 @@ __global__ void __launch_bounds__(kWWarps * 32, 3) bh_walk_kernel(WalkArgs a) {
   }
 }
 
-template <bool COUNT, bool BUCKET, int TW>
-static void launch_walk_t(WalkArgs w, const WarpTask* tasks, int64_t ntasks, uint32_t* ctr,
-                          cudaStream_t st) {
-  if (ntasks <= 0) return;
-  w.tasks = tasks;
-  w.ntasks = ntasks;
-  w.task_ctr = ctr;
-  constexpr size_t smem = sizeof(WalkShared) * kWWarps;
-  auto kern = bh_walk_kernel<COUNT, BUCKET, TW>;
-  NBGB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  static const int occ = [&] {
-    int b = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kern, kWWarps * 32, smem);
-    return std::max(b, 1);
-  }();
-  // one resident wave of persistent warps
+// Short walks of large systems (launch_walk has the line): the union of 32 targets'
+// paths node by node, all lanes on one node, each with its own target.  No stack,
+// no lists and no shared memory, so 48 to 64 warps per SM cover each other's loads;
+// a visited node costs 40 instructions whatever the targets decide, which is why long
+// walks take half as many the other way.  A short one is bound by the chain of that
+// way's steps (first child and next sibling, seven levels of up to eight): 1M bodies in
+// a cube at theta 1.5 257 us here, 563 there; at theta 0.5 2,922 and 1,958.
+template <bool COUNT, bool BUCKET>
+__global__ void __launch_bounds__(256, BUCKET ? 6 : (COUNT ? 7 : 8))
+    bh_union_walk_kernel(WalkArgs a) {
+  const uint32_t total = a.nstart[a.n];
+  const bool tree_ok = (int64_t)total <= a.cap;
+  const int lane = threadIdx.x & 31;
+  while (true) {
+    uint32_t t32 = 0;
+    if (lane == 0) t32 = atomicAdd(a.task_ctr, 1u);
+    t32 = __shfl_sync(0xffffffffu, t32, 0);
+    if ((int64_t)t32 >= a.ntasks) break;
+    const WarpTask task = a.tasks[t32];
+    const int64_t k = task.first + lane;
+    const bool valid = k < task.end;
+    const float4 pi = valid ? a.spm[k] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const f2 pi_xy = f2_make(pi.x, pi.y);
+    float sx = 0.f, sy = 0.f, sz = 0.f;
+    int cnt = 0;
+    int resume = valid ? 0 : 0x7fffffff;
+    int node = tree_ok ? a.seg_root[task.seg] : 0;
+    const int node_end = tree_ok ? a.seg_end[task.seg] : 0;
+    while (node < node_end) {
+      f2 cm_xy, cm_zw, g_xy, g_zw;
+      ld_node2(&a.nodes[node], cm_xy, cm_zw, g_xy, g_zw);
+      float4 cm, g;
+      f2_split(cm_xy, cm.x, cm.y);
+      f2_split(cm_zw, cm.z, cm.w);
+      f2_split(g_xy, g.x, g.y);
+      f2_split(g_zw, g.z, g.w);
+      float tx, ty;  // target minus cube centre
+      f2_split(f2_sub(pi_xy, g_xy), tx, ty);
+      int4 w;  // the body range is for buckets alone
+      if (BUCKET) {
+        w = __ldg(&a.nodes[node].walk);
+      } else {
+        const int2 w2 = __ldg(reinterpret_cast<const int2*>(&a.nodes[node].walk));
+        w = make_int4(w2.x, w2.y, 0, 0);
+      }
+      const int skip = w.x & (int)(kWalkZero - 1u);
+      if ((uint32_t)w.x >= kWalkZero) {  // a leaf, or without mass
+        if ((uint32_t)w.x & kWalkZero) {  // force_barnes_hut.cu:172-173
+          node = skip;
+          continue;
+        }
+        if (node >= resume) {  // force_barnes_hut.cu:185-203
+          float me = cm.w, cx = cm.x, cy = cm.y, cz = cm.z;
+          bool use = true;
+          if (fabsf(tx) <= g.w && fabsf(ty) <= g.w && fabsf(__fsub_rn(pi.z, g.z)) <= g.w) {
+            me = __fsub_rn(cm.w, pi.w);  // the leaf without the target
+            use = me > 0.0f;
+            if (use) {
+              cx = __fdiv_rn(__fsub_rn(__fmul_rn(cm.x, cm.w), __fmul_rn(pi.x, pi.w)), me);
+              cy = __fdiv_rn(__fsub_rn(__fmul_rn(cm.y, cm.w), __fmul_rn(pi.y, pi.w)), me);
+              cz = __fdiv_rn(__fsub_rn(__fmul_rn(cm.z, cm.w), __fmul_rn(pi.z, pi.w)), me);
+            }
+          }
+          if (use) {
+            bh_add(cx, cy, cz, me, pi.x, pi.y, pi.z, a.eps2, sx, sy, sz);
+            if (COUNT) ++cnt;
+          }
+        }
+        node = skip;
+        continue;
+      }
+      // internal node (force_barnes_hut.cu:205-243)
+      const bool active = node >= resume;
+      const bool contains =
+          fabsf(tx) <= g.w && fabsf(ty) <= g.w && fabsf(__fsub_rn(pi.z, g.z)) <= g.w;
+      float dx, dy;
+      f2_split(f2_sub(cm_xy, pi_xy), dx, dy);
+      const float dz = __fsub_rn(cm.z, pi.z);
+      const float d2 = __fadd_rn(__fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx))), a.eps2);
+      const bool accept =
+          !contains && opening_accept(__int_as_float(w.y), d2, a.th_lo, a.th_hi, a.theta2);
+      const bool open = active && !accept;
+      if (active && accept) {
+        const float r = rsqrt_approx(d2);
+        const float f = (cm.w * r) * (r * r);
+        sx = fmaf(f, dx, sx);
+        sy = fmaf(f, dy, sy);
+        sz = fmaf(f, dz, sz);
+        if (COUNT) ++cnt;
+        resume = skip;
+      }
+      if (BUCKET && (int)((uint32_t)w.w & ~kWalkNext) <= a.leaf_cap) {
+        // the targets that open a bucket sum its bodies (one broadcast load each)
+        if (open) {
+          const int64_t self = k - w.z;
+          const int nb = (int)((uint32_t)w.w & ~kWalkNext);
+          for (int j = 0; j < nb; ++j) {
+            const float4 q = __ldg(&a.spm[w.z + j]);
+            if (j != self) {
+              bh_add(q.x, q.y, q.z, q.w, pi.x, pi.y, pi.z, a.eps2, sx, sy, sz);
+              if (COUNT) ++cnt;
+            }
+          }
+        }
+        node = skip;
+        continue;
+      }
+      node = __any_sync(0xffffffffu, open) ? node + 1 : skip;
+    }
+    if (valid) {
+      const int64_t i = a.sv.arena(a.body[k]);
+      a.ax[i] = a.G * sx;
+      a.ay[i] = a.G * sy;
+      a.az[i] = a.G * sz;
+      if (COUNT && a.counts) a.counts[i] = cnt;
+    }
+    if (COUNT && a.inter_total) {
+      unsigned long long c = valid ? (unsigned long long)cnt : 0ull;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) c += __shfl_down_sync(0xffffffffu, c, o);
+      if (lane == 0) atomicAdd(a.inter_total, c);
+    }
+  }
+}
+
+// One resident wave of persistent warps on some of the tasks.
+// (Not chained: blocks placed beside the build's last ones share SMs while others
+// stay empty, forces at 20 K bodies 355 us instead of 293.)
+template <typename K>
+static void launch_tasks(K kern, int occ, size_t smem, WalkArgs w, const BHState& h, int64_t first,
+                         int64_t last, int launch, cudaStream_t st) {
+  w.tasks = h.tasks_p + first;
+  w.ntasks = last - first;
+  w.task_ctr = h.walk_ctr.ptr + launch;
+  if (w.ntasks <= 0) return;
   const int64_t blocks = std::max<int64_t>(
-      1, std::min<int64_t>(ceil_div(ntasks, kWWarps), (int64_t)num_sms() * occ));
-  // (not chained: blocks placed beside the build's last ones share SMs while others
-  // stay empty, forces at 20 K bodies 355 us instead of 293)
+      1, std::min<int64_t>(ceil_div(w.ntasks, kWWarps), (int64_t)num_sms() * occ));
   kern<<<(unsigned)blocks, kWWarps * 32, smem, st>>>(w);
   NBGB_LAUNCH_CHECK();
 }
 
-// The tasks of 32 targets come first in the table, then those of 16.
-template <bool COUNT, bool BUCKET>
-static void launch_walk(const BHState& h, const WalkArgs& w, cudaStream_t st) {
-  launch_walk_t<COUNT, BUCKET, 32>(w, h.tasks_p, h.ntasks32, h.walk_ctr.ptr, st);
-  launch_walk_t<COUNT, BUCKET, 16>(w, h.tasks_p + h.ntasks32, h.ntasks - h.ntasks32,
-                                   h.walk_ctr.ptr + 1, st);
+template <typename K>
+static int walk_occupancy(K kern, size_t smem) {
+  int b = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kern, kWWarps * 32, smem);
+  return std::max(b, 1);
 }
+
+template <bool COUNT, bool BUCKET, int TW>
+static void launch_walk_t(const WalkArgs& w, const BHState& h, int64_t first, int64_t last,
+                          int launch, cudaStream_t st) {
+  constexpr size_t smem = sizeof(WalkShared) * kWWarps;
+  auto kern = bh_walk_kernel<COUNT, BUCKET, TW>;
+  NBGB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  static const int occ = walk_occupancy(kern, smem);
+  launch_tasks(kern, occ, smem, w, h, first, last, launch, st);
+}
+
+// Sizes from which a short walk goes node by node, and from which it does so at a
+// smaller theta.
+constexpr int64_t kWalkUnionMin = 196608;
+constexpr int64_t kWalkUnionLarge = 1310720;
+constexpr int64_t kWalk32MinBodies = 32768;
 
 // Targets per warp for a system of n bodies: 16 give twice as many, shorter
 // warps with smaller boxes, which pays while one system alone leaves SMs idle;
@@ -614,7 +747,33 @@ static void launch_walk(const BHState& h, const WalkArgs& w, cudaStream_t st) {
 // system alone (about 60,000 bodies) because many systems walked together fill
 // the GPU.  Walk of one system, us (16 / 32 targets): N = 20 K 202 / 261, 50 K
 // 299 / 350, 100 K 485 / 441, 1M 4,555 / 3,472.
-int bh_walk_targets(int64_t n) { return n < kWalk32MinBodies ? 16 : 32; }
+int bh_walk_class(int64_t n) {
+  return n > kWalkUnionLarge ? 0 : n >= kWalkUnionMin ? 1 : n >= kWalk32MinBodies ? 2 : 3;
+}
+
+// The walk's time, us, 32 nodes per step / node by node (Plummer sphere; cube):
+//   200 K  theta 1.0   290 / 382;   194 / 206    leaf 16  391 / 380;   222 / 190
+//          theta 1.25  242 / 250;   163 / 128    leaf 16  303 / 261;   178 / 120
+//   1M     theta 1.0  1274 / 1481;  744 / 615    leaf 16 1648 / 1555;  789 / 647
+//          theta 1.25 1070 / 955;   629 / 372
+//   2M     theta 0.75 3273 / 5036; 1935 / 2081;  theta 1.0 2389 / 2913; 1407 / 1099
+//   100 K  theta 1.25  143 / 202;   102 / 115
+// Which way is shorter depends on the bodies, too (in a cube the lists are shorter than in
+// a sphere): the lines keep the loss against the shorter way below a quarter on both
+// sides.  A system's own size and the parameters decide, as above.
+template <bool COUNT, bool BUCKET>
+static void launch_walk(const BHState& h, const WalkArgs& w, float theta, cudaStream_t st) {
+  const int64_t t32 = h.ntasks_upto[2];
+  int64_t t = 0;
+  if (theta > 0.875f) t = theta > 1.125f || w.leaf_cap > 8 ? h.ntasks_upto[1] : h.ntasks_upto[0];
+  if (t > 0) {
+    auto kern = bh_union_walk_kernel<COUNT, BUCKET>;
+    static const int occ = walk_occupancy(kern, 0);
+    launch_tasks(kern, occ, 0, w, h, 0, t, 0, st);
+  }
+  launch_walk_t<COUNT, BUCKET, 32>(w, h, t, t32, 1, st);
+  launch_walk_t<COUNT, BUCKET, 16>(w, h, t32, h.ntasks, 2, st);
+}
 
 void bh_reference_walk(BHState& h, const BHWalkParams& p, float* ax, float* ay, float* az,
                        int32_t* counts, unsigned long long* inter_total, cudaStream_t st) {
@@ -625,6 +784,7 @@ void bh_reference_walk(BHState& h, const BHWalkParams& p, float* ax, float* ay, 
   w.nstart = h.nstart.ptr;
   w.sv = SegView{h.seg_off_p, h.seg_base_p, h.seg_of.ptr, h.box.ptr};
   w.seg_root = h.seg_root.ptr;
+  w.seg_end = h.seg_end.ptr;
   w.n = h.n;
   w.cap = h.cap;
   w.theta2 = p.theta * p.theta;
@@ -645,14 +805,14 @@ void bh_reference_walk(BHState& h, const BHWalkParams& p, float* ax, float* ay, 
   const bool bucket = p.leaf_capacity > 1;
   if (count) {
     if (bucket)
-      launch_walk<true, true>(h, w, st);
+      launch_walk<true, true>(h, w, p.theta, st);
     else
-      launch_walk<true, false>(h, w, st);
+      launch_walk<true, false>(h, w, p.theta, st);
   } else {
     if (bucket)
-      launch_walk<false, true>(h, w, st);
+      launch_walk<false, true>(h, w, p.theta, st);
     else
-      launch_walk<false, false>(h, w, st);
+      launch_walk<false, false>(h, w, p.theta, st);
   }
 }
 
