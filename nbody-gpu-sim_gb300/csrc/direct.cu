@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(kDirThreads, 2) direct_kernel(DirectArgs a) {
 // long inner loop without block barriers sustains up to 2 % more than the kernel
 // above (350,000 bodies 44.0 against 44.5 ms, 1M 391.5 against 401), but its blocks of
 // 1,024 targets and whole tiles split unevenly below (65,536 bodies 1.65 against
-// 1.58 ms, 131,072 6.38 against 6.30, 262,144 24.99 against 24.92).
+// 1.58 ms, 131,072 6.38 against 6.30; plan_direct has the line).
 template <bool COMP, bool ZERO_SOFT>
 __global__ void __launch_bounds__(kDirHalf) direct_ring_kernel(DirectArgs a) {
   constexpr int I = 8;
@@ -257,8 +257,50 @@ __global__ void direct_runs_kernel(DirectArgs a) {
 // 15 runs; 42 with one target, unsplit), N = 16,384 107 (two, 19 runs; 130
 // with one target, unsplit), N = 131,072 6,262 (two, 19 runs; 6,417 with
 // one); four targets per thread were nowhere faster (6,333 at N = 131,072).
-// Small systems go to steps.cu, those from kDirRingMin bodies on to the ring kernel.
+// Small systems go to steps.cu.  The ring kernel takes those from kDirRingMin bodies
+// on, and from kDirRingFit on where whole waves of its CTAs keep the SMs busy for 98.5 %
+// of the time: its rate per busy SM is 1.6 % higher, its waves are coarser.  us, ring
+// against direct_kernel: N = 262,144 (97.8 % busy) 24,993 / 24,910, 265,000 (99.2)
+// 25,294 / 25,481, 270,000 (99.0) 26,191 / 26,708, 275,000 (98.1) 27,626 / 27,392,
+// 280,000 (95.8) 29,119 / 28,563, 285,000 (97.1) 29,658 / 29,429, 290,000 (99.1)
+// 30,195 / 30,645, 294,911 (99.0) 31,196 / 31,812.
+constexpr int64_t kDirRingFit = 262144;
 constexpr int64_t kDirRingMin = 294912;
+constexpr double kDirRingBusy = 0.985;
+
+// The ring kernel's plan for n bodies: runs so that the CTAs fill whole waves.
+// `busy`: the part of its waves' time that is spent on the n^2 interactions.
+static DirectPlan plan_ring(int64_t n, int max_splits, double* busy) {
+  static const int occ = [] {
+    int b = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, direct_ring_kernel<true, false>, kDirHalf, 0);
+    return std::max(b, 1);
+  }();
+  constexpr int64_t T = (int64_t)kDirHalf * 8;
+  const int64_t slots = (int64_t)num_sms() * occ;
+  DirectPlan p;
+  p.ring = true;
+  p.per_thread = 8;
+  p.i_blocks = ceil_div(n, T);
+  p.n_tgt_pad = p.i_blocks * T;
+  const int64_t tiles = ceil_div(n, (int64_t)kRingTile);
+  double eff = -1.0;
+  for (int64_t s = 1; s <= std::min<int64_t>(max_splits, tiles / 4); ++s) {
+    const double waves = (double)(p.i_blocks * s) / (double)slots;
+    const double e = waves / std::ceil(waves);
+    const int64_t per = ceil_div(tiles, s);
+    if (s > 1 && ceil_div(tiles, per) != s) continue;
+    if (s == 1 || e > eff + 0.02) {
+      eff = e;
+      p.splits = (int)s;
+      p.jper = per * kRingTile;
+    }
+    if (e >= 0.97) break;
+  }
+  *busy = (double)n * (double)n /
+          ((double)(ceil_div(p.i_blocks * p.splits, slots) * slots) * (double)(p.jper * T));
+  return p;
+}
 
 DirectPlan plan_direct(int64_t n, int max_splits) {
   constexpr double kCtaClocks = 3000.0, kRunClocks = 60.0;
@@ -266,34 +308,10 @@ DirectPlan plan_direct(int64_t n, int max_splits) {
   const int64_t sms = num_sms();
   DirectPlan best;
   if ((best.small = direct_small_fit(n))) return best;
-  if (n >= kDirRingMin) {
-    // runs so that the CTAs fill whole waves
-    static const int occ = [] {
-      int b = 0;
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, direct_ring_kernel<true, false>, kDirHalf,
-                                                    0);
-      return std::max(b, 1);
-    }();
-    best.ring = true;
-    best.per_thread = 8;
-    best.i_blocks = ceil_div(n, (int64_t)kDirHalf * 8);
-    best.n_tgt_pad = best.i_blocks * kDirHalf * 8;
-    const int64_t tiles = ceil_div(n, (int64_t)kRingTile);
-    double eff = -1.0;
-    for (int64_t s = 1; s <= std::min<int64_t>(max_splits, tiles / 4);
-         ++s) {
-      const double waves = (double)(best.i_blocks * s) / (double)(sms * occ);
-      const double e = waves / std::ceil(waves);
-      const int64_t per = ceil_div(tiles, s);
-      if (s > 1 && ceil_div(tiles, per) != s) continue;
-      if (s == 1 || e > eff + 0.02) {
-        eff = e;
-        best.splits = (int)s;
-        best.jper = per * kRingTile;
-      }
-      if (e >= 0.97) break;
-    }
-    return best;
+  if (n > kDirRingFit) {
+    double busy = 0.0;
+    const DirectPlan ring = plan_ring(n, max_splits, &busy);
+    if (n >= kDirRingMin || busy >= kDirRingBusy) return ring;
   }
   double best_t = 1e300;
   for (int I = 1; I <= 2; ++I) {
