@@ -375,6 +375,7 @@ nbgb_status nbgb_calculator_create(nbgb_method method, const nbgb_params* params
     NBGB_CUDA(cudaStreamCreate(&c->stream));
     c->own_stream = true;
     c->err.ensure(1);
+    c->anchor.ensure(1);
     *out = c.release();
   });
 }

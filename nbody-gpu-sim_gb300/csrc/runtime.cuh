@@ -170,6 +170,10 @@ struct nbgb_calculator {
   nbgb::DevBuf<float4> partial;   // direct: finished runs per target block (zero between
                                   // calls), then the partial sums of the source runs
   nbgb::ErrorWord err;            // device error word
+  // Never used: keeps the driver's block of small allocations mapped.  Without any small
+  // allocation left, each system's first one maps the block again and its last one
+  // unmaps it (a small system created and destroyed 190 + 73 us instead of 96 + 18).
+  nbgb::DevBuf<uint32_t> anchor;
   nbgb::DevBuf<int32_t> counts;   // per-target interaction / neighbour counts
   nbgb::DevBuf<double> red;       // reduction partials
   nbgb::HostPinned<double> h_red;
