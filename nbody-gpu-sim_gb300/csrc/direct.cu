@@ -587,9 +587,10 @@ __global__ void __launch_bounds__(256) direct_f64_state_kernel(
 
 // Reciprocal square root in FP64: an FP32 seed y (relative error below 2^-22)
 // and one third-order step, y + y e (1/2 + 3/8 e) with e = 1 - d y^2 (the
-// binomial series of (1 - e)^(-1/2), remainder 5/16 e^3 < 2^-63); y^2 is exact
-// in FP64.  5 FP64 operations and two conversions.  Outside the seed's safe
-// range (and for zero, infinity and NaN) the math library's rsqrt.
+// binomial series of (1 - e)^(-1/2), remainder 5/16 e^3 < 2^-63, so that the last
+// operation's rounding is what remains); y^2 is exact in FP64.  5 FP64 operations and
+// two conversions.  Outside the seed's safe range (and for zero, infinity and NaN) the
+// math library's rsqrt.
 __device__ __forceinline__ double rsqrt_f64(double d) {
   const uint32_t hi = (uint32_t)__double2hiint(d);
   if (hi - 0x38f00000u > 0x0e000000u) return rsqrt(d);  // outside 2^-112 .. 2^112
@@ -602,9 +603,10 @@ __device__ __forceinline__ double rsqrt_f64(double d) {
 // one launch.  PE: every unordered pair once, as 64 x 64 tiles of the upper
 // triangle dealt out to the CTAs (a thread keeps one target of the tile, the
 // sources are read from shared memory).  Bound by the FP64 pipe (2 lanes per
-// clock and SM, 12 operations per pair): small tiles, so that few bodies
-// still reach every SM.  N = 8,191: 6.9 ms as one 256-target CTA per row of
-// ordered pairs (32 CTAs), 0.93 ms now (0.64 at the FP64 rate).
+// clock and SM; 12 operations per pair, and the two conversions run there as well):
+// small tiles, so that few bodies still reach every SM.  N = 8,191: 6.9 ms as one
+// 256-target CTA per row of ordered pairs (32 CTAs), 0.93 ms now with the pipe 87 %
+// busy (0.75 at its full rate).
 constexpr int kPeTile = 64;
 
 __global__ void __launch_bounds__(kPeTile) energy_f64_kernel(EnergyArgs a) {
