@@ -73,15 +73,6 @@ __global__ void seg_of_kernel(const int64_t* __restrict__ base, int nseg, int64_
   }
 }
 
-// Order-preserving float <-> uint32 (for exact min/max with integer atomics).
-__device__ __forceinline__ uint32_t f2ord(float f) {
-  const uint32_t u = __float_as_uint(f);
-  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
-__device__ __forceinline__ float ord2f(uint32_t u) {
-  return __uint_as_float((u & 0x80000000u) ? (u & 0x7fffffffu) : ~u);
-}
-
 // Per-segment min/max of the bodies, and from them the reference's derived
 // constants with its float operations
 //   Morton scale  inv = 1.0f / (max - min + 0.001f)            (:313-320)
@@ -105,7 +96,7 @@ __device__ __forceinline__ void seg_box(const uint32_t* mm, int nseg, int s, BBo
   BBox o;
   bool ok = true;
   for (int a = 0; a < 3; ++a) {
-    const float mn = ord2f(~__ldcg(&mm[a * nseg + s])), mx = ord2f(__ldcg(&mm[(3 + a) * nseg + s]));
+    const float mn = float_of(~__ldcg(&mm[a * nseg + s])), mx = float_of(__ldcg(&mm[(3 + a) * nseg + s]));
     o.min[a] = mn;
     o.max[a] = mx;
     ok = ok && isfinite(mn) && isfinite(mx);
@@ -161,8 +152,8 @@ __global__ void seg_bounds_kernel(const float4* pm, SegView sv, int64_t n, int n
         const float w[6] = {fminf(1e30f, p.x),  fminf(1e30f, p.y),  fminf(1e30f, p.z),
                             fmaxf(-1e30f, p.x), fmaxf(-1e30f, p.y), fmaxf(-1e30f, p.z)};
         for (int a = 0; a < 3; ++a) {
-          atomicMax(&mm[a * nseg + s], ~f2ord(w[a]));
-          atomicMax(&mm[(3 + a) * nseg + s], f2ord(w[3 + a]));
+          atomicMax(&mm[a * nseg + s], ~ord_of(w[a]));
+          atomicMax(&mm[(3 + a) * nseg + s], ord_of(w[3 + a]));
         }
       }
     }
@@ -183,7 +174,7 @@ __global__ void seg_bounds_kernel(const float4* pm, SegView sv, int64_t n, int n
       float x = s_red[0][a];
       for (int w = 1; w < (int)(blockDim.x >> 5); ++w)
         x = a < 3 ? fminf(x, s_red[w][a]) : fmaxf(x, s_red[w][a]);
-      atomicMax(&mm[a * nseg + s0], a < 3 ? ~f2ord(x) : f2ord(x));
+      atomicMax(&mm[a * nseg + s0], a < 3 ? ~ord_of(x) : ord_of(x));
     }
   }
   __threadfence();

@@ -56,21 +56,6 @@ struct GroupWalkArgs {
   unsigned long long* cost_acc;     // out: total cost, groups
 };
 
-// Floats as unsigned integers with the same order (finite values).
-__device__ __forceinline__ uint32_t ord_of(float f) {
-  const uint32_t u = __float_as_uint(f);
-  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
-__device__ __forceinline__ float float_of(uint32_t o) {
-  return __uint_as_float((o & 0x80000000u) ? (o & 0x7fffffffu) : ~o);
-}
-
-__device__ __forceinline__ void f2_sum(f2 v, float& s) {
-  float lo, hi;
-  f2_split(v, lo, hi);
-  s = lo + hi;
-}
-
 // One pair of list entries (packed x, y, z, m) added to one target.
 template <bool ZERO_EPS>
 __device__ __forceinline__ void pair_add(f2 xj, f2 yj, f2 zj, f2 m, f2 px, f2 py, f2 pz, f2 e2,
@@ -481,13 +466,8 @@ __global__ void __launch_bounds__(kGWarps * 32, TWO ? 3 : 4) bh_group_walk_kerne
     if (COUNT)
       selfmask = (uint64_t)__reduce_or_sync(full, (uint32_t)selfmask) |
                  ((uint64_t)__reduce_or_sync(full, (uint32_t)(selfmask >> 32)) << 32);
-    float fx, fy, fz, hx, hy, hz;
-    f2_sum(ax2, fx);
-    f2_sum(ay2, fy);
-    f2_sum(az2, fz);
-    f2_sum(bx2, hx);
-    f2_sum(by2, hy);
-    f2_sum(bz2, hz);
+    float fx = f2_sum(ax2), fy = f2_sum(ay2), fz = f2_sum(az2);
+    const float hx = f2_sum(bx2), hy = f2_sum(by2), hz = f2_sum(bz2);
     if (K > 1) {  // the warps' sums, in order, through their rings
       float* r = s_ring[wid][0];
       if (tw > 0) {

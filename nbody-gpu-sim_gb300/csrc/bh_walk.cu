@@ -138,15 +138,6 @@ __device__ __forceinline__ void list_eval(const float (&e)[4][kWRing], const uin
   }
 }
 
-// Floats as unsigned integers with the same order (finite values).
-__device__ __forceinline__ uint32_t walk_ord(float f) {
-  const uint32_t u = __float_as_uint(f);
-  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
-__device__ __forceinline__ float walk_unord(uint32_t o) {
-  return __uint_as_float((o & 0x80000000u) ? (o & 0x7fffffffu) : ~o);
-}
-
 template <bool COUNT, bool BUCKET, int TW>
 __global__ void __launch_bounds__(kWWarps * 32, 3) bh_walk_kernel(WalkArgs a) {
   constexpr int REP = 32 / TW;
@@ -175,12 +166,12 @@ __global__ void __launch_bounds__(kWWarps * 32, 3) bh_walk_kernel(WalkArgs a) {
     // the targets' box: centre and half sizes, the halves widened past rounding
     float bx, by, bz, hx, hy, hz;
     {
-      const float lx = walk_unord(__reduce_min_sync(all, walk_ord(pi.x)));
-      const float ly = walk_unord(__reduce_min_sync(all, walk_ord(pi.y)));
-      const float lz = walk_unord(__reduce_min_sync(all, walk_ord(pi.z)));
-      const float ux = walk_unord(__reduce_max_sync(all, walk_ord(pi.x)));
-      const float uy = walk_unord(__reduce_max_sync(all, walk_ord(pi.y)));
-      const float uz = walk_unord(__reduce_max_sync(all, walk_ord(pi.z)));
+      const float lx = float_of(__reduce_min_sync(all, ord_of(pi.x)));
+      const float ly = float_of(__reduce_min_sync(all, ord_of(pi.y)));
+      const float lz = float_of(__reduce_min_sync(all, ord_of(pi.z)));
+      const float ux = float_of(__reduce_max_sync(all, ord_of(pi.x)));
+      const float uy = float_of(__reduce_max_sync(all, ord_of(pi.y)));
+      const float uz = float_of(__reduce_max_sync(all, ord_of(pi.z)));
       bx = __fmul_rn(__fadd_rn(lx, ux), 0.5f);
       by = __fmul_rn(__fadd_rn(ly, uy), 0.5f);
       bz = __fmul_rn(__fadd_rn(lz, uz), 0.5f);

@@ -142,6 +142,21 @@ __device__ __forceinline__ f2 f2_make(float lo, float hi) {
 __device__ __forceinline__ void f2_split(f2 a, float& lo, float& hi) {
   asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(a.v));
 }
+__device__ __forceinline__ float f2_sum(f2 a) {
+  float lo, hi;
+  f2_split(a, lo, hi);
+  return lo + hi;
+}
+
+// Floats as unsigned integers with the same order (finite values), for exact
+// minima and maxima by integer instructions.
+__device__ __forceinline__ uint32_t ord_of(float f) {
+  const uint32_t u = __float_as_uint(f);
+  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+__device__ __forceinline__ float float_of(uint32_t o) {
+  return __uint_as_float((o & 0x80000000u) ? (o & 0x7fffffffu) : ~o);
+}
 __device__ __forceinline__ f2 f2_sub(f2 a, f2 b) {
   f2 r;
   asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));

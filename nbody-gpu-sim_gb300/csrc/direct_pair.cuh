@@ -7,12 +7,6 @@
 
 namespace nbgb {
 
-__device__ __forceinline__ float f2_sum(f2 a) {
-  float lo, hi;
-  f2_split(a, lo, hi);
-  return lo + hi;
-}
-
 // Adds t to a running sum: error-free into (s, e), or in plain FP32.
 template <bool COMP>
 __device__ __forceinline__ void fold(float t, float& s, float& e) {
