@@ -551,8 +551,9 @@ static void launch_group_walk_t(const GroupWalkArgs& g, int64_t n, cudaStream_t 
     launch_chained(bh_group_walk_kernel<CNT, ZERO_EPS, TWO, K>, (unsigned)blocks, kGWarps * 32, 0,
                    st, g);
   } else {
-    // (not chained: a full wave placed beside the build's last blocks, 1M bodies 2743 us
-    // instead of 2731, a burst of 24 served systems 21.0 ms instead of 20.8)
+    // (not chained: a full wave placed beside the build's last blocks costs as much as the
+    // launch saves; 1M bodies chained / not 2,747 / 2,734 us in each of three runs that
+    // differ by 0.1 % in themselves, 200 K with buckets 813 / 815, served systems the same)
     bh_group_walk_kernel<CNT, ZERO_EPS, TWO, K><<<(unsigned)blocks, kGWarps * 32, 0, st>>>(g);
     NBGB_LAUNCH_CHECK();
   }

@@ -468,7 +468,8 @@ __global__ void groups_kernel(const Node* nodes, const uint32_t* nstart,
 //                   at once, with the centres of mass that are done, so that a level
 //                   works in shared memory.
 constexpr int kComBodies = 512;  // bodies per block of the centre-of-mass kernel
-constexpr int kComSlots = 1280;  // nodes a block holds in shared memory (1.5 per body)
+constexpr int kComSlots = 1280;  // nodes a block holds in shared memory (2.5 per body; about 1.5
+                                 // occur)
 
 struct ComArgs {
   Node* nodes;

@@ -129,7 +129,7 @@ __global__ void ens_admit_kernel(const float* __restrict__ stage, int64_t n, int
 // memory: x, y, z, vx, vy, vz (n doubles each), ax, ay, az, m (n floats each), the
 // device error word (bounded waits, tree capacity, non-finite bounds) and 0.  One
 // launch per system, where a kick and eleven copies took 12 places in the stream
-// (a burst of 24 systems that finish together 21.6 ms, now 20.9).
+// (a burst of 24 systems that finish together 21.6 ms, 20.9 with it).
 __global__ void ens_retire_kernel(int64_t n, const double* __restrict__ x,
                                   const double* __restrict__ y, const double* __restrict__ z,
                                   const double* __restrict__ vx, const double* __restrict__ vy,
@@ -224,8 +224,8 @@ template <int T, int I, bool P>
 static int occ_of() {
   int b = 0;
   // the tree build's kernels need up to 195 KB of shared memory on an SM beside
-  // this kernel, which its own 12 KB would not leave (a 24-system burst 19.4 ms
-  // against 19.7)
+  // this kernel, which its own 12 KB would not leave (a 24-system burst 20.9 ms
+  // against 21.1 in each of three runs)
   NBGB_CUDA(cudaFuncSetAttribute(ens_direct_kernel<T, I, P>,
                                  cudaFuncAttributePreferredSharedMemoryCarveout,
                                  cudaSharedmemCarveoutMaxShared));
@@ -862,7 +862,7 @@ static void run_tick(nbgb_ensemble* e) {
     // occupancy; 2 per SM 5.86, one per two SMs 5.83).  Alone, full occupancy.
     // The build waits until these CTAs have their places: with its blocks on the
     // SMs first, all 152 could end up on 16 of them (a tick 1.49 ms instead of
-    // 0.78, a burst of 24 systems 31 ms instead of 19.4).
+    // 0.78, a burst of 24 systems 31 ms instead of 22).
     const int grid = bh_work ? num_sms() : num_sms() * e->direct_occ[e->config];
     launch_config(e->config, grid, e->d_items.ptr, e->n_items, e->d_counter.ptr, e->pm.ptr,
                   e->ax.ptr, e->ay.ptr, e->az.ptr, e->cfg.softening * e->cfg.softening, e->cfg.G,

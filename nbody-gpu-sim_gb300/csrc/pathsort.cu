@@ -454,7 +454,7 @@ void path_sort(const float4* pm, const SegView& sv, const int32_t* first, int nb
     launch_chained(ps_count_kernel, gc, 256, (size_t)nb * 16, st, a);
   } else {
     // (not chained: blocks placed beside the ranking's last ones share SMs to the end,
-    // the keys of 1M bodies 85 us instead of 68)
+    // the keys of 1M bodies 85 us instead of 65)
     ps_count_kernel<<<gc, 256, (size_t)nb * 16, st>>>(a);
     NBGB_LAUNCH_CHECK();
   }
