@@ -408,6 +408,8 @@ static unsigned grid1d(int64_t n, int threads = 256) {
       1, std::min<int64_t>(ceil_div(std::max<int64_t>(n, 1), threads), (int64_t)num_sms() * 32));
 }
 
+constexpr int64_t kHashMaxCells = 100000000;  // the reference's cap
+
 // How the gather's work is split (in us, uniform cubes):
 //  threads per pair  at 8 bodies per cell 30 K: 9 take 14, 4 take 18, 1 takes 43;
 //                    400 K: 90, 80, 93; 1M: 215, 186, 176;
@@ -447,13 +449,19 @@ void hash_forces(nbgb_calculator* c, const float4* pm, int64_t n, float* ax, flo
     volatile float hi = hb->max[a] + 0.001f;
     float ext = hi - lo;
     volatile float q = ext / cell;
+    const float cells = std::ceil((float)q);
     g.bmin[a] = lo;
-    g.dims[a] = (int)std::ceil((float)q) + 1;
-    total *= (int64_t)g.dims[a];
+    // (checked per axis: a product of three could wrap around, as could the conversion)
+    if (cells < (float)kHashMaxCells) {
+      g.dims[a] = (int)cells + 1;
+      total *= (int64_t)g.dims[a];
+    } else {
+      total = kHashMaxCells + 1;
+    }
+    if (total > kHashMaxCells)
+      fail(NBGB_ERR_OVERFLOW, "Spatial hash grid too large: reduce cell_size or bounding box");
   }
   g.cell = cell;
-  if (total > 100000000)
-    fail(NBGB_ERR_OVERFLOW, "Spatial hash grid too large: reduce cell_size or bounding box");
   h.n = n;
   h.total = total;
   h.cell = cell;
