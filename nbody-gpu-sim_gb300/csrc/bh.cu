@@ -259,7 +259,7 @@ struct TieRun {
   int64_t first, count;
 };
 
-__device__ void tie_sort_run(TieRun t, const BBox& b, uint32_t* body, u64* lo, float4* spm) {
+__device__ __noinline__ void tie_sort_run(TieRun t, const BBox& b, uint32_t* body, u64* lo, float4* spm) {
   const int tid = threadIdx.x;
   const int64_t m = t.count;
   body += t.first;
@@ -306,15 +306,14 @@ __global__ void __launch_bounds__(kTieThreads)
   for (int64_t k0 = blockIdx.x * (int64_t)kTieThreads; k0 + 1 < n;
        k0 += (int64_t)gridDim.x * kTieThreads) {
     const int64_t k = k0 + threadIdx.x;
-    if (threadIdx.x == 0) s_runs = 0;
-    __syncthreads();
+    int64_t count = 0;  // of a long run that starts here
     if (k + 1 < n && same(k, k + 1) && !(k > 0 && same(k - 1, k))) {
       int64_t e = k + 1, step = 1;  // the run's last body
       for (; e + step < n && same(k, e + step); step <<= 1) e += step;
       for (; step > 0; step >>= 1)
         if (e + step < n && same(k, e + step)) e += step;
       if (e - k >= kTieRun) {
-        s_run[atomicAdd(&s_runs, 1)] = TieRun{k, e - k + 1};
+        count = e - k + 1;
       } else {
         const BBox b = sv.box[kseg[k]];
         lo[k] = low_key(spm[k], b);
@@ -335,9 +334,12 @@ __global__ void __launch_bounds__(kTieThreads)
         }
       }
     }
+    if (!__syncthreads_or(count > 0)) continue;
+    if (threadIdx.x == 0) s_runs = 0;
     __syncthreads();
-    const int runs = s_runs;
-    for (int r = 0; r < runs; ++r)
+    if (count > 0) s_run[atomicAdd(&s_runs, 1)] = TieRun{k, count};
+    __syncthreads();
+    for (int r = 0; r < s_runs; ++r)
       tie_sort_run(s_run[r], sv.box[kseg[s_run[r].first]], body, lo, spm);
     __syncthreads();
   }
