@@ -178,6 +178,11 @@ __global__ void __launch_bounds__(kWWarps * 32, 3) bh_walk_kernel(WalkArgs a) {
       hx = __fmul_rn(fmaxf(__fsub_rn(ux, bx), __fsub_rn(bx, lx)), kBoxWiden);
       hy = __fmul_rn(fmaxf(__fsub_rn(uy, by), __fsub_rn(by, ly)), kBoxWiden);
       hz = __fmul_rn(fmaxf(__fsub_rn(uz, bz), __fsub_rn(bz, lz)), kBoxWiden);
+      // a NaN position, which the minima and maxima need not show: target by target
+      if (__any_sync(all, isnan(pi.x + pi.y + pi.z))) {
+        bx = by = bz = 0.f;
+        hx = hy = hz = INFINITY;
+      }
     }
     f2 ax = f2_make(0.f, 0.f), ay = ax, az = ax;
     float sx = 0.f, sy = 0.f, sz = 0.f;  // single additions
