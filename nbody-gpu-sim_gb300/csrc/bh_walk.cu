@@ -408,7 +408,8 @@ __global__ void __launch_bounds__(kWWarps * 32, 3) bh_walk_kernel(WalkArgs a) {
                       uz = __fmaf_rn(cz, kOut, hz);
           const float dmin = __fmaf_rn(nz, nz, __fmaf_rn(ny, ny, __fmaf_rn(nx, nx, a.eps2)));
           const float dmax = __fmaf_rn(uz, uz, __fmaf_rn(uy, uy, __fmaf_rn(ux, ux, a.eps2)));
-          const bool every = apart && dmin > 1e-30f && dmin < 1e37f && size2 > 1e-30f &&
+          // (a NaN centre of mass shows in dmax, not in dmin, and is decided there too)
+          const bool every = apart && dmin > 1e-30f && dmax < 1e37f && size2 > 1e-30f &&
                              size2 < __fmul_rn(dmin, a.th_all_lo);
           const bool none = size2 > 1e-30f && dmax < 1e37f && dmax > 1e-30f &&
                             size2 > __fmul_rn(dmax, a.th_all_hi);
