@@ -97,8 +97,9 @@ typedef struct nbgb_params {
  * after computeForces).  Clear it to enqueue asynchronously and check with
  * nbgb_calculator_synchronize(). */
 #define NBGB_FLAG_SYNC 0x1u
-/* Per-target compensated (two-sum) accumulation across j-tiles.  Clear it
- * for the plain FP32 sum (one running FP32 accumulator, as the reference). */
+/* Per-target compensated (two-sum) accumulation of partial sums, each of at most
+ * 304 sources in two plain FP32 sums or 256 in one.  Clear it for plain FP32 sums
+ * throughout. */
 #define NBGB_FLAG_COMPENSATED 0x2u
 /* Record per-target accepted-interaction counts (Barnes-Hut) or neighbour
  * counts (spatial hash) for nbgb_copy_interaction_counts(). */
